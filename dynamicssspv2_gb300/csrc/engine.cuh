@@ -101,7 +101,9 @@ struct __align__(128) Ctl {
     // line 3: relaxation lists, round r reads slot r%3
     unsigned rcT[3];
     unsigned rcC[3];
-    unsigned pad3[26];
+    unsigned rsteps[3];  // steps of the local stretch that wrote the list (the most of any warp)
+    unsigned rstop[3];   // ... set by a CTA whose share of it has grown too large: the stretch ends
+    unsigned pad3[20];
     // line 4: cut-off lists (level L appends to slot (L+1)%3), pointer jumping
     unsigned ltT[3];
     unsigned ltC[3];
@@ -110,12 +112,12 @@ struct __align__(128) Ctl {
     unsigned pjf[3];
     unsigned fc[2];  // near-far: far-list counts (double buffer)
     unsigned pad4[19];
-    // line 4b: near-far threshold reduction (double buffer)
-    unsigned long long fmin[2];
+    // line 4b: near-far threshold reduction
+    unsigned long long fmin;
     // small steps run by CTA 0 alone hand their end state to the grid here
     unsigned long long solo[4];
     unsigned solo_n[2];  // list sizes of the first round after solo relaxation rounds
-    unsigned pad4b[18];
+    unsigned pad4b[20];
     // line 5: barrier diagnostics (first timed-out barrier, arrivals then, CTAs that timed
     // out, max barrier count at exit, 0xFFFFFFFF - min barrier count at exit)
     unsigned diag[8];

@@ -54,6 +54,17 @@ constexpr int kAddsPerCheck = 32;          // entries a warp may add between two
                                            // for its four adds instead)
 static_assert(kBuf > kAddsPerCheck, "a push buffer must take one visit's adds after a check");
 constexpr int kSoloSteps = 256;            // consecutive solo steps before the grid re-syncs
+constexpr unsigned kQueue = 256;           // items of a CTA's queue in a local stretch (two queues)
+constexpr unsigned kLocalDeg = 32;         // rows above this leave a local stretch through the lists
+constexpr int kLocalTe = 16;               // thread items of more edges than this keep to the rounds
+constexpr unsigned kFarBuf = 64;           // per-warp staging of far-list pushes
+constexpr int kSpill = 64;                 // per-warp staging of vertices that leave a stretch
+constexpr unsigned kStretch = 256;         // steps of a local stretch at most
+static_assert(64 * (kLocalTe / 4) <= kQueue, "a CTA's first items must fit its queue");
+// a stretch keeps all of it in the push buffers: per warp kSpill entries pushed, then a share of
+// the two queues, then the far staging
+constexpr unsigned kShare = 2 * kQueue / kMaxWarps;
+static_assert(kSpill + kShare + kFarBuf / 4 <= kBuf && kSpill >= 2 * 32, "a stretch fits the push buffers");
 
 __shared__ unsigned s_nbar;        // grid barriers this CTA has passed
 __shared__ unsigned s_gen;         // barrier generation this CTA waits on next (ctl->bar_gen)
@@ -64,6 +75,10 @@ __shared__ unsigned s_ggen;        // group-barrier generation this CTA waits on
 __shared__ unsigned s_solo_cnt[3][2];
 __shared__ unsigned s_spin_limit;  // polls before a grid barrier gives up
 __shared__ uint4 s_pbuf[kMaxWarps][kBuf];  // (vertex, degree, row start) pushed, not yet expanded
+__shared__ unsigned s_stop;                // ... another CTA has ended the stretch
+__shared__ unsigned s_qcnt[3];             // local stretches: items of the steps' queues, rotating
+__shared__ unsigned s_near[2];  // far_advance: the sizes of the near list
+__shared__ unsigned long long s_lstat[8];  // ... their counters, added to the kernel's at the end
 __shared__ unsigned s_wlist[kMaxWarps][kListRegion];  // k_delete / k_append list staging
 
 // Per-thread counters (32 bits: a thread's share stays far below 2^32 in any run; the block
@@ -80,9 +95,10 @@ struct LocalStats {
 // complete before every CTA has arrived), so arriving costs no load.  With a and b given,
 // the two counters the caller needs next are read once per CTA together with the status
 // word and returned in va and vb.
-__device__ bool grid_sync(Ctl* ctl, const unsigned* a, const unsigned* b, unsigned& va, unsigned& vb) {
+__device__ bool grid_sync(Ctl* ctl, const unsigned* a, const unsigned* b, unsigned& va, unsigned& vb,
+                          const unsigned* c, unsigned& vc) {
     __shared__ int s_go;
-    __shared__ unsigned s_va, s_vb;
+    __shared__ unsigned s_va, s_vb, s_vc;
     __syncthreads();
     if (threadIdx.x == 0) {
         const unsigned gen = s_gen;
@@ -112,12 +128,19 @@ __device__ bool grid_sync(Ctl* ctl, const unsigned* a, const unsigned* b, unsign
         const int st = __ldcg(&ctl->status);
         s_va = a ? __ldcg(a) : 0u;
         s_vb = b ? __ldcg(b) : 0u;
+        s_vc = c ? __ldcg(c) : 0u;
         s_go = st == 0;
     }
     __syncthreads();
     va = s_va;
     vb = s_vb;
+    vc = s_vc;
     return s_go != 0;
+}
+
+__device__ __forceinline__ bool grid_sync(Ctl* ctl, const unsigned* a, const unsigned* b, unsigned& va, unsigned& vb) {
+    unsigned x;
+    return grid_sync(ctl, a, b, va, vb, nullptr, x);
 }
 
 // Barrier of the first G CTAs (a group running mid-size steps while the others wait at the
@@ -771,22 +794,211 @@ __device__ void run_items(Op& op, const UpdParams& p, const Item* tl, unsigned n
     op.finish();
 }
 
-// Block-reduced statistics: one atomic per block and counter.
-__device__ void flush_stats(Ctl* ctl, const LocalStats& ls) {
-    __shared__ unsigned long long s_acc[8];
-    if (threadIdx.x < 8) s_acc[threadIdx.x] = 0;
-    __syncthreads();
-    const unsigned long long v[8] = {ls.edges_relax, ls.edges_inv, ls.updates, ls.dist_ovf,
-                                     ls.frontier, ls.items, ls.marked, ls.edges_pull};
+// ---- local stretches -------------------------------------------------------------------------
+// A relaxation round of few items is one chain of dependent accesses plus a grid barrier, about
+// 8 us however small it is.  A local stretch replaces a run of such rounds: every CTA takes a share
+// of the round's items into a queue in shared memory and relaxes on from there for up to `steps`
+// steps, pushing what it improves into the next step's queue, with one block barrier a step and
+// no grid barrier.  Four lanes share an item of at most four entries, and the chain of a step is
+// two accesses long: the entry beside the vertex's own state, then the offer beside the
+// neighbour's row descriptor (which the next step needs if the offer wins).  What still waits at
+// the end, rows above kLocalDeg and what does not fit the queue go to the grid's lists, claimed as
+// in a round; distances at or above the near-far threshold go to the far list.  The order of
+// relaxations differs from the rounds', the fixpoint does not: every strict improvement is pushed
+// by the thread that made it, and an item is dropped only if its vertex has been improved again
+// since (then that thread has pushed it).  The queue's pushes mark chg_tag, not push_tag, whose
+// tag says "claimed for the next list".
+//
+// Bound: the latency of the two accesses, 940 and 1,200-1,300 cycles of a step's 3,500-3,900 (clock
+// counts on grids of 1.6M and 16.8M vertices), then the push, the block barrier and, per stretch,
+// a grid barrier with a new deal of the work.  A queue per CTA, not per warp: with one per warp a
+// step was 2.05 us instead of 2.7 (with its share of the deals), but a queue that grew past 32
+// entries took several steps a hop and the others waited for it (4096^2 grid, 100k changes: 21,476
+// steps, 46 ms a batch, against 12,310 and 36 ms).  A CTA whose queue passes one and a half passes
+// ends everybody's stretch (rstop), so the work is dealt out again when it is needed and not every
+// 16 or 64 steps (27.1 ms against 28.6 and 36).  Measured against rounds throughout: that batch
+// 95.0 -> 27.1 ms, a 1021 x 1543 grid with 9k changes 23.3 -> 7.8 ms, the tree of a 2048^2 grid
+// 38.0 -> 12.0 ms, ER graphs of 10k and 300k vertices 0.157 -> 0.130 and 0.264 -> 0.211 ms of k_update.
+// A round is a local stretch when it holds thread items only, no more than one pass of every CTA:
+// above that the grid is busy and the rounds' throughput counts.  (Half or a quarter of a pass:
+// the same on grids and ER graphs within 2 %, 64 pooled ER graphs 0.405 -> 0.410 and 0.424 ms.)
+__device__ __forceinline__ bool local_step(const UpdParams& p, unsigned nt, unsigned nc) {
+    return nc == 0 && nt <= gridDim.x * (blockDim.x >> 2) && p.te <= kLocalTe && p.group_ctas == 0;
+}
+
+// Item i of queue q (0 or 1): (vertex, distance, slots, count), at most 4 slots each.
+__device__ __forceinline__ uint4& queue_at(unsigned q, unsigned i) {
+    const unsigned k = q * kQueue + i;
+    return s_pbuf[k / kShare][kSpill + k % kShare];
+}
+__device__ __forceinline__ unsigned* far_buf() {
+    return reinterpret_cast<unsigned*>(&s_pbuf[threadIdx.x >> 5][kSpill + kShare]);
+}
+
+__device__ __forceinline__ void keep_stats(const LocalStats& ls);
+
+struct Stretch {
+    const UpdParams* p;
+    Out out;
+    Far far;
+    unsigned tag;
+    PushBuf pb;
+    unsigned nfar;
+    LocalStats ls;
+
+    __device__ __forceinline__ void spill(bool pred, unsigned v, const RowDesc& rd) {
+        if (pb.count + 32 > kSpill) pb.expand_all(*p, out, ls);
+        pb.add(pred, v, rd);
+        ls.frontier += pred ? 1 : 0;
+    }
+
+    __device__ __forceinline__ void flush_far() {
+        __syncwarp();
+        const unsigned* lfar = far_buf();
+        for (unsigned b = 0; b < nfar; b += 32)
+            far_push(*p, far, b + lane_id() < nfar, lfar[(b + lane_id()) & (kFarBuf - 1)]);
+        nfar = 0;
+        __syncwarp();
+    }
+
+    // One item's entry per lane (warp-collective): x = the item (count 0: none), next = the
+    // number of the next step's queue, with its counter.
+    __device__ __forceinline__ void visit(const uint4& x, unsigned next, unsigned* next_cnt) {
+        const unsigned lane = lane_id(), lt = (1u << lane) - 1u, sub = lane & 3u;
+        unsigned long long* const state = p->g.state;
+        const bool act = sub < (x.w >> 8);
+        const long long j = (long long)((unsigned long long)(x.w & 0xFFu) << 32 | x.z) + sub;
+        const int2 e = act ? ld_stream(&p->g.adj[j]) : make_int2(0, -1);
+        const unsigned long long du = act ? __ldcg(&state[x.x]) >> 32 : kDistInf;
+        const bool live = du < kDistInf && du >= x.y;  // below: improved since, and pushed again then
+        const unsigned c = (unsigned)e.x;
+        const unsigned long long nd = du + (unsigned)e.y;
+        RowDesc rd{0, 0, 0};
+        bool push = false;
+        if (live && e.y >= 0) {
+            rd = p->g.rows[c];
+            if (e.y == 0) {
+                push = relax_to(p->g, p->epoch, c, nd, x.x, 0, __ldcg(&state[c]), ls);
+            } else if (nd < kDistInf) {
+                const unsigned long long cand = (nd << 32) | x.x;
+                const unsigned long long old = atomicMin(&state[c], cand);
+                push = (old >> 32) > nd;
+                if (push) ls.updates++;
+                else if (old > cand && p->g.chg_tag) p->g.chg_tag[c] = p->epoch;
+            } else if (__ldcg(&state[c]) == kInfState) {
+                ls.dist_ovf++;
+            }
+        }
+        ls.edges_relax += live ? 1 : 0;
+        if (!__any_sync(kFull, push)) return;
+        const bool later = push && nd >= far.T;
+        const bool near = push && !later && rd.deg > 0;
+        // queue places: ceil(deg / 4) items a row, ranked in the warp by the bits of (items - 1)
+        const bool shrt = near && rd.deg <= (int)kLocalDeg;
+        const unsigned extra = shrt ? ((unsigned)rd.deg - 1u) >> 2 : 0u;
+        const unsigned m = __ballot_sync(kFull, shrt);
+        bool in = false;
+        if (m) {
+            unsigned rank = __popc(m & lt), total = __popc(m);
+            if (__any_sync(kFull, extra != 0)) {
 #pragma unroll
-    for (int s = 0; s < 8; s++) {
-        const unsigned long long x = warp_sum_u64(v[s]);
-        if (lane_id() == 0 && x) atomicAdd(&s_acc[s], x);
+                for (int b = 0; b < 3; b++) {
+                    const unsigned mb = __ballot_sync(kFull, extra & (1u << b));
+                    rank += __popc(mb & lt) << b;
+                    total += __popc(mb) << b;
+                }
+            }
+            unsigned base = 0;
+            if (lane == 0) base = atomicAdd(next_cnt, total);
+            const unsigned at = __shfl_sync(kFull, base, 0) + rank;
+            in = shrt && at + extra < kQueue;
+            if (in) {
+                long long lo = rd.start;
+                for (unsigned k = 0; k <= extra; k++, lo += 4)
+                    queue_at(next, at + k) =
+                        make_uint4(c, (unsigned)nd, (unsigned)lo, (unsigned)((unsigned long long)lo >> 32) |
+                                                                      (min(4u, (unsigned)rd.deg - 4 * k) << 8));
+                if (p->g.chg_tag) p->g.chg_tag[c] = p->epoch;
+                ls.frontier++;
+            } else if (shrt) {  // does not fit: its places stay empty
+                for (unsigned k = at; k < kQueue; k++) queue_at(next, k) = make_uint4(0, 0, 0, 0);
+            }
+        }
+        if (__any_sync(kFull, near && !in)) {
+            const bool won = near && !in && atomicExch(&p->g.push_tag[c], tag) != tag;
+            spill(won, c, rd);
+        }
+        const unsigned fmask = __ballot_sync(kFull, later);
+        if (fmask) {
+            if (nfar + __popc(fmask) > kFarBuf) flush_far();
+            if (later) far_buf()[nfar + __popc(fmask & lt)] = c;
+            nfar += __popc(fmask);
+        }
+    }
+};
+
+// CTA-collective; reads list r (nt thread items) and appends to list r + 1.  A function of its
+// own, with its own counters, so that the rounds keep their registers.
+__device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigned nt, unsigned steps_max,
+                                         unsigned rbase, unsigned adv, unsigned long long T) {
+    Ctl* const ctl = p.g.ctl;
+    const bool odd = (r & 1) != 0;
+    const unsigned slot = (r + 1) % 3;
+    const Item* const tl = odd ? p.g.rt1 : p.g.rt0;
+    const unsigned lane = lane_id(), per = blockDim.x >> 2, parts = (unsigned)p.te >> 2, limit = per + per / 2;
+    Stretch st{&p,
+               Out{odd ? p.g.rt0 : p.g.rt1, &ctl->rcT[slot], p.g.tcap, odd ? p.g.rc0 : p.g.rc1, &ctl->rcC[slot], p.g.ccap},
+               Far{(adv & 1) ? p.g.far1 : p.g.far0, &ctl->fc[adv & 1], p.g.far_tag, rbase + adv, (unsigned)p.g.n, T},
+               rbase + r + 2u, PushBuf{s_pbuf[threadIdx.x >> 5], 0}, 0, LocalStats{}};
+    // items blockIdx, blockIdx + gridDim, ... of the list, at most `per` of them
+    const unsigned mine = nt > blockIdx.x ? (nt - blockIdx.x - 1) / gridDim.x + 1 : 0u;
+    for (unsigned i = threadIdx.x; i < mine; i += blockDim.x) {
+        const Item it = __ldcg(&tl[blockIdx.x + (unsigned long long)i * gridDim.x]);
+        for (unsigned k = 0; k < parts; k++) {
+            const long long lo = item_lo(it) + 4 * k;
+            const unsigned cnt = it.w > 4 * k ? min(4u, it.w - 4 * k) : 0u;
+            queue_at(0, i * parts + k) =
+                make_uint4(it.z, 0u, (unsigned)lo, (unsigned)((unsigned long long)lo >> 32) | (cnt << 8));
+        }
+    }
+    if (threadIdx.x == 0) {
+        s_qcnt[0] = mine * parts;
+        s_qcnt[1] = 0;
+        s_stop = 0;
     }
     __syncthreads();
-    const int idx[8] = {ST_EDGES_RELAX, ST_EDGES_INV, ST_UPDATES, ST_DIST_OVF, ST_FRONTIER, ST_ITEMS, ST_INV,
-                        ST_EDGES_PULL};
-    if (threadIdx.x < 8 && s_acc[threadIdx.x]) atomicAdd(&ctl->stat[idx[threadIdx.x]], s_acc[threadIdx.x]);
+    unsigned k = 0, n, cur = 0, nxt = 1, old = 2;  // the steps' counters rotate
+    for (;; k++) {
+        n = min(s_qcnt[cur], kQueue);
+        if (n == 0 || k >= steps_max || s_stop) break;
+        if (n > limit && k > 0) {  // too much for this CTA: everybody's work is dealt out again
+            if (threadIdx.x == 0) atomicExch(&ctl->rstop[slot], 1u);
+            break;
+        }
+        if (threadIdx.x == 0) s_qcnt[old] = 0;  // read by every thread before the last barrier
+        const unsigned stop = threadIdx.x == blockDim.x - 1 ? __ldcg(&ctl->rstop[slot]) : 0u;
+        for (unsigned b = (threadIdx.x & ~31u) >> 2; b < n; b += per) {  // warp-uniform
+            const unsigned i = b + (lane >> 2);
+            st.visit(i < n ? queue_at(k & 1, i) : make_uint4(0, 0, 0, 0), (k + 1) & 1, &s_qcnt[nxt]);
+        }
+        if (stop) s_stop = 1;
+        const unsigned t = old;
+        old = cur;
+        cur = nxt;
+        nxt = t;
+        __syncthreads();
+    }
+    st.flush_far();
+    for (unsigned b = threadIdx.x & ~31u; b < n; b += blockDim.x) {
+        const uint4 x = b + lane < n ? queue_at(k & 1, b + lane) : make_uint4(0, 0, 0, 0);
+        const bool has = (x.w >> 8) != 0;
+        RowDesc rd;
+        const bool won = claim_with_row(p, has, x.x, st.tag, rd);  // the whole row, once
+        st.spill(won, x.x, rd);
+    }
+    st.pb.flush_cta(p, st.out, st.ls);
+    if (threadIdx.x == 0 && k) atomicMax(&ctl->rsteps[slot], k);
+    keep_stats(st.ls);
 }
 
 __device__ void block_max(unsigned long long* dst, unsigned long long x) {
@@ -798,6 +1010,271 @@ __device__ void block_max(unsigned long long* dst, unsigned long long x) {
     if (lane_id() == 0 && x) atomicMax(&s_max, x);
     __syncthreads();
     if (threadIdx.x == 0 && s_max) atomicMax(dst, s_max);
+}
+
+// Adds a phase's counters to the CTA's (whole warps).
+__device__ __forceinline__ void keep_stats(const LocalStats& ls) {
+    const unsigned v[8] = {ls.edges_relax, ls.edges_inv, ls.updates, ls.dist_ovf,
+                           ls.frontier, ls.items, ls.marked, ls.edges_pull};
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const unsigned x = __reduce_add_sync(kFull, v[q]);
+        if (lane_id() == 0 && x) atomicAdd(&s_lstat[q], (unsigned long long)x);
+    }
+}
+
+// Near-far: the near frontier is empty, nfar vertices wait in list cf.  Moves the threshold on and
+// splits the list into list r (near) and the other far list (generation fgen + 1).  The next
+// threshold is one width on; with `least`, it is the least waiting distance plus the width, which
+// takes a pass and a barrier more.  Returns the new threshold, 0 when nothing waits or the kernel
+// must stop; the sizes of list r are left in s_near.
+__device__ __noinline__ unsigned long long far_advance(const UpdParams& p, unsigned r, unsigned nfar, unsigned rbase,
+                                                       unsigned adv, unsigned long long T, bool least) {
+    const int cf = (int)(adv & 1u);  // the list that is split; generations and lists follow the advances
+    const unsigned fgen = rbase + adv;
+    Ctl* const ctl = p.g.ctl;
+    const DevGraph& g = p.g;
+    const unsigned lane = lane_id(), gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+    const unsigned* fl = cf ? g.far1 : g.far0;
+    unsigned long long tn = T + p.delta;
+    if (least) {
+        unsigned long long mn = ~0ull;
+        for (unsigned i = gtid; i < nfar; i += nthreads) {
+            const unsigned long long d = __ldcg(&g.state[__ldcg(&fl[i])]) >> 32;
+            if (d >= T && d < mn) mn = d;  // below T: settled by an earlier near phase
+        }
+        block_max(&ctl->fmin, ~mn);  // max of ~d = min of d; 0 = nothing waits
+        if (!grid_sync(ctl)) return 0;
+        const unsigned long long fm = __ldcg(&ctl->fmin);
+        if (fm == 0) return 0;
+        tn = ~fm + p.delta;
+    }
+    const Far nxt{cf ? g.far0 : g.far1, &ctl->fc[cf ^ 1], g.far_tag, fgen + 1, (unsigned)g.n, tn};
+    const Out near{(r & 1) ? g.rt1 : g.rt0, &ctl->rcT[r % 3], g.tcap, (r & 1) ? g.rc1 : g.rc0, &ctl->rcC[r % 3], g.ccap};
+    const unsigned tagr = rbase + r + 1u;  // the tag of list r
+    PushBuf pb{s_pbuf[threadIdx.x >> 5], 0};
+    LocalStats ls;
+    for (unsigned base = gtid - lane; base < nfar; base += nthreads) {
+        const unsigned i = base + lane;
+        const unsigned v = i < nfar ? __ldcg(&fl[i]) : 0u;
+        const unsigned long long d = i < nfar ? __ldcg(&g.state[v]) >> 32 : 0ull;
+        const bool live = i < nfar && d >= T;
+        far_push(p, nxt, live && d >= tn, v);
+        RowDesc rd;
+        const bool doit = claim_with_row(p, live && d < tn, v, tagr, rd);
+        ls.frontier += doit ? 1 : 0;
+        pb.add(doit, v, rd);
+        pb.flush(p, near, ls);
+    }
+    pb.flush_cta(p, near, ls);
+    keep_stats(ls);
+    unsigned nt, nc;
+    if (!grid_sync(ctl, &ctl->rcT[r % 3], &ctl->rcC[r % 3], nt, nc)) return 0;
+    if (gtid == 0) {  // every CTA has read both
+        ctl->fc[cf] = 0;  // the next advance appends there
+        ctl->fmin = 0;
+    }
+    if (threadIdx.x == 0) {
+        s_near[0] = nt;
+        s_near[1] = nc;
+    }
+    __syncthreads();
+    return tn;
+}
+
+// ---- A. cut-off subtrees (grid-wide) -----------------------------------------------------------
+// Returns
+// the sizes of the lists it and ic, every cut-off vertex's items (~0: the kernel must stop).
+__device__ __forceinline__ unsigned long long walk(const UpdParams& p) {
+    Ctl* const ctl = p.g.ctl;
+    const DevGraph& g = p.g;
+    const unsigned lane = lane_id(), gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+    const bool leader = gtid == 0;
+    uint4* pbuf = s_pbuf[threadIdx.x >> 5];
+    LocalStats ls;
+    // Level L processes items [lo, hi) of the lists it/ic and appends the items of the
+    // vertices it cuts off after hi through the level's own counters lt*[(L+1)%3], so
+    // every CTA derives the same level bounds while faster CTAs already append.
+    const unsigned nroots = __ldcg(&ctl->inv_count);  // written by k_delete
+    {
+        const Out lvl0{g.it, &ctl->ltT[0], g.tcap, g.ic, &ctl->ltC[0], g.ccap};
+        PushBuf pb{pbuf, 0};
+        for (unsigned base = gtid - lane; base < nroots; base += nthreads) {
+            const unsigned i = base + lane;
+            const unsigned v = i < nroots ? __ldcg(&g.invq[i]) : 0u;
+            pb.add(i < nroots, v, row_if(p, i < nroots, v));
+            pb.flush(p, lvl0, ls);
+        }
+        pb.flush_cta(p, lvl0, ls);
+    }
+    if (leader) ls.marked += nroots;
+    unsigned loT = 0, loC = 0, hiT, hiC;
+    if (!grid_sync(ctl, &ctl->ltT[0], &ctl->ltC[0], hiT, hiC)) return ~0ull;
+    int level = 0;
+    bool need_pj = false;
+    for (;;) {
+        if (loT >= hiT && loC >= hiC) break;
+        if (level >= p.bfs_levels) {
+            need_pj = true;
+            break;
+        }
+        if (small_step(hiT - loT, hiC - loC, p.solo_waves)) {
+            // small levels: CTA 0 walks on alone while they stay small; the others wait
+            if (blockIdx.x == 0) {
+                if (threadIdx.x < 6) s_solo_cnt[threadIdx.x / 2][threadIdx.x % 2] = 0;
+                __syncthreads();
+                for (int steps = 0; steps < kSoloSteps; steps++) {
+                    if ((loT >= hiT && loC >= hiC) || level >= p.bfs_levels || !small_step(hiT - loT, hiC - loC, p.solo_waves))
+                        break;
+                    unsigned* cnt = s_solo_cnt[(level + 1) % 3];
+                    if (threadIdx.x == 0) {
+                        s_solo_cnt[(level + 2) % 3][0] = 0;
+                        s_solo_cnt[(level + 2) % 3][1] = 0;
+                    }
+                    MarkOp op{&p, Out{g.it + hiT, &cnt[0], g.tcap - hiT, g.ic + hiC, &cnt[1], g.ccap - hiC},
+                              PushBuf{pbuf, 0}, &ls};
+                    run_items(op, p, g.it + loT, hiT - loT, g.ic + loC, hiC - loC, 0, 1);
+                    __syncthreads();
+                    loT = hiT;
+                    loC = hiC;
+                    hiT += cnt[0];
+                    hiC += cnt[1];
+                    level++;
+                    __syncthreads();  // every thread has read the counters before the next reset
+                }
+                if (threadIdx.x == 0) {
+                    ctl->solo[0] = ((unsigned long long)hiT << 32) | loT;
+                    ctl->solo[1] = ((unsigned long long)hiC << 32) | loC;
+                    ctl->solo[2] = (unsigned long long)level;
+                    ctl->ltT[(level + 1) % 3] = 0;  // the grid's next level appends here
+                    ctl->ltC[(level + 1) % 3] = 0;
+                }
+            }
+            if (!grid_sync(ctl)) return ~0ull;
+            const unsigned long long a = __ldcg(&ctl->solo[0]), b = __ldcg(&ctl->solo[1]);
+            loT = (unsigned)a;
+            hiT = (unsigned)(a >> 32);
+            loC = (unsigned)b;
+            hiC = (unsigned)(b >> 32);
+            level = (int)__ldcg(&ctl->solo[2]);
+            continue;
+        }
+        if (leader) {
+            ctl->ltT[(level + 2) % 3] = 0;
+            ctl->ltC[(level + 2) % 3] = 0;
+        }
+        MarkOp op{&p,
+                  Out{g.it + hiT, &ctl->ltT[(level + 1) % 3], g.tcap - hiT, g.ic + hiC, &ctl->ltC[(level + 1) % 3],
+                      g.ccap - hiC},
+                  PushBuf{pbuf, 0}, &ls};
+        run_items(op, p, g.it + loT, hiT - loT, g.ic + loC, hiC - loC, blockIdx.x, gridDim.x);
+        unsigned addT, addC;
+        if (!grid_sync(ctl, &ctl->ltT[(level + 1) % 3], &ctl->ltC[(level + 1) % 3], addT, addC)) return ~0ull;
+        loT = hiT;
+        loC = hiC;
+        hiT += addT;
+        hiC += addC;
+        level++;
+    }
+    if (leader) ctl->stat[ST_LEVELS] = (unsigned long long)level;
+    if (need_pj) {
+        // pointer jumping: jm[v] climbs towards the root until it meets a cut-off vertex
+        // (kTagInv) or the root / an unreachable vertex (kTagOk); O(log depth) passes
+        for (unsigned v = gtid; v < (unsigned)g.n; v += nthreads) {
+            unsigned t;
+            if (__ldcg(&g.inv_tag[v]) == p.epoch) {
+                t = kTagInv;
+            } else {
+                const unsigned par = (unsigned)__ldcg(&g.state[v]);
+                t = (par == v || par == kNone) ? kTagOk : par;  // a root, or unreachable
+            }
+            g.jm[v] = t;
+        }
+        if (!grid_sync(ctl)) return ~0ull;
+        int pass = 0;
+        for (;; pass++) {
+            if (pass >= 64) {
+                if (leader) set_status(ctl, -7 /* BAD_TREE: parent cycle */);
+                grid_sync(ctl);
+                return ~0ull;
+            }
+            if (leader) ctl->pjf[(pass + 1) % 3] = 0;
+            int moving = 0;
+            for (unsigned v = gtid; v < (unsigned)g.n; v += nthreads) {
+                const unsigned j = __ldcg(&g.jm[v]);
+                if (j < kTagInv) {
+                    const unsigned jj = __ldcg(&g.jm[j]);
+                    g.jm[v] = jj;
+                    moving |= jj < kTagInv;
+                }
+            }
+            moving = __syncthreads_or(moving);
+            if (moving && threadIdx.x == 0) atomicOr(&ctl->pjf[pass % 3], 1u);
+            if (!grid_sync(ctl)) return ~0ull;
+            if (__ldcg(&ctl->pjf[pass % 3]) == 0) break;
+        }
+        if (leader) ctl->stat[ST_PJ] = (unsigned long long)(pass + 1);
+        const Out pjo{g.it + hiT, &ctl->pjT, g.tcap - hiT, g.ic + hiC, &ctl->pjC, g.ccap - hiC};
+        PushBuf pb{pbuf, 0};
+        for (unsigned base = gtid - lane; base < (unsigned)g.n; base += nthreads) {
+            const unsigned v = base + lane;
+            bool newinv = false;
+            const bool inv = v < (unsigned)g.n && __ldcg(&g.jm[v]) == kTagInv;
+            if (inv && __ldcg(&g.inv_tag[v]) != p.epoch) {
+                g.inv_tag[v] = p.epoch;
+                newinv = true;
+            }
+            // also the roots: one that an insertion re-parented may hold a distance
+            // through a cut-off vertex (the pull gives it its best live value again)
+            if (inv) g.state[v] = kInfState;
+            ls.marked += newinv ? 1 : 0;
+            pb.add(newinv, v, row_if(p, newinv, v));
+            pb.flush(p, pjo, ls);
+        }
+        pb.flush_cta(p, pjo, ls);
+        if (!grid_sync(ctl)) return ~0ull;
+        hiT += __ldcg(&ctl->pjT);
+        hiC += __ldcg(&ctl->pjC);
+    }
+    keep_stats(ls);
+    return ((unsigned long long)hiC << 32) | hiT;
+}
+
+// ---- B. the seeds of k_append become work items; cut-off vertices pull their best live neighbour ----
+__device__ __forceinline__ void seed_and_pull(const UpdParams& p, unsigned hiT, unsigned hiC, unsigned rbase,
+                                           unsigned long long T) {
+    Ctl* const ctl = p.g.ctl;
+    const DevGraph& g = p.g;
+    const unsigned lane = lane_id(), gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+    const unsigned tag0 = rbase + 1;
+    const Out relax0{g.rt0, &ctl->rcT[0], g.tcap, g.rc0, &ctl->rcC[0], g.ccap};
+    uint4* pbuf = s_pbuf[threadIdx.x >> 5];
+    LocalStats ls;
+    {
+        const unsigned ns = __ldcg(&ctl->seed_count);
+        PushBuf pb{pbuf, 0};
+        for (unsigned base = gtid - lane; base < ns; base += nthreads) {
+            const unsigned i = base + lane;
+            const unsigned v = i < ns ? __ldcg(&p.seedq[i]) : 0u;
+            pb.add(i < ns, v, row_if(p, i < ns, v));
+            pb.flush(p, relax0, ls);
+        }
+        pb.flush_cta(p, relax0, ls);
+    }
+    {
+        PullOp op{&p, tag0, relax0, PushBuf{pbuf, 0}, &ls, Far{g.far0, &ctl->fc[0], g.far_tag, rbase, (unsigned)g.n, T}, kInfState, false};
+        run_items(op, p, g.it, hiT, g.ic, hiC, blockIdx.x, gridDim.x);
+    }
+    keep_stats(ls);
+}
+
+// The CTA's counters, one atomic each.
+__device__ void flush_stats(Ctl* ctl, const LocalStats& ls) {
+    keep_stats(ls);
+    __syncthreads();
+    const int idx[8] = {ST_EDGES_RELAX, ST_EDGES_INV, ST_UPDATES, ST_DIST_OVF, ST_FRONTIER, ST_ITEMS, ST_INV,
+                        ST_EDGES_PULL};
+    if (threadIdx.x < 8 && s_lstat[threadIdx.x]) atomicAdd(&ctl->stat[idx[threadIdx.x]], s_lstat[threadIdx.x]);
 }
 
 __device__ void block_add(unsigned long long* dst, unsigned long long x) {
@@ -1197,7 +1674,7 @@ __global__ void k_append(UpdParams p) {
 }
 
 template <bool kAgg>
-__device__ void update_body(UpdParams& p);
+__device__ void update_body(const UpdParams& p);
 
 // 3 CTAs of 256 threads per SM: 80 registers a thread without spills.  Every walk level and
 // relaxation round waits on its slowest CTA's chain of dependent accesses, so shorter chains
@@ -1206,7 +1683,8 @@ __device__ void update_body(UpdParams& p);
 // kAgg: warp-aggregated distance offers (opts.warp_agg), compiled as its own kernel so that
 // the default kernel keeps its register allocation.
 template <bool kAgg>
-__global__ void __launch_bounds__(256, 3) k_update(UpdParams p) {
+__global__ void __launch_bounds__(256, 3) k_update(const __grid_constant__ UpdParams p) {
+    if (threadIdx.x < 8) s_lstat[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         s_nbar = 0;
         s_gen = ld_acquire(&p.g.ctl->bar_gen);
@@ -1224,9 +1702,9 @@ __global__ void __launch_bounds__(256, 3) k_update(UpdParams p) {
 }
 
 template <bool kAgg>
-__device__ void update_body(UpdParams& p) {
+__device__ void update_body(const UpdParams& p) {
     Ctl* ctl = p.g.ctl;
-    DevGraph& g = p.g;
+    const DevGraph& g = p.g;
     __shared__ int s_skip;
     if (threadIdx.x == 0) s_skip = __ldcg(&ctl->status) != 0;  // set before launch: same for every CTA
     __syncthreads();
@@ -1266,11 +1744,10 @@ __device__ void update_body(UpdParams& p) {
     // call's round base).
     const bool nf = p.delta != 0 && g.far0 != nullptr && g.far1 != nullptr && g.far_tag != nullptr;
     unsigned long long T = nf ? (p.mode == 1 ? p.delta : 0ull) : ~0ull;
-    unsigned fgen = rbase;
-    int cf = 0;
-    unsigned adv = 0;
-    auto far_of = [&](int which, unsigned gen, unsigned long long thr) {
-        return Far{which ? g.far1 : g.far0, &ctl->fc[which], g.far_tag, gen, (unsigned)g.n, thr};
+    unsigned adv = 0;     // advances: far list adv & 1 takes this near phase's far pushes, generation rbase + adv
+    bool sparse = false;  // an advance by one width has found nothing
+    auto far_now = [&]() {
+        return Far{(adv & 1) ? g.far1 : g.far0, &ctl->fc[adv & 1], g.far_tag, rbase + adv, (unsigned)g.n, T};
     };
 
     unsigned nT = 0, nC = 0;  // the sizes of the next relaxation round's lists
@@ -1287,245 +1764,81 @@ __device__ void update_body(UpdParams& p) {
         pb.flush_cta(p, relax0, ls);
         if (!grid_sync(ctl, &ctl->rcT[0], &ctl->rcC[0], nT, nC)) return;
     } else {
-        // ---- A. cut-off subtrees ------------------------------------------------------------
-        // Level L processes items [lo, hi) of the lists it/ic and appends the items of the
-        // vertices it cuts off after hi through the level's own counters lt*[(L+1)%3], so
-        // every CTA derives the same level bounds while faster CTAs already append.
-        const unsigned nroots = __ldcg(&ctl->inv_count);  // written by k_delete
-        {
-            const Out lvl0{g.it, &ctl->ltT[0], g.tcap, g.ic, &ctl->ltC[0], g.ccap};
-            PushBuf pb{pbuf, 0};
-            for (unsigned base = gtid - lane; base < nroots; base += nthreads) {
-                const unsigned i = base + lane;
-                const unsigned v = i < nroots ? __ldcg(&g.invq[i]) : 0u;
-                pb.add(i < nroots, v, row_if(p, i < nroots, v));
-                pb.flush(p, lvl0, ls);
-            }
-            pb.flush_cta(p, lvl0, ls);
-        }
-        if (leader) ls.marked += nroots;
-        unsigned loT = 0, loC = 0, hiT, hiC;
-        if (!grid_sync(ctl, &ctl->ltT[0], &ctl->ltC[0], hiT, hiC)) return;
-        int level = 0;
-        bool need_pj = false;
-        for (;;) {
-            if (loT >= hiT && loC >= hiC) break;
-            if (level >= p.bfs_levels) {
-                need_pj = true;
-                break;
-            }
-            if (small_step(hiT - loT, hiC - loC, p.solo_waves)) {
-                // small levels: CTA 0 walks on alone while they stay small; the others wait
-                if (blockIdx.x == 0) {
-                    if (threadIdx.x < 6) s_solo_cnt[threadIdx.x / 2][threadIdx.x % 2] = 0;
-                    __syncthreads();
-                    for (int steps = 0; steps < kSoloSteps; steps++) {
-                        if ((loT >= hiT && loC >= hiC) || level >= p.bfs_levels || !small_step(hiT - loT, hiC - loC, p.solo_waves))
-                            break;
-                        unsigned* cnt = s_solo_cnt[(level + 1) % 3];
-                        if (threadIdx.x == 0) {
-                            s_solo_cnt[(level + 2) % 3][0] = 0;
-                            s_solo_cnt[(level + 2) % 3][1] = 0;
-                        }
-                        MarkOp op{&p, Out{g.it + hiT, &cnt[0], g.tcap - hiT, g.ic + hiC, &cnt[1], g.ccap - hiC},
-                                  PushBuf{pbuf, 0}, &ls};
-                        run_items(op, p, g.it + loT, hiT - loT, g.ic + loC, hiC - loC, 0, 1);
-                        __syncthreads();
-                        loT = hiT;
-                        loC = hiC;
-                        hiT += cnt[0];
-                        hiC += cnt[1];
-                        level++;
-                        __syncthreads();  // every thread has read the counters before the next reset
-                    }
-                    if (threadIdx.x == 0) {
-                        ctl->solo[0] = ((unsigned long long)hiT << 32) | loT;
-                        ctl->solo[1] = ((unsigned long long)hiC << 32) | loC;
-                        ctl->solo[2] = (unsigned long long)level;
-                        ctl->ltT[(level + 1) % 3] = 0;  // the grid's next level appends here
-                        ctl->ltC[(level + 1) % 3] = 0;
-                    }
-                }
-                if (!grid_sync(ctl)) return;
-                const unsigned long long a = __ldcg(&ctl->solo[0]), b = __ldcg(&ctl->solo[1]);
-                loT = (unsigned)a;
-                hiT = (unsigned)(a >> 32);
-                loC = (unsigned)b;
-                hiC = (unsigned)(b >> 32);
-                level = (int)__ldcg(&ctl->solo[2]);
-                continue;
-            }
-            if (leader) {
-                ctl->ltT[(level + 2) % 3] = 0;
-                ctl->ltC[(level + 2) % 3] = 0;
-            }
-            MarkOp op{&p,
-                      Out{g.it + hiT, &ctl->ltT[(level + 1) % 3], g.tcap - hiT, g.ic + hiC, &ctl->ltC[(level + 1) % 3],
-                          g.ccap - hiC},
-                      PushBuf{pbuf, 0}, &ls};
-            run_items(op, p, g.it + loT, hiT - loT, g.ic + loC, hiC - loC, blockIdx.x, gridDim.x);
-            unsigned addT, addC;
-            if (!grid_sync(ctl, &ctl->ltT[(level + 1) % 3], &ctl->ltC[(level + 1) % 3], addT, addC)) return;
-            loT = hiT;
-            loC = hiC;
-            hiT += addT;
-            hiC += addC;
-            level++;
-        }
-        if (leader) ctl->stat[ST_LEVELS] = (unsigned long long)level;
-        if (need_pj) {
-            // pointer jumping: jm[v] climbs towards the root until it meets a cut-off vertex
-            // (kTagInv) or the root / an unreachable vertex (kTagOk); O(log depth) passes
-            for (unsigned v = gtid; v < (unsigned)g.n; v += nthreads) {
-                unsigned t;
-                if (__ldcg(&g.inv_tag[v]) == p.epoch) {
-                    t = kTagInv;
-                } else {
-                    const unsigned par = (unsigned)__ldcg(&g.state[v]);
-                    t = (par == v || par == kNone) ? kTagOk : par;  // a root, or unreachable
-                }
-                g.jm[v] = t;
-            }
-            if (!grid_sync(ctl)) return;
-            int pass = 0;
-            for (;; pass++) {
-                if (pass >= 64) {
-                    if (leader) set_status(ctl, -7 /* BAD_TREE: parent cycle */);
-                    grid_sync(ctl);
-                    return;
-                }
-                if (leader) ctl->pjf[(pass + 1) % 3] = 0;
-                int moving = 0;
-                for (unsigned v = gtid; v < (unsigned)g.n; v += nthreads) {
-                    const unsigned j = __ldcg(&g.jm[v]);
-                    if (j < kTagInv) {
-                        const unsigned jj = __ldcg(&g.jm[j]);
-                        g.jm[v] = jj;
-                        moving |= jj < kTagInv;
-                    }
-                }
-                moving = __syncthreads_or(moving);
-                if (moving && threadIdx.x == 0) atomicOr(&ctl->pjf[pass % 3], 1u);
-                if (!grid_sync(ctl)) return;
-                if (__ldcg(&ctl->pjf[pass % 3]) == 0) break;
-            }
-            if (leader) ctl->stat[ST_PJ] = (unsigned long long)(pass + 1);
-            const Out pjo{g.it + hiT, &ctl->pjT, g.tcap - hiT, g.ic + hiC, &ctl->pjC, g.ccap - hiC};
-            PushBuf pb{pbuf, 0};
-            for (unsigned base = gtid - lane; base < (unsigned)g.n; base += nthreads) {
-                const unsigned v = base + lane;
-                bool newinv = false;
-                const bool inv = v < (unsigned)g.n && __ldcg(&g.jm[v]) == kTagInv;
-                if (inv && __ldcg(&g.inv_tag[v]) != p.epoch) {
-                    g.inv_tag[v] = p.epoch;
-                    newinv = true;
-                }
-                // also the roots: one that an insertion re-parented may hold a distance
-                // through a cut-off vertex (the pull gives it its best live value again)
-                if (inv) g.state[v] = kInfState;
-                ls.marked += newinv ? 1 : 0;
-                pb.add(newinv, v, row_if(p, newinv, v));
-                pb.flush(p, pjo, ls);
-            }
-            pb.flush_cta(p, pjo, ls);
-            if (!grid_sync(ctl)) return;
-            hiT += __ldcg(&ctl->pjT);
-            hiC += __ldcg(&ctl->pjC);
-        }
+        unsigned hiT, hiC;
+        const unsigned long long ends = walk(p);
+        if (ends == ~0ull) return;
+        hiT = (unsigned)ends;
+        hiC = (unsigned)(ends >> 32);
         if (leader) ctl->ts[1] = globaltimer();
 
-        // ---- B. the seeds of k_append become work items; cut-off vertices pull their best
-        // live neighbour --------------------------------------------------------------------
-        {
-            const unsigned ns = __ldcg(&ctl->seed_count);
-            PushBuf pb{pbuf, 0};
-            for (unsigned base = gtid - lane; base < ns; base += nthreads) {
-                const unsigned i = base + lane;
-                const unsigned v = i < ns ? __ldcg(&p.seedq[i]) : 0u;
-                pb.add(i < ns, v, row_if(p, i < ns, v));
-                pb.flush(p, relax0, ls);
-            }
-            pb.flush_cta(p, relax0, ls);
-        }
-        {
-            PullOp op{&p, tag0, relax0, PushBuf{pbuf, 0}, &ls, far_of(cf, fgen, T), kInfState, false};
-            run_items(op, p, g.it, hiT, g.ic, hiC, blockIdx.x, gridDim.x);
-        }
+        seed_and_pull(p, hiT, hiC, rbase, T);
         if (!grid_sync(ctl, &ctl->rcT[0], &ctl->rcC[0], nT, nC)) return;
     }
     if (leader) ctl->ts[2] = globaltimer();
 
     // ---- C. relaxation rounds ---------------------------------------------------------------
-    long long r = 0;
+    // r counts the lists (a round or a local stretch each), hops the rounds and the steps of
+    // the stretches: the depth of the dependent relaxations
+    unsigned r = 0, hops = 0;
     for (;; r++) {
         // nT, nC: the sizes of round r's lists (read at the barrier before)
         if (nT == 0 && nC == 0) {
             if (!nf) break;
             // near frontier empty: advance the threshold past the least waiting distance
-            const unsigned nfar = __ldcg(&ctl->fc[cf]);
+            const unsigned nfar = __ldcg(&ctl->fc[adv & 1]);
             if (nfar == 0) break;
-            const unsigned* fl = cf ? g.far1 : g.far0;
-            unsigned long long mn = ~0ull;
-            for (unsigned i = gtid; i < nfar; i += nthreads) {
-                const unsigned long long d = __ldcg(&g.state[__ldcg(&fl[i])]) >> 32;
-                if (d >= T && d < mn) mn = d;  // below T: settled by an earlier near phase
-            }
-            block_max(&ctl->fmin[adv & 1], ~mn);  // max of ~d = min of d; 0 = nothing waits
-            if (leader) {
-                ctl->fmin[(adv + 1) & 1] = 0;  // read by every CTA before the last barrier
-                ctl->fc[cf ^ 1] = 0;           // the previous advance's source list
-            }
-            if (!grid_sync(ctl)) break;
-            const unsigned long long fm = __ldcg(&ctl->fmin[adv & 1]);
-            if (fm == 0) break;
-            const unsigned long long tn = ~fm + p.delta;
-            const Far nxt = far_of(cf ^ 1, fgen + 1, tn);
-            const Out near{(r & 1) ? g.rt1 : g.rt0, &ctl->rcT[r % 3], g.tcap, (r & 1) ? g.rc1 : g.rc0,
-                           &ctl->rcC[r % 3], g.ccap};
-            const unsigned tagr = rbase + (unsigned)r + 1u;  // the tag of round r's list
-            PushBuf pb{pbuf, 0};
-            for (unsigned base = gtid - lane; base < nfar; base += nthreads) {
-                const unsigned i = base + lane;
-                const unsigned v = i < nfar ? __ldcg(&fl[i]) : 0u;
-                const unsigned long long d = i < nfar ? __ldcg(&g.state[v]) >> 32 : 0ull;
-                const bool live = i < nfar && d >= T;
-                far_push(p, nxt, live && d >= tn, v);
-                RowDesc rd;
-                const bool doit = claim_with_row(p, live && d < tn, v, tagr, rd);
-                ls.frontier += doit ? 1 : 0;
-                pb.add(doit, v, rd);
-                pb.flush(p, near, ls);
-            }
-            pb.flush_cta(p, near, ls);
+            const bool least = T == 0 || sparse;
+            const unsigned long long tn = far_advance(p, r, nfar, rbase, adv, T, least);
+            if (tn == 0) break;
             T = tn;
-            fgen++;
-            cf ^= 1;
             adv++;
-            if (!grid_sync(ctl, &ctl->rcT[r % 3], &ctl->rcC[r % 3], nT, nC)) break;
+            nT = s_near[0];
+            nC = s_near[1];
+            if (!least && nT == 0 && nC == 0) {  // nothing within one width: look for the least
+                sparse = true;
+                r--;
+                continue;
+            }
         }
-        if (r >= p.max_rounds) {
+        if (hops >= p.max_rounds) {
             if (leader) set_status(ctl, -5 /* NO_CONVERGENCE */);
             break;
+        }
+        if (!kAgg && local_step(p, nT, nC)) {
+            if (leader) {
+                ctl->rcT[(r + 2) % 3] = 0;
+                ctl->rcC[(r + 2) % 3] = 0;
+                ctl->rsteps[(r + 2) % 3] = 0;
+                ctl->rstop[(r + 2) % 3] = 0;
+            }
+            const long long left = p.max_rounds - hops;
+            relax_local(p, r, nT, left < (long long)kStretch ? (unsigned)left : kStretch, rbase, adv, T);
+            unsigned t2, used;
+            if (!grid_sync(ctl, &ctl->rcT[(r + 1) % 3], &ctl->rcC[(r + 1) % 3], t2, nC, &ctl->rsteps[(r + 1) % 3], used))
+                break;
+            nT = t2;
+            hops += used;
+            continue;
         }
         if (small_step(nT, nC, p.solo_waves)) {
             // small rounds: CTA 0 relaxes on alone while they stay small; the others wait.  An
             // empty frontier goes back to the grid (near-far advance or the end).
             if (blockIdx.x == 0) {
-                long long rr = r;
+                unsigned rr = r;
                 unsigned t = nT, c = nC;
                 if (threadIdx.x < 6) s_solo_cnt[threadIdx.x / 2][threadIdx.x % 2] = 0;
                 __syncthreads();
                 for (int steps = 0; steps < kSoloSteps; steps++) {
-                    if ((t == 0 && c == 0) || !small_step(t, c, p.solo_waves) || rr >= p.max_rounds) break;
+                    if ((t == 0 && c == 0) || !small_step(t, c, p.solo_waves) || hops + (rr - r) >= p.max_rounds) break;
                     unsigned* cnt = s_solo_cnt[(rr + 1) % 3];
                     if (threadIdx.x == 0) {
                         s_solo_cnt[(rr + 2) % 3][0] = 0;
                         s_solo_cnt[(rr + 2) % 3][1] = 0;
                     }
                     const bool odd = (rr & 1) != 0;
-                    RelaxOp<kAgg> op{&p, rbase + (unsigned)rr + 2u,
+                    RelaxOp<kAgg> op{&p, rbase + rr + 2u,
                                Out{odd ? g.rt0 : g.rt1, &cnt[0], g.tcap, odd ? g.rc0 : g.rc1, &cnt[1], g.ccap},
-                               PushBuf{pbuf, 0}, &ls, far_of(cf, fgen, T), true};
+                               PushBuf{pbuf, 0}, &ls, far_now(), true};
                     run_items(op, p, odd ? g.rt1 : g.rt0, t, odd ? g.rc1 : g.rc0, c, 0, 1);
                     __syncthreads();
                     rr++;
@@ -1541,10 +1854,14 @@ __device__ void update_body(UpdParams& p) {
                     ctl->rcC[rr % 3] = c;
                     ctl->rcT[(rr + 1) % 3] = 0;  // the grid's round rr appends here
                     ctl->rcC[(rr + 1) % 3] = 0;
+                    ctl->rsteps[(rr + 1) % 3] = 0;
+                    ctl->rstop[(rr + 1) % 3] = 0;
                 }
             }
             if (!grid_sync(ctl, &ctl->solo_n[0], &ctl->solo_n[1], nT, nC)) break;
-            r = (long long)__ldcg(&ctl->solo[3]) - 1;  // the loop steps to the first round left
+            const unsigned rr = (unsigned)__ldcg(&ctl->solo[3]);
+            hops += rr - r;
+            r = rr - 1;  // the loop steps to the first round left
             continue;
         }
         if (group_step(p, nT, nC)) {
@@ -1553,19 +1870,19 @@ __device__ void update_body(UpdParams& p) {
             // counters are the grid's, so the hand-over is the same as after solo rounds.
             const unsigned G = p.group_ctas;
             if (blockIdx.x < G) {
-                long long rr = r;
+                unsigned rr = r;
                 unsigned t = nT, c = nC;
                 for (int steps = 0; steps < kSoloSteps; steps++) {
-                    if ((t == 0 && c == 0) || !group_step(p, t, c) || rr >= p.max_rounds) break;
+                    if ((t == 0 && c == 0) || !group_step(p, t, c) || hops + (rr - r) >= p.max_rounds) break;
                     if (blockIdx.x == 0 && threadIdx.x == 0) {
                         ctl->rcT[(rr + 2) % 3] = 0;
                         ctl->rcC[(rr + 2) % 3] = 0;
                     }
                     const bool odd = (rr & 1) != 0;
-                    RelaxOp<kAgg> op{&p, rbase + (unsigned)rr + 2u,
+                    RelaxOp<kAgg> op{&p, rbase + rr + 2u,
                                      Out{odd ? g.rt0 : g.rt1, &ctl->rcT[(rr + 1) % 3], g.tcap, odd ? g.rc0 : g.rc1,
                                          &ctl->rcC[(rr + 1) % 3], g.ccap},
-                                     PushBuf{pbuf, 0}, &ls, far_of(cf, fgen, T),
+                                     PushBuf{pbuf, 0}, &ls, far_now(),
                                      (unsigned long long)t + (unsigned long long)c * blockDim.x <=
                                          (unsigned long long)G * blockDim.x};
                     run_items(op, p, odd ? g.rt1 : g.rt0, t, odd ? g.rc1 : g.rc0, c, blockIdx.x, G);
@@ -1584,30 +1901,37 @@ __device__ void update_body(UpdParams& p) {
                     ctl->rcC[rr % 3] = c;
                     ctl->rcT[(rr + 1) % 3] = 0;  // the grid's round rr appends here
                     ctl->rcC[(rr + 1) % 3] = 0;
+                    ctl->rsteps[(rr + 1) % 3] = 0;
+                    ctl->rstop[(rr + 1) % 3] = 0;
                 }
             }
             if (!grid_sync(ctl, &ctl->solo_n[0], &ctl->solo_n[1], nT, nC)) break;
-            r = (long long)__ldcg(&ctl->solo[3]) - 1;  // the loop steps to the first round left
+            const unsigned rr = (unsigned)__ldcg(&ctl->solo[3]);
+            hops += rr - r;
+            r = rr - 1;  // the loop steps to the first round left
             continue;
         }
         if (leader) {
             ctl->rcT[(r + 2) % 3] = 0;
             ctl->rcC[(r + 2) % 3] = 0;
+            ctl->rsteps[(r + 2) % 3] = 0;
+            ctl->rstop[(r + 2) % 3] = 0;
         }
         const bool odd = (r & 1) != 0;
-        RelaxOp<kAgg> op{&p, rbase + (unsigned)r + 2u,
+        RelaxOp<kAgg> op{&p, rbase + r + 2u,
                    Out{odd ? g.rt0 : g.rt1, &ctl->rcT[(r + 1) % 3], g.tcap, odd ? g.rc0 : g.rc1,
                        &ctl->rcC[(r + 1) % 3], g.ccap},
-                   PushBuf{pbuf, 0}, &ls, far_of(cf, fgen, T),
+                   PushBuf{pbuf, 0}, &ls, far_now(),
                    (unsigned long long)nT + (unsigned long long)nC * blockDim.x <= (unsigned long long)nthreads};
         run_items(op, p, odd ? g.rt1 : g.rt0, nT, odd ? g.rc1 : g.rc0, nC, blockIdx.x, gridDim.x);
         if (!grid_sync(ctl, &ctl->rcT[(r + 1) % 3], &ctl->rcC[(r + 1) % 3], nT, nC)) break;
+        hops++;
     }
     flush_stats(ctl, ls);
     if (leader) {
-        ctl->stat[ST_ROUNDS] = (unsigned long long)r;
+        ctl->stat[ST_ROUNDS] = (unsigned long long)hops;
         ctl->stat[ST_ADVANCES] = (unsigned long long)adv;
-        ctl->round_base = rbase + (unsigned)r + 4u;
+        ctl->round_base = rbase + r + 4u;
         ctl->ts[3] = globaltimer();
     }
 }

@@ -731,3 +731,66 @@ def test_create_with_null_opts_and_edgeless_graph():
         g.tree_compute(0)
         p, d = g.tree_read()
         assert d[0] == 0 and (p[1:] == -1).all()
+
+
+def _combs(deg, spine, wlo, rng):
+    """Two long spines from vertex 0 whose vertices carry leaves up to degree `deg`."""
+    u, v = [], []
+    n = 1
+    for _ in range(2):
+        prev = 0
+        for _ in range(spine):
+            at = n
+            n += 1
+            u.append(prev), v.append(at)
+            for _ in range(deg - 2):
+                u.append(at), v.append(n)
+                n += 1
+            prev = at
+    w = rng.integers(wlo, 40, len(u))
+    return n, np.array(u, np.int32), np.array(v, np.int32), w.astype(np.int32)
+
+
+@pytest.mark.parametrize("wlo", [0, 1])
+@pytest.mark.parametrize("opts", [{}, {"delta": 64}, {"small_deg": 16}, {"small_deg": 20}, {"block": 32},
+                                  {"block": 96, "ctas_per_sm": 1, "small_deg": 8}])
+def test_local_stretches_on_combs(opts, wlo):
+    """Rounds that run in CTA queues: rows at the edges of an item, of the queue's longest row
+    (32 entries) and above, stretches longer than one stretch may be; the tree and a batch that
+    cuts both spines, against the oracle and (positive weights) the rounds' own parents."""
+    rng = np.random.default_rng(7 + wlo)
+    for deg, spine in ((3, 700), (4, 90), (5, 90), (31, 30), (32, 30), (33, 30), (34, 300)):
+        n, u, v, w = _combs(deg, spine, wlo, rng)
+        ch = D.gen_changes(n, u, v, w, 40, 40, seed=deg)
+        near = np.flatnonzero((u == 0) | (v == 0))[:1]
+        cut = D.make_changes(u[near], v[near], w[near], np.zeros(len(near)))
+        ch = np.concatenate([ch, cut])
+        got = []
+        for extra in ({}, {"group_ctas": 2, "solo_waves": 0}):  # local stretches; rounds only
+            with D.Graph(n, u, v, w, **{**opts, **extra}) as g:
+                g.tree_compute(0)
+                p0, d0 = g.tree_read()
+                check_against_oracle(n, u, v, w, None, 0, p0, d0, f"tree, deg {deg}")
+                g.apply_batch(ch)
+                p1, d1 = g.tree_read()
+                check_against_oracle(n, u, v, w, ch, 0, p1, d1, f"batch, deg {deg}")
+                got.append((p0, p1))
+        if wlo:
+            assert all(np.array_equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("leaves", [29183, 29184, 29185, 60000])
+def test_local_stretches_around_their_widest_round(leaves):
+    """A star whose leaves go on in chains of three: the frontier is about one item per place of
+    the widest local stretch, one below, one above, and twice that."""
+    hub = np.zeros(leaves, np.int64)
+    a = 1 + np.arange(leaves)
+    u = np.concatenate([hub, a, a + leaves])
+    v = np.concatenate([a, a + leaves, a + 2 * leaves])
+    n = 1 + 3 * leaves
+    w = 1 + (np.arange(len(u)) * 2654435761 % 97)
+    u, v, w = (np.ascontiguousarray(x, np.int32) for x in (u, v, w))
+    with D.Graph(n, u, v, w) as g:
+        g.tree_compute(0)
+        p, d = g.tree_read()
+    check_against_oracle(n, u, v, w, None, 0, p, d, f"{leaves} leaves")
