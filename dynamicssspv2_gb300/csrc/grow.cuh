@@ -1,0 +1,359 @@
+// grow.cuh -- growth of the rows that a batch's insertions overflow, on the device.
+//
+// k_append lists the insertions that found their row full (ovf), and with the first of them the row
+// itself, cut into chunks of kGrowChunk slots.  k_update then starts with the growth: a growing
+// row keeps only its live entries, in their order, so the sorted prefix stays sorted and the
+// tombstones are gone.  When those entries and the overflow fit its own region with an eighth of
+// them (at least one slot) to spare, the row is compacted in place, through scratch slots at the
+// free end of the spare region; otherwise it moves to a region of 2 * (live + overflow) +
+// slack_min slots from the spare region (a bump allocator).  Every moved entry leaves its final
+// slot in its old twin word, through which its partner and the batch's recorded slots find it.
+// The first four phases write only free slots, twin words and the work arrays: until the last
+// one (grow_finish) the rows stand as k_append left them, and grow_finish may be run again.
+//
+// A warp per chunk, not per row: rows of 10^5 entries grow in a stream on a skewed graph, and a warp
+// that walked one alone took up to 2 ms (RMAT scale 22, 10^6 changes a batch).  Inside k_update,
+// not as kernels of its own: with the host between them (status read, eight launches, three
+// synchronisations) a growth of a dozen rows took 0.11 ms.  A dozen rows are grown by one
+// CTA with block barriers.
+#pragma once
+
+// Chunks a row of `cap` slots is cut into (at least one: a row without slots grows too).
+__device__ __forceinline__ unsigned grow_chunks(int cap) {
+    return cap > 0 ? ((unsigned)cap + kGrowChunk - 1) / kGrowChunk : 1u;
+}
+
+// k_append: lists row r, entry j of the grow list, with its chunks from c0 on.
+__device__ __forceinline__ void grow_list_row(const UpdParams& p, unsigned j, unsigned c0, int r, unsigned chunks) {
+    p.grow.row[j] = (unsigned)r;
+    p.grow.chunk0[j] = c0;
+    p.grow.done[j] = 0;
+    p.grow.lsorted[j] = 0;
+    p.grow.gidx[r] = (int)j + 1;
+    for (unsigned q = 0; q < chunks; q++) p.grow.chunk_row[c0 + q] = j;
+}
+
+// k_append, warp-collective: lists the ends of record i (c) that found their rows (rx, ry) full
+// (ovx, ovy; px, py are the positions they were given), with one atomic per warp and list, and
+// the record's slots (ax, ay), -1 - k for the k-th overflowed end of its row.
+__device__ __forceinline__ void list_overflow(const UpdParams& p, long long i, const int4& c, const RowDesc& rx,
+                                              const RowDesc& ry, int px, int py, bool ovx, bool ovy, long long ax,
+                                              long long ay) {
+    const unsigned lane = lane_id(), lt = (1u << lane) - 1u;
+    const unsigned mx = __ballot_sync(kFull, ovx), my = __ballot_sync(kFull, ovy);
+    if ((mx | my) == 0) return;
+    unsigned base = 0;
+    if (lane == 0) base = (unsigned)atomicAdd(&p.g.ctl->ovf_count, __popc(mx) + __popc(my));
+    base = __shfl_sync(kFull, base, 0);
+    if (ovx) p.ovf[base + __popc(mx & lt)] = make_int4(c.x, c.y, c.z, (int)(2 * i));
+    if (ovy) p.ovf[base + __popc(mx) + __popc(my & lt)] = make_int4(c.y, c.x, c.z, (int)(2 * i + 1));
+    if (ovx || ovy) {
+        p.slot[2 * i] = ovx ? -1ll - (px - rx.cap) : ax;
+        p.slot[2 * i + 1] = ovy ? -1ll - (py - ry.cap) : ay;
+    }
+    const bool fx = ovx && px == rx.cap, fy = ovy && py == ry.cap;  // the first of its row
+    if (!__any_sync(kFull, fx || fy)) return;
+    const unsigned nx = fx ? grow_chunks(rx.cap) : 0u, ny = fy ? grow_chunks(ry.cap) : 0u;
+    const unsigned nr = (fx ? 1u : 0u) + (fy ? 1u : 0u);
+    const unsigned ir = warp_incl_scan(nr), ic = warp_incl_scan(nx + ny);
+    unsigned long long at = 0;
+    if (lane == 31) at = atomicAdd(&p.g.ctl->grow_list, ((unsigned long long)ic << 32) | ir);
+    at = __shfl_sync(kFull, at, 31);
+    unsigned j = (unsigned)at + ir - nr, ch = (unsigned)(at >> 32) + ic - (nx + ny);
+    if (fx) {
+        grow_list_row(p, j, ch, c.x, nx);
+        j++;
+        ch += nx;
+    }
+    if (fy) grow_list_row(p, j, ch, c.y, ny);
+}
+
+// Everything a growth phase reads may have been written in this kernel by another SM, and the
+// rows it reads are written by the last one: all through the L2.
+__device__ __forceinline__ RowDesc ld_row(const RowDesc* r) {
+    const uint4 x = __ldcg(reinterpret_cast<const uint4*>(r));
+    return RowDesc{(long long)(((unsigned long long)x.y << 32) | x.x), (int)x.z, (int)x.w};
+}
+
+// The threads that take part in a growth: the grid, or one CTA of it.
+struct GrowTeam {
+    unsigned thread, threads;
+    __device__ __forceinline__ unsigned warp() const { return thread >> 5; }
+    __device__ __forceinline__ unsigned warps() const { return threads >> 5; }
+};
+
+// Phase 1: live entries of every chunk; the warp that counts a row's last chunk ranks them and
+// decides where the row goes.
+__device__ void grow_plan(const UpdParams& p, const GrowTeam& t, unsigned chunks) {
+    const DevGrow& q = p.grow;
+    const unsigned lane = lane_id();
+    unsigned dropped = 0;
+    for (unsigned c = t.warp(); c < chunks; c += t.warps()) {
+        const unsigned j = __ldcg(&q.chunk_row[c]);
+        const unsigned r = __ldcg(&q.row[j]), c0 = __ldcg(&q.chunk0[j]);
+        const RowDesc rd = ld_row(&p.g.rows[r]);
+        const int sl = __ldcg(&p.g.sorted_len[r]);
+        const int lo = (int)(c - c0) * kGrowChunk, hi = min(lo + kGrowChunk, rd.cap);
+        unsigned n = 0, ns = 0;
+#pragma unroll
+        for (int k = 0; k < kGrowChunk / 32; k++) {
+            const int e = lo + 32 * k + (int)lane;
+            const bool live = e < hi && __ldcg(&p.g.adj[rd.start + e].y) >= 0;
+            n += live ? 1u : 0u;
+            ns += live && e < sl ? 1u : 0u;
+        }
+        n = __reduce_add_sync(kFull, n);
+        ns = __reduce_add_sync(kFull, ns);
+        const unsigned parts = grow_chunks(rd.cap);
+        unsigned total = n;
+        if (lane == 0) q.chunk_live[c] = (int)n;
+        if (parts == 1) {
+            if (lane == 0) {
+                q.chunk_off[c] = 0;
+                q.lsorted[j] = (int)ns;
+            }
+        } else {
+            unsigned d = 0;
+            if (lane == 0) {
+                atomicAdd(&q.lsorted[j], (int)ns);
+                __threadfence();
+                d = atomicAdd(&q.done[j], 1u);
+            }
+            if (__shfl_sync(kFull, d, 0) != parts - 1) continue;
+            __threadfence();
+            total = 0;
+            for (unsigned b = 0; b < parts; b += 32) {
+                const unsigned x = b + lane < parts ? (unsigned)__ldcg(&q.chunk_live[c0 + b + lane]) : 0u;
+                const unsigned incl = warp_incl_scan(x);
+                if (b + lane < parts) q.chunk_off[c0 + b + lane] = (int)(total + incl - x);
+                total += __shfl_sync(kFull, incl, 31);
+            }
+        }
+        if (lane != 0) continue;
+        const long long live = total, need = rd.deg - rd.cap;
+        const long long room = live / 8 > 1 ? live / 8 : 1;  // free slots left after an in-place compaction
+        dropped += (unsigned)(rd.cap - live);
+        q.live[j] = (int)live;
+        if (live + need + room <= rd.cap) {
+            const unsigned long long at = atomicAdd(&p.g.ctl->scr_used, (unsigned long long)live);
+            q.fin[j] = rd.start;
+            q.scr[j] = (long long)(__ldcg(&q.spare[1]) - at - (unsigned long long)live);  // checked by grow()
+            q.ncap[j] = rd.cap;
+        } else {
+            const long long nc = 2 * (live + need) + q.slack_min;
+            if (nc > 0x7FFFFFFFLL) atomicExch(&p.g.ctl->grow_fail, 1u);
+            q.fin[j] = (long long)atomicAdd(&q.spare[0], (unsigned long long)nc);
+            q.scr[j] = -1;
+            q.ncap[j] = (int)(nc > 0x7FFFFFFFLL ? 0x7FFFFFFFLL : nc);
+        }
+        q.ndeg[j] = (int)(live + need);
+    }
+    if (lane == 0 && dropped) atomicAdd(&p.g.ctl->grow_dropped, (unsigned long long)dropped);
+}
+
+// Phase 2: the live entries to where their row goes (or its scratch), a forwarding pointer in
+// each one's old twin word.
+__device__ void grow_out(const UpdParams& p, const GrowTeam& t, unsigned chunks) {
+    const DevGrow& q = p.grow;
+    const unsigned lane = lane_id(), lt = (1u << lane) - 1u;
+    for (unsigned c = t.warp(); c < chunks; c += t.warps()) {
+        const unsigned j = __ldcg(&q.chunk_row[c]);
+        const RowDesc rd = ld_row(&p.g.rows[__ldcg(&q.row[j])]);
+        const int lo = (int)(c - __ldcg(&q.chunk0[j])) * kGrowChunk, hi = min(lo + kGrowChunk, rd.cap);
+        const long long off = __ldcg(&q.chunk_off[c]), fin = __ldcg(&q.fin[j]) + off, scr = __ldcg(&q.scr[j]);
+        const long long dst = scr >= 0 ? scr + off : fin;
+        int idx = 0;
+        for (int b = lo; b < hi; b += 128) {
+            int2 x[4];
+            unsigned tw[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int e = b + 32 * k + (int)lane;
+                x[k] = e < hi ? __ldcg(&p.g.adj[rd.start + e]) : make_int2(0, -1);
+                tw[k] = p.g.twin && e < hi ? __ldcg(&p.g.twin[rd.start + e]) : kNoTwin;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const bool live = x[k].y >= 0;
+                const unsigned m = __ballot_sync(kFull, live);
+                if (live) {
+                    const int at = idx + __popc(m & lt);
+                    p.g.adj[dst + at] = x[k];
+                    if (p.g.twin) {
+                        p.g.twin[dst + at] = tw[k];  // the partner's old slot, re-linked by the next phase
+                        p.g.twin[rd.start + b + 32 * k + (int)lane] = (unsigned)(fin + at);
+                    }
+                }
+                idx += __popc(m);
+            }
+        }
+    }
+}
+
+// Phase 3: every moved entry takes its partner's final slot, from the partner's forwarding pointer
+// when the partner's row grows too; else the partner stays and gets this entry's final slot.
+__device__ void grow_relink(const UpdParams& p, const GrowTeam& t, unsigned chunks) {
+    const DevGrow& q = p.grow;
+    const unsigned lane = lane_id();
+    for (unsigned c = t.warp(); c < chunks; c += t.warps()) {
+        const unsigned j = __ldcg(&q.chunk_row[c]);
+        const int live = __ldcg(&q.chunk_live[c]);
+        const long long off = __ldcg(&q.chunk_off[c]), fin = __ldcg(&q.fin[j]) + off, scr = __ldcg(&q.scr[j]);
+        const long long at0 = scr >= 0 ? scr + off : fin;
+        for (int b = 0; b < live; b += 128) {
+            unsigned tw[4];
+            int gi[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int e = b + 32 * k + (int)lane;
+                tw[k] = e < live ? __ldcg(&p.g.twin[at0 + e]) : kNoTwin;
+                gi[k] = e < live ? __ldcg(&q.gidx[__ldcg(&p.g.adj[at0 + e].x)]) : 0;
+                if (tw[k] != kNoTwin && (long long)tw[k] >= p.g.cap_total) {  // internal error: report, skip
+                    set_status(p.g.ctl, -4);
+                    tw[k] = kNoTwin;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int e = b + 32 * k + (int)lane;
+                if (tw[k] == kNoTwin) continue;
+                if (gi[k]) p.g.twin[at0 + e] = __ldcg(&p.g.twin[tw[k]]);
+                else p.g.twin[tw[k]] = (unsigned)(fin + e);
+            }
+        }
+    }
+}
+
+// Phase 4: the final slot of every overflowed end and of its partner, which is told at once when
+// it did fit (it lies where phase 2 left it).
+__device__ void grow_place(const UpdParams& p, const GrowTeam& t, unsigned novf) {
+    const DevGrow& q = p.grow;
+    for (unsigned o = t.thread; o < novf; o += t.threads) {
+        const int4 x = __ldcg(&p.ovf[o]);  // row, column, weight, 2 * record + side
+        const unsigned s = (unsigned)x.w;
+        const long long raw = __ldcg(&p.slot[s]), praw = __ldcg(&p.slot[s ^ 1u]);
+        const unsigned j = (unsigned)__ldcg(&q.gidx[x.x]) - 1u;
+        const long long own = __ldcg(&q.fin[j]) + __ldcg(&q.live[j]) + (-1 - raw);
+        if (!p.g.twin) {
+            q.place[o] = make_uint2((unsigned)own, (unsigned)((unsigned long long)own >> 32));
+            continue;
+        }
+        const int pj = __ldcg(&q.gidx[x.y]) - 1;
+        long long partner = praw;
+        if (praw < 0) {
+            partner = __ldcg(&q.fin[pj]) + __ldcg(&q.live[pj]) + (-1 - praw);
+        } else {
+            long long cur = praw;
+            if (pj >= 0) {
+                const long long fin = __ldcg(&q.fin[pj]), scr = __ldcg(&q.scr[pj]);
+                partner = __ldcg(&p.g.twin[praw]);
+                cur = scr >= 0 ? scr + (partner - fin) : partner;
+            }
+            if (cur >= 0 && cur < p.g.cap_total) p.g.twin[cur] = (unsigned)own;
+            else set_status(p.g.ctl, -4);  // internal error
+        }
+        q.place[o] = make_uint2((unsigned)own, (unsigned)partner);
+    }
+}
+
+// Phase 5: compacted rows back from their scratch, the overflowed ends behind the live entries, the
+// new descriptors.  Reads only what the phases before it wrote, so it may run again.
+__device__ void grow_finish(const UpdParams& p, const GrowTeam& t, unsigned rows, unsigned chunks, unsigned novf) {
+    const DevGrow& q = p.grow;
+    const unsigned lane = lane_id();
+    for (unsigned c = t.warp(); c < chunks; c += t.warps()) {
+        const unsigned j = __ldcg(&q.chunk_row[c]);
+        const long long off = __ldcg(&q.chunk_off[c]), fin = __ldcg(&q.fin[j]) + off, scr = __ldcg(&q.scr[j]);
+        if (scr < 0) continue;
+        const int live = __ldcg(&q.chunk_live[c]);
+        for (int e = (int)lane; e < live; e += 32) {
+            p.g.adj[fin + e] = __ldcg(&p.g.adj[scr + off + e]);
+            if (p.g.twin) p.g.twin[fin + e] = __ldcg(&p.g.twin[scr + off + e]);
+        }
+    }
+    for (unsigned o = t.thread; o < novf; o += t.threads) {
+        const int4 x = __ldcg(&p.ovf[o]);
+        const uint2 s = __ldcg(&q.place[o]);
+        const long long own = p.g.twin ? (long long)s.x : (long long)(((unsigned long long)s.y << 32) | s.x);
+        p.g.adj[own] = make_int2(x.y, x.z);
+        if (p.g.twin) p.g.twin[own] = s.y;
+    }
+    for (unsigned j = t.thread; j < rows; j += t.threads) {
+        const unsigned r = __ldcg(&q.row[j]);
+        RowDesc nr;
+        nr.start = __ldcg(&q.fin[j]);
+        nr.deg = __ldcg(&q.ndeg[j]);
+        nr.cap = __ldcg(&q.ncap[j]);
+        p.g.rows[r] = nr;
+        p.g.sorted_len[r] = __ldcg(&q.lsorted[j]);
+        q.gidx[r] = 0;
+    }
+}
+
+// The spare region cannot take the moves and the scratch: nothing has been written, the host
+// repacks (which folds the overflow list in).
+__device__ __forceinline__ bool grow_fits(const UpdParams& p) {
+    return __ldcg(&p.g.ctl->grow_fail) == 0 &&
+           __ldcg(&p.grow.spare[0]) + __ldcg(&p.g.ctl->scr_used) <= __ldcg(&p.grow.spare[1]);
+}
+
+__device__ __forceinline__ void grow_give_up(const UpdParams& p, const GrowTeam& t, unsigned rows) {
+    for (unsigned j = t.thread; j < rows; j += t.threads) p.grow.gidx[__ldcg(&p.grow.row[j])] = 0;
+    if (t.thread == 0) set_status(p.g.ctl, kStatusOverflowPending);
+}
+
+// The whole growth (grid-wide).  Returns false when the kernel must stop.
+__device__ __noinline__ bool grow(const UpdParams& p) {
+    Ctl* const ctl = p.g.ctl;
+    const unsigned novf = (unsigned)__ldcg(&ctl->ovf_count);
+    const unsigned long long list = __ldcg(&ctl->grow_list);
+    const unsigned rows = (unsigned)list, chunks = (unsigned)(list >> 32);
+    if (chunks <= blockDim.x >> 5 && novf <= blockDim.x) {  // one CTA, a chunk a warp
+        if (blockIdx.x == 0) {
+            const GrowTeam t{threadIdx.x, blockDim.x};
+            grow_plan(p, t, chunks);
+            __threadfence();
+            __syncthreads();
+            if (grow_fits(p)) {
+                grow_out(p, t, chunks);
+                __threadfence();
+                __syncthreads();
+                if (p.g.twin) grow_relink(p, t, chunks);
+                __threadfence();
+                __syncthreads();
+                grow_place(p, t, novf);
+                __threadfence();
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    ctl->spare_top = __ldcg(&p.grow.spare[0]);
+                    ctl->grow_done = gridDim.x;
+                }
+                grow_finish(p, t, rows, chunks, novf);
+            } else {
+                grow_give_up(p, t, rows);
+            }
+        }
+        return grid_sync(ctl);
+    }
+    const GrowTeam t{blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x};
+    grow_plan(p, t, chunks);
+    if (!grid_sync(ctl)) return false;
+    if (!grow_fits(p)) {
+        grow_give_up(p, t, rows);
+        return false;
+    }
+    grow_out(p, t, chunks);
+    if (!grid_sync(ctl)) return false;
+    if (p.g.twin) grow_relink(p, t, chunks);
+    if (!grid_sync(ctl)) return false;
+    grow_place(p, t, novf);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (blockIdx.x == 0) ctl->spare_top = __ldcg(&p.grow.spare[0]);
+        __threadfence();
+        atomicAdd(&ctl->grow_done, 1u);  // every CTA's: the last phase may run (or be run again)
+    }
+    if (!grid_sync(ctl)) return false;
+    grow_finish(p, t, rows, chunks, novf);
+    return grid_sync(ctl);
+}

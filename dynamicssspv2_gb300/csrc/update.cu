@@ -1467,6 +1467,7 @@ constexpr int kTailList = 32;
 struct LongTail {
     long long lo, hi;
     int col, w;
+    bool twin;
 };
 __shared__ LongTail s_tails[kMaxWarps][kTailList];
 __shared__ unsigned s_ntails[kMaxWarps];
@@ -1539,14 +1540,18 @@ __global__ void k_delete(UpdParams p) {
                 const RowDesc& rs = use_a ? ra : rb;
                 const int sl = p.g.sorted_len[use_a ? a : b];
                 const int col = (int)(use_a ? b : a);
+                // a self-loop's two entries lie in the one row: the search meets both, each is
+                // counted by its own compare-and-swap (by the other's twin store as well, a loop
+                // deleted by two records of a batch was counted twice)
+                const bool tw = a != b;
                 if (!kTails || rs.deg - sl <= kCoopTail) {  // a short unsorted tail: this lane scans it too
-                    probed += tombstone_row(p, rs, sl, col, c.z, true, dead);
+                    probed += tombstone_row(p, rs, sl, col, c.z, tw, dead);
                 } else {  // a long one goes to the warp's list (or, when that is full, to this lane)
                     long long tlo, thi;
-                    probed += tombstone_prefix(p, rs, sl, col, c.z, true, dead, tlo, thi);
+                    probed += tombstone_prefix(p, rs, sl, col, c.z, tw, dead, tlo, thi);
                     const unsigned at = atomicAdd(&s_ntails[warp], 1u);
-                    if (at < (unsigned)kTailList) s_tails[warp][at] = LongTail{tlo, thi, col, c.z};
-                    else probed += tombstone_tail(p, tlo, thi, col, c.z, true, dead);
+                    if (at < (unsigned)kTailList) s_tails[warp][at] = LongTail{tlo, thi, col, c.z, tw};
+                    else probed += tombstone_tail(p, tlo, thi, col, c.z, tw, dead);
                 }
             } else {
                 probed += tombstone_row(p, ra, p.g.sorted_len[a], (int)b, c.z, false, dead);
@@ -1565,7 +1570,7 @@ __global__ void k_delete(UpdParams p) {
             const LongTail lt = s_tails[warp][t];
             for (long long j = lt.lo + lane; j < lt.hi; j += 32) {
                 const int2 e = p.g.adj[j];
-                if (e.x == lt.col && e.y == lt.w) dead += tombstone_at(p, j, lt.w, true);
+                if (e.x == lt.col && e.y == lt.w) dead += tombstone_at(p, j, lt.w, lt.twin);
             }
             if (lane == 0) probed += (unsigned long long)(lt.hi - lt.lo);
         }

@@ -794,3 +794,21 @@ def test_local_stretches_around_their_widest_round(leaves):
         g.tree_compute(0)
         p, d = g.tree_read()
     check_against_oracle(n, u, v, w, None, 0, p, d, f"{leaves} leaves")
+
+
+def test_a_self_loop_deleted_by_many_records_is_counted_once():
+    """Self-loops among which many are one line repeated, each deleted by many records of one
+    batch: the live count afterwards is exact (every entry is tombstoned and counted once)."""
+    n = 400
+    loops = np.repeat(np.arange(n), 8)
+    u = np.concatenate([np.arange(n - 1), loops]).astype(np.int32)
+    v = np.concatenate([np.arange(1, n), loops]).astype(np.int32)
+    w = np.concatenate([np.full(n - 1, 3), np.full(len(loops), 5)]).astype(np.int32)
+    many = np.repeat(np.arange(n), 16)
+    ch = D.make_changes(many, many, np.full(len(many), 5), np.zeros(len(many)))
+    for _ in range(5):
+        with D.Graph(n, u, v, w) as g:
+            g.tree_compute(0)
+            st = g.apply_batch(ch)
+            assert st.tombstoned == 2 * len(loops)
+            assert g.health()["live"] == 2 * (n - 1) and g.validate()["violations"] == 0
