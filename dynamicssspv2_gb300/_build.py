@@ -31,7 +31,7 @@ CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-fopenmp", "-Wall", "-Wno-unused-fun
 
 CUDA_UNITS = ["update.cu", "graph.cu", "noalloc.cu"]
 HOST_UNITS = ["gen.cpp", "textio.cpp", "binio.cpp", "serve.cpp", "autotune.cpp"]
-HEADERS = ["engine.cuh", "host_common.h"]
+HEADERS = ["engine.cuh", "grow.cuh", "host_common.h"]
 
 
 def _nvcc() -> str:

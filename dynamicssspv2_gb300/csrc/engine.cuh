@@ -32,7 +32,8 @@ constexpr unsigned kNone = 0xFFFFFFFFu;
 constexpr unsigned long long kDistInf = 0xFFFFFFFFull;
 constexpr unsigned kTagOk = 0xFFFFFFFFu;   // pointer jumping: reaches the root untouched
 constexpr unsigned kTagInv = 0xFFFFFFFEu;  // pointer jumping: below a cut-off vertex
-constexpr int kStatusOverflowPending = 1;  // internal: an insertion did not fit its row
+constexpr int kStatusOverflowPending = 1;  // internal: the spare region cannot take the growing rows
+constexpr int kGrowChunk = 256;            // slots of a growing row that one warp handles
 constexpr unsigned kNoTwin = 0xFFFFFFFFu;   // twin not known yet (the other end overflowed)
 constexpr unsigned long long kHashEmpty = 0xFFFFFFFFFFFFFFFFull;
 constexpr int kHashNoWeight = -1;  // 0xFF byte fill; deletions with w < 0 are not hashed
@@ -87,11 +88,17 @@ struct __align__(128) Ctl {
     unsigned pad0[27];
     // line 1
     int status;
-    int ovf_count;
+    int ovf_count;       // ends of insertions that found their row full
     unsigned inv_count;  // roots appended by k_delete
     unsigned killed;     // insertions removed by a deletion of the same batch
     unsigned seed_count;  // vertices k_append seeded into the first frontier
-    unsigned pad1[27];
+    unsigned grow_fail;   // row growth: a row of more than 2^31 slots
+    unsigned long long grow_list;     // growing rows (low word) and their chunks (high word)
+    unsigned long long scr_used;      // scratch slots taken from the free end of the spare region
+    unsigned long long grow_dropped;  // tombstones dropped
+    unsigned long long spare_top;     // the spare region's bump pointer after the growth (0: none)
+    unsigned grow_done;   // CTAs past the growth's last phase but one (all: that phase has run or may)
+    unsigned pad1[17];
     // line 2
     unsigned bar_count;
     unsigned pad2[31];
@@ -168,15 +175,35 @@ struct DevGraph {
     int src;  // lowest root (informational; kernels treat any vertex that is its own parent as a root)
 };
 
+// Work arrays of a batch's row growth: per growing row, per chunk of one, per overflowed end.
+struct DevGrow {
+    unsigned* row;         // the vertex
+    unsigned* chunk0;      // its first chunk
+    unsigned* done;        // chunks counted
+    int* live;             // live entries
+    int* lsorted;          // ... of them in the neighbour-sorted prefix
+    int* ndeg;             // degree and capacity after the growth
+    int* ncap;
+    long long* fin;        // first slot after the growth
+    long long* scr;        // scratch of a row compacted in place, -1: the row moves
+    unsigned* chunk_row;   // per chunk: its row's place in the list
+    int* chunk_live;       // ... live entries, and those before it in its row
+    int* chunk_off;
+    uint2* place;          // per overflowed end: its slot and its partner's (without twins: 64 bits)
+    int* gidx;             // per vertex: 1 + its place in the list (0 = not growing)
+    unsigned long long* spare;  // {top, end} of the spare region
+    int slack_min;
+};
+
 struct UpdParams {
     DevGraph g;
+    DevGrow grow;
     const int4* chg;  // (u, v, w, op) records
     long long k;
-    int* ins_state;   // per record: 1 = insertion that survives the batch
     DelSlot* hset;    // deletion set: endpoint pair -> weight (open addressing)
     unsigned long long hmask;
-    int4* ovf;        // insertions that did not fit their row: (row, col, wt, record)
-    long long* slot;  // per record, both directions: slot of the appended entry, -1 = overflowed
+    int4* ovf;        // ends that did not fit their row: (row, col, wt, 2 * record + side)
+    long long* slot;  // of their records, both directions: slot of the entry, -1 - k = the row's k-th overflow
     unsigned epoch;
     int te;           // edges per thread item
     int large_deg;    // rows above this become CTA items

@@ -4,8 +4,9 @@
 // The graph store replaces the reference's host vector-of-vectors adjacency that is rebuilt
 // and re-copied for every batch (all_structure_undir.cuh:178-198, SSSPmainForUndirected.cu:
 // 42-91): rows live on the device, sorted by neighbour, each with free slots so insertions
-// append in place.  A row that runs out of slots triggers a repack (rows re-sorted, tombstones
-// dropped, slack restored) and the batch resumes after it.
+// append in place.  A row that runs out of slots grows inside the update kernel (grow.cuh); only when
+// the spare region is used up is the adjacency repacked (rows re-sorted, tombstones dropped, slack
+// restored) and the update kernel run again.
 #include <algorithm>
 #include <atomic>
 #include <cstdio>
@@ -27,6 +28,7 @@ cudaError_t launch_front(const UpdParams& p, int grid, cudaStream_t s, cudaEvent
                          cudaEvent_t after_delete);
 cudaError_t update_occupancy(int block, int* blocks_per_sm);
 cudaError_t launch_update(const UpdParams& p, int grid, int block, cudaStream_t s);
+cudaError_t launch_grow_finish(const UpdParams& p, int grid, cudaStream_t s);
 void batch_kernels(const void* fns[4]);
 const void* update_kernel(bool warp_agg);
 const void* delete_kernel(bool tails);
@@ -174,308 +176,6 @@ __global__ void k_pack_ovf(const int4* ovf, int novf, const long long* poff, int
     if (i >= novf) return;
     const int4 o = ovf[i];
     keys[poff[o.x] + atomicAdd(&cursor[o.x], 1)] = make_key(o.y, o.z);
-}
-
-// ---- row growth: rows that ran out of slack are compacted in place or move to the spare region ----
-
-struct GrowParams {
-    RowDesc* rows;
-    int2* adj;
-    unsigned* twin;
-    const int4* ovf;
-    int novf;
-    const int4* chg;
-    long long k;
-    const int* ins_state;
-    long long* slot;
-    int* need;                 // per vertex: overflowed entries of its row (0 = row not growing)
-    int* gidx;                 // per vertex: 1 + index in the grow list (0 = not growing)
-    unsigned* grow_list;       // rows that grow
-    unsigned* grow_count;
-    long long* old_start;      // per grow-list entry
-    int* old_cap;
-    unsigned long long* spare; // {top, end} of the spare region (bump allocator)
-    int* fail;
-    int slack_min;
-    long long cap_total;
-    // compacting growth (with the twin index)
-    int* sorted_len;
-    long long* new_start;             // per grow-list entry: the row's first slot after growth
-    long long* scratch;               // per grow-list entry: scratch of a row compacted in place, -1: moves
-    int* live;                        // per grow-list entry: live entries (tombstones are dropped)
-    int* live_sorted;                 // ... of them in the neighbour-sorted prefix
-    int* ncap;                        // per grow-list entry: capacity after growth
-    unsigned long long* scr_used;     // scratch slots taken from the free end of the spare region
-    unsigned long long* dropped;      // tombstones dropped
-};
-
-__global__ void k_grow_count(GrowParams q) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= q.novf) return;
-    const int r = q.ovf[i].x;
-    if (atomicAdd(&q.need[r], 1) == 0) {
-        const unsigned j = atomicAdd(q.grow_count, 1u);
-        q.grow_list[j] = (unsigned)r;
-        q.gidx[r] = (int)j + 1;
-    }
-}
-
-// Without the twin index (slot counts above 32 bits): warp per growing row, a region of
-// 2 * (cap + need) + slack_min slots from the spare region, the row's cap stored entries
-// (tombstones included) copied there.
-__global__ void k_grow_move(GrowParams q) {
-    const unsigned j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31;
-    if (j >= *q.grow_count) return;
-    const unsigned r = q.grow_list[j];
-    const RowDesc rd = q.rows[r];
-    const long long ncap = 2LL * (rd.cap + q.need[r]) + q.slack_min;
-    unsigned long long pos = 0;
-    if (lane == 0) pos = atomicAdd(&q.spare[0], (unsigned long long)ncap);
-    pos = __shfl_sync(0xFFFFFFFFu, pos, 0);
-    if (pos + (unsigned long long)ncap > q.spare[1] || ncap > 0x7FFFFFFFLL) {
-        if (lane == 0) atomicExch(q.fail, 1);
-        return;
-    }
-    for (int e = (int)lane; e < rd.cap; e += 32) {
-        q.adj[pos + e] = q.adj[rd.start + e];
-        if (q.twin) q.twin[pos + e] = q.twin[rd.start + e];
-    }
-    if (lane == 0) {
-        q.old_start[j] = rd.start;
-        q.old_cap[j] = rd.cap;
-        RowDesc nr;
-        nr.start = (long long)pos;
-        nr.deg = rd.cap;  // the entries actually stored; overflowed ones are placed next
-        nr.cap = (int)ncap;
-        q.rows[r] = nr;
-    }
-}
-
-// Warp per grown row: every live entry re-links with its reverse entry, wherever either moved.
-// Each moved entry reads only its own twin word, which no other thread writes.
-__global__ void k_grow_fix(GrowParams q) {
-    const unsigned j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31;
-    if (j >= *q.grow_count || !q.twin) return;
-    const unsigned r = q.grow_list[j];
-    const long long ns = q.rows[r].start;
-    for (int e = (int)lane; e < q.old_cap[j]; e += 32) {
-        const long long at = ns + e;
-        const int2 x = q.adj[at];
-        const unsigned t = q.twin[at];
-        if (x.y < 0 || t == kNoTwin) continue;
-        const int c = x.x;  // the reverse entry lives in row c
-        const int gc = q.gidx[c];
-        // A moved partner re-links itself from its own (old) twin word, so only our own word
-        // is written for it; a partner that stayed gets our new slot.
-        const long long t2 = gc ? q.rows[c].start + ((long long)t - q.old_start[gc - 1]) : (long long)t;
-        if (t2 < 0 || t2 >= q.cap_total) {  // internal error: report, skip the access
-            atomicExch(q.fail, 2);
-            continue;
-        }
-        q.twin[at] = (unsigned)t2;
-        if (!gc) q.twin[t2] = (unsigned)at;
-    }
-}
-
-// Places the overflowed ends of every surviving insertion into its grown row and pairs twins.
-__global__ void k_grow_place(GrowParams q) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= q.k) return;
-    const int4 c = q.chg[i];
-    if (c.w != 1 || q.ins_state[i] != 1) return;
-    long long at[2] = {q.slot[2 * i], q.slot[2 * i + 1]};
-    if (at[0] >= 0 && at[1] >= 0) return;
-#pragma unroll
-    for (int side = 0; side < 2; side++) {
-        if (at[side] >= 0) {
-            // the end that fitted may sit in a row that moved in this growth step
-            const int r = side ? c.y : c.x;
-            const int gr = q.gidx[r];
-            if (gr) at[side] = q.rows[r].start + (at[side] - q.old_start[gr - 1]);
-            continue;
-        }
-        const int r = side ? c.y : c.x, col = side ? c.x : c.y;
-        const int pos = atomicAdd(&q.rows[r].deg, 1);
-        at[side] = q.rows[r].start + pos;
-        q.adj[at[side]] = make_int2(col, c.z);
-        q.slot[2 * i + side] = at[side];
-    }
-    if (q.twin) {
-        q.twin[at[0]] = (unsigned)at[1];
-        q.twin[at[1]] = (unsigned)at[0];
-    }
-}
-
-__global__ void k_grow_reset(GrowParams q) {
-    const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= *q.grow_count) return;
-    const unsigned r = q.grow_list[j];
-    q.need[r] = 0;
-    q.gidx[r] = 0;
-}
-
-// ---- compacting growth (twin index): a growing row keeps only its live entries, in their
-// order (the sorted prefix stays sorted).  A row whose live entries and overflow fit its own
-// region with room to spare is compacted in place (through scratch slots at the free end of the
-// spare region, so it uses none of that region); the others move to a region of
-// 2 * (live + need) + slack_min slots.  Every moved live entry leaves its final slot in its old
-// twin word (a forwarding pointer), through which the twins and the batch's recorded slots are
-// re-linked.  Warp per growing row unless noted.
-
-__global__ void k_grow_plan(GrowParams q) {
-    const unsigned j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31;
-    if (j >= *q.grow_count) return;
-    const unsigned r = q.grow_list[j];
-    const RowDesc rd = q.rows[r];
-    const int sl = q.sorted_len[r];
-    int live = 0, ls = 0;
-    for (int e = (int)lane; e < rd.cap; e += 32) {
-        const bool l = q.adj[rd.start + e].y >= 0;
-        live += l ? 1 : 0;
-        ls += l && e < sl ? 1 : 0;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        live += __shfl_xor_sync(0xFFFFFFFFu, live, o);
-        ls += __shfl_xor_sync(0xFFFFFFFFu, ls, o);
-    }
-    if (lane != 0) return;
-    const long long need = q.need[r];
-    const long long room = live / 8 > 1 ? live / 8 : 1;  // free slots left after an in-place compaction
-    q.live[j] = live;
-    q.live_sorted[j] = ls;
-    atomicAdd(q.dropped, (unsigned long long)(rd.cap - live));
-    if (live + need + room <= rd.cap) {
-        const unsigned long long at = atomicAdd(q.scr_used, (unsigned long long)live);
-        q.new_start[j] = rd.start;
-        q.scratch[j] = (long long)(q.spare[1] - at - (unsigned long long)live);  // checked on the host
-        q.ncap[j] = rd.cap;
-    } else {
-        const long long nc = 2 * (live + need) + q.slack_min;
-        const unsigned long long pos = atomicAdd(&q.spare[0], (unsigned long long)nc);
-        if (pos + (unsigned long long)nc > q.spare[1] || nc > 0x7FFFFFFFLL) atomicExch(q.fail, 1);
-        q.new_start[j] = (long long)pos;
-        q.scratch[j] = -1;
-        q.ncap[j] = (int)(nc > 0x7FFFFFFFLL ? 0x7FFFFFFFLL : nc);
-    }
-    q.old_start[j] = rd.start;
-    q.old_cap[j] = rd.cap;
-}
-
-__global__ void k_grow_out(GrowParams q) {
-    const unsigned j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31;
-    if (j >= *q.grow_count) return;
-    const long long os = q.old_start[j], fin = q.new_start[j];
-    const long long dst = q.scratch[j] >= 0 ? q.scratch[j] : fin;
-    const int cap = q.old_cap[j];
-    int idx = 0;
-    for (int b = 0; b < cap; b += 32) {
-        const int e = b + (int)lane;
-        const int2 x = e < cap ? q.adj[os + e] : make_int2(0, -1);
-        const bool l = x.y >= 0;
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, l);
-        const int at = idx + __popc(m & ((1u << lane) - 1u));
-        if (l) {
-            q.adj[dst + at] = x;
-            q.twin[dst + at] = q.twin[os + e];  // the partner's old slot, re-linked below
-            q.twin[os + e] = (unsigned)(fin + at);
-        }
-        idx += __popc(m);
-    }
-}
-
-// Each compacted entry takes its partner's final slot: from the partner's forwarding pointer
-// when the partner's row grows too, else the partner stays and gets this entry's final slot.
-__global__ void k_grow_relink(GrowParams q) {
-    const unsigned j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31;
-    if (j >= *q.grow_count) return;
-    const long long fin = q.new_start[j];
-    const long long at0 = q.scratch[j] >= 0 ? q.scratch[j] : fin;
-    const int live = q.live[j];
-    for (int e = (int)lane; e < live; e += 32) {
-        const unsigned t = q.twin[at0 + e];
-        if (t == kNoTwin) continue;
-        const int c = q.adj[at0 + e].x;  // the partner lives in row c
-        if ((long long)t >= q.cap_total) {  // internal error: report, skip the access
-            atomicExch(q.fail, 2);
-            continue;
-        }
-        unsigned t2 = t;
-        if (q.gidx[c]) t2 = q.twin[t];
-        else q.twin[t] = (unsigned)(fin + e);
-        if ((long long)t2 >= q.cap_total) {
-            atomicExch(q.fail, 2);
-            continue;
-        }
-        q.twin[at0 + e] = t2;
-    }
-}
-
-// Thread per record: the recorded slot of an inserted end that fitted into a growing row.
-__global__ void k_grow_translate(GrowParams q) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= q.k) return;
-    const int4 c = q.chg[i];
-    if (c.w != 1 || q.ins_state[i] != 1) return;
-#pragma unroll
-    for (int side = 0; side < 2; side++) {
-        const long long at = q.slot[2 * i + side];
-        const int r = side ? c.y : c.x;
-        if (at >= 0 && q.gidx[r]) q.slot[2 * i + side] = (long long)q.twin[at];
-    }
-}
-
-__global__ void k_grow_back(GrowParams q) {
-    const unsigned j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned lane = threadIdx.x & 31;
-    if (j >= *q.grow_count) return;
-    const long long fin = q.new_start[j], scr = q.scratch[j];
-    const int live = q.live[j];
-    if (scr >= 0)
-        for (int e = (int)lane; e < live; e += 32) {
-            q.adj[fin + e] = q.adj[scr + e];
-            q.twin[fin + e] = q.twin[scr + e];
-        }
-    if (lane == 0) {
-        const unsigned r = q.grow_list[j];
-        RowDesc nr;
-        nr.start = fin;
-        nr.deg = live;
-        nr.cap = q.ncap[j];
-        q.rows[r] = nr;
-        q.sorted_len[r] = q.live_sorted[j];
-    }
-}
-
-// Thread per record: the overflowed ends go after the live entries of their grown rows, and
-// every surviving insertion's two ends are paired.
-__global__ void k_grow_place2(GrowParams q) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= q.k) return;
-    const int4 c = q.chg[i];
-    if (c.w != 1 || q.ins_state[i] != 1) return;
-    long long at[2] = {q.slot[2 * i], q.slot[2 * i + 1]};
-    if (at[0] >= 0 && at[1] >= 0) return;  // paired by the batch (and re-linked if moved)
-#pragma unroll
-    for (int side = 0; side < 2; side++) {
-        if (at[side] >= 0) continue;
-        const int r = side ? c.y : c.x, col = side ? c.x : c.y;
-        const int pos = atomicAdd(&q.rows[r].deg, 1);
-        if (pos >= q.rows[r].cap) {  // cannot happen: growth sized the row for its overflow
-            atomicExch(q.fail, 3);
-            return;
-        }
-        at[side] = q.rows[r].start + pos;
-        q.adj[at[side]] = make_int2(col, c.z);
-        q.slot[2 * i + side] = at[side];
-    }
-    q.twin[at[0]] = (unsigned)at[1];
-    q.twin[at[1]] = (unsigned)at[0];
 }
 
 __global__ void k_int_to_ll(const int* a, int n, long long* b) {
@@ -774,27 +474,16 @@ struct dsssp_graph {
     // batch buffers
     int4* d_chg = nullptr;
     long long chg_cap = 0;
-    int* d_ins_state = nullptr;
     int4* d_ovf = nullptr;
     long long* d_slot = nullptr;        // per record: slots of both appended ends
     unsigned* d_seedq = nullptr;        // vertices seeded by the insertions of a batch
-    // in-place row growth
-    unsigned long long* d_spare = nullptr;  // {top, end} of the spare region
-    int* d_need = nullptr;
+    // row growth (DevGrow): {top, end} of the spare region, per-vertex list places, and the
+    // work arrays, carved from one allocation
+    unsigned long long* d_spare = nullptr;
     int* d_gidx = nullptr;
-    unsigned* d_grow_list = nullptr;
-    unsigned* d_grow_count = nullptr;
-    long long* d_old_start = nullptr;
-    int* d_old_cap = nullptr;
-    long long* d_gnew = nullptr;            // per grow-list entry: first slot after growth
-    long long* d_gscr = nullptr;            // per grow-list entry: scratch of an in-place compaction
-    int* d_glive = nullptr;                 // per grow-list entry: live entries, of them sorted, capacity
-    int* d_gsorted = nullptr;
-    int* d_gncap = nullptr;
-    unsigned long long* d_gwords = nullptr; // scratch slots used, tombstones dropped
-    long long grow_dropped = 0;             // tombstones the last row growth dropped
-    int* d_fail = nullptr;
-    long long grow_cap = 0;
+    unsigned char* d_grow = nullptr;
+    DevGrow grow{};
+    long long grow_rows = 0, grow_chunks = 0, grow_ends = 0;  // what the work arrays hold
     unsigned long long s_spare[2] = {0, 0};  // spare words saved with the snapshot
     long long s_spare_lo = 0;                // and the first slot of its spare region
     DelSlot* d_hset = nullptr;  // deletion set of the batch
@@ -942,40 +631,67 @@ int ensure_batch(dsssp_graph* g, long long k) {
     unsigned long long h = 64;
     while (h < 2ull * (unsigned long long)cap) h <<= 1;
     dfree(g->d_chg);
-    dfree(g->d_ins_state);
     dfree(g->d_ovf);
     dfree(g->d_hset);
     dfree(g->d_slot);
     dfree(g->d_seedq);
-    dfree(g->d_grow_list);
-    dfree(g->d_old_start);
-    dfree(g->d_old_cap);
-    dfree(g->d_gnew); dfree(g->d_gscr); dfree(g->d_glive); dfree(g->d_gsorted); dfree(g->d_gncap);
-    g->grow_cap = 0;
     g->chg_cap = 0;
     g->hcap = 0;
     int rc = dalloc(&g->d_chg, (size_t)cap, "change buffer");
-    if (!rc) rc = dalloc(&g->d_ins_state, (size_t)cap, "insertion state");
     if (!rc) rc = dalloc(&g->d_ovf, (size_t)cap * 2, "overflow buffer");
     if (!rc) rc = dalloc(&g->d_hset, (size_t)h, "deletion set");
     if (!rc) rc = dalloc(&g->d_slot, (size_t)cap * 2, "slot buffer");
     const long long gl = 2 * cap < g->n ? 2 * cap : g->n;
-    if (!rc) rc = dalloc(&g->d_grow_list, (size_t)gl, "grow list");
     if (!rc) rc = dalloc(&g->d_seedq, (size_t)gl, "seed list");
-    if (!rc) rc = dalloc(&g->d_old_start, (size_t)gl, "grow list");
-    if (!rc) rc = dalloc(&g->d_old_cap, (size_t)gl, "grow list");
-    if (!rc) rc = dalloc(&g->d_gnew, (size_t)gl, "grow list");
-    if (!rc) rc = dalloc(&g->d_gscr, (size_t)gl, "grow list");
-    if (!rc) rc = dalloc(&g->d_glive, (size_t)gl, "grow list");
-    if (!rc) rc = dalloc(&g->d_gsorted, (size_t)gl, "grow list");
-    if (!rc) rc = dalloc(&g->d_gncap, (size_t)gl, "grow list");
-    if (!rc && !g->d_gwords) rc = dalloc(&g->d_gwords, 2, "grow list");
-    if (!rc) g->grow_cap = gl;
     if (!rc) {
         g->chg_cap = cap;
         g->hcap = h;
     }
     return rc;
+}
+
+// Work arrays of the row growth for batches of the buffers' size: every overflowed end may be the
+// first of its row, and the growing rows' chunks are those of the adjacency at most.
+int ensure_grow(dsssp_graph* g, cudaStream_t s) {
+    if (!g->d_gidx) {
+        int rc = dalloc(&g->d_gidx, (size_t)g->n, "row growth");
+        if (rc) return rc;
+        CK(cudaMemsetAsync(g->d_gidx, 0, sizeof(int) * (size_t)g->n, s), "row growth");
+    }
+    const long long rows = 2 * g->chg_cap < g->n ? 2 * g->chg_cap : g->n;
+    const long long chunks = g->cap_total / kGrowChunk + rows;
+    const long long ends = 2 * g->chg_cap;
+    if (rows <= g->grow_rows && chunks <= g->grow_chunks && ends <= g->grow_ends) return DSSSP_OK;
+    dfree(g->d_grow);
+    g->grow_rows = g->grow_chunks = g->grow_ends = 0;
+    const size_t R = ((size_t)rows + 1) & ~(size_t)1, C = ((size_t)chunks + 1) & ~(size_t)1, E = (size_t)ends;
+    int rc = dalloc(&g->d_grow, R * (7 * 4 + 2 * 8) + C * 12 + E * 8, "row growth");
+    if (rc) return rc;
+    DevGrow& q = g->grow;
+    unsigned char* at = g->d_grow;
+    auto carve = [&](auto*& ptr, size_t n) {
+        ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(at);
+        at += n * sizeof(*ptr);
+    };
+    carve(q.fin, R);  // 8-byte arrays first; the others have an even length
+    carve(q.scr, R);
+    carve(q.place, E);
+    carve(q.row, R);
+    carve(q.chunk0, R);
+    carve(q.done, R);
+    carve(q.live, R);
+    carve(q.lsorted, R);
+    carve(q.ndeg, R);
+    carve(q.ncap, R);
+    carve(q.chunk_row, C);
+    carve(q.chunk_live, C);
+    carve(q.chunk_off, C);
+    q.gidx = g->d_gidx;
+    q.spare = g->d_spare;
+    g->grow_rows = rows;
+    g->grow_chunks = chunks;
+    g->grow_ends = ends;
+    return DSSSP_OK;
 }
 
 // deg (int, n) -> deg64 (n+1, last 0) and poff = exclusive scan (n+1, last = total)
@@ -1159,11 +875,12 @@ UpdParams make_params(const dsssp_graph* g, const int4* chg, long long k, int mo
     p.g.cap_total = g->cap_total;
     p.chg = chg;
     p.k = k;
-    p.ins_state = g->d_ins_state;
     p.hset = g->d_hset;
     p.hmask = g->hcap ? g->hcap - 1 : 0;
     p.ovf = g->d_ovf;
     p.slot = g->d_slot;
+    p.grow = g->grow;
+    p.grow.slack_min = g->o.slack_min > 4 ? g->o.slack_min : 4;
     p.epoch = g->epoch;
     p.te = g->o.small_deg;
     p.large_deg = g->o.large_deg;
@@ -1295,115 +1012,6 @@ void fill_stats(const dsssp_graph* g, const Ctl& c, dsssp_stats* st, bool events
                          8.0 * seed_upd + 8.0 * seed_front;
     st->bytes_alg_update = upd;
     st->bytes_alg = upd + front;
-}
-
-constexpr int kSpareExhausted = 1;
-
-// Moves every row that overflowed in this batch into the spare region and places its
-// overflowed entries; kSpareExhausted if the region is too small (nothing lost: the caller
-// repacks, which folds the overflow list in).
-// Row growth with the twin index: rows compacted in place or moved, tombstones dropped (the
-// kernels above).  kSpareExhausted when the moves and the scratch do not both fit the spare
-// region (nothing has been written then: the caller repacks).
-int grow_rows_compacting(dsssp_graph* g, const GrowParams& q, int novf, long long rows_max, unsigned wb,
-                         cudaStream_t s) {
-    CK(cudaMemsetAsync(g->d_gwords, 0, 2 * sizeof(unsigned long long), s), "row growth");
-    k_grow_count<<<blocks_for(novf), kThreads, 0, s>>>(q);
-    k_grow_plan<<<wb, kThreads, 0, s>>>(q);
-    count_launch(2);
-    int fail = 0;
-    unsigned long long sp[2] = {0, 0}, words[2] = {0, 0};
-    CK(cudaMemcpyAsync(&fail, g->d_fail, sizeof(int), cudaMemcpyDeviceToHost, s), "row growth");
-    CK(cudaMemcpyAsync(sp, g->d_spare, sizeof(sp), cudaMemcpyDeviceToHost, s), "row growth");
-    CK(cudaMemcpyAsync(words, g->d_gwords, sizeof(words), cudaMemcpyDeviceToHost, s), "row growth");
-    CK(cudaStreamSynchronize(s), "row growth");
-    if (fail || sp[0] + words[0] > sp[1]) {
-        k_grow_reset<<<blocks_for(rows_max), kThreads, 0, s>>>(q);
-        count_launch(1);
-        CK(cudaStreamSynchronize(s), "row growth");
-        return kSpareExhausted;
-    }
-    k_grow_out<<<wb, kThreads, 0, s>>>(q);
-    k_grow_relink<<<wb, kThreads, 0, s>>>(q);
-    k_grow_translate<<<blocks_for(g->pend_k), kThreads, 0, s>>>(q);
-    k_grow_back<<<wb, kThreads, 0, s>>>(q);
-    k_grow_place2<<<blocks_for(g->pend_k), kThreads, 0, s>>>(q);
-    k_grow_reset<<<blocks_for(rows_max), kThreads, 0, s>>>(q);
-    count_launch(6);
-    CK(cudaMemcpyAsync(&fail, g->d_fail, sizeof(int), cudaMemcpyDeviceToHost, s), "row growth");
-    CK(cudaStreamSynchronize(s), "row growth");
-    if (fail) return dsssp::fail(DSSSP_E_CUDA, "row growth: internal error %d", fail);
-    g->spare_top = (long long)sp[0];
-    g->grow_dropped = (long long)words[1];
-    return DSSSP_OK;
-}
-
-int grow_rows(dsssp_graph* g, int novf, cudaStream_t s) {
-    if (novf <= 0) return DSSSP_OK;
-    if (!g->d_need) {
-        int rc = dalloc(&g->d_need, (size_t)g->n, "row growth");
-        if (!rc) rc = dalloc(&g->d_gidx, (size_t)g->n, "row growth");
-        if (rc) return rc;
-        CK(cudaMemsetAsync(g->d_need, 0, sizeof(int) * (size_t)g->n, s), "row growth");
-        CK(cudaMemsetAsync(g->d_gidx, 0, sizeof(int) * (size_t)g->n, s), "row growth");
-    }
-    GrowParams q;
-    q.rows = g->dg.rows;
-    q.adj = g->dg.adj;
-    q.twin = g->dg.twin;
-    q.ovf = g->d_ovf;
-    q.novf = novf;
-    q.chg = g->pend_chg;
-    q.k = g->pend_k;
-    q.ins_state = g->d_ins_state;
-    q.slot = g->d_slot;
-    q.need = g->d_need;
-    q.gidx = g->d_gidx;
-    q.grow_list = g->d_grow_list;
-    q.grow_count = g->d_grow_count;
-    q.old_start = g->d_old_start;
-    q.old_cap = g->d_old_cap;
-    q.spare = g->d_spare;
-    q.fail = g->d_fail;
-    q.slack_min = g->o.slack_min > 4 ? g->o.slack_min : 4;
-    q.cap_total = g->cap_total;
-    q.sorted_len = g->dg.sorted_len;
-    q.new_start = g->d_gnew;
-    q.scratch = g->d_gscr;
-    q.live = g->d_glive;
-    q.live_sorted = g->d_gsorted;
-    q.ncap = g->d_gncap;
-    q.scr_used = g->d_gwords;
-    q.dropped = g->d_gwords + 1;
-    g->grow_dropped = 0;
-    CK(cudaMemsetAsync(g->d_grow_count, 0, sizeof(unsigned), s), "row growth");
-    CK(cudaMemsetAsync(g->d_fail, 0, sizeof(int), s), "row growth");
-    const long long rows_max = novf < g->grow_cap ? novf : g->grow_cap;
-    const unsigned wb = (unsigned)((rows_max * 32 + kThreads - 1) / kThreads);
-    if (g->dg.twin) return grow_rows_compacting(g, q, novf, rows_max, wb, s);
-    k_grow_count<<<blocks_for(novf), kThreads, 0, s>>>(q);
-    k_grow_move<<<wb, kThreads, 0, s>>>(q);
-    count_launch(2);
-    int fail = 0;
-    CK(cudaMemcpyAsync(&fail, g->d_fail, sizeof(int), cudaMemcpyDeviceToHost, s), "row growth");
-    CK(cudaStreamSynchronize(s), "row growth");
-    if (fail) {
-        k_grow_reset<<<blocks_for(rows_max), kThreads, 0, s>>>(q);
-        count_launch(1);
-        CK(cudaStreamSynchronize(s), "row growth");
-        return kSpareExhausted;
-    }
-    k_grow_fix<<<wb, kThreads, 0, s>>>(q);
-    k_grow_place<<<blocks_for(g->pend_k), kThreads, 0, s>>>(q);
-    k_grow_reset<<<blocks_for(rows_max), kThreads, 0, s>>>(q);
-    count_launch(3);
-    CK(cudaMemcpyAsync(&fail, g->d_fail, sizeof(int), cudaMemcpyDeviceToHost, s), "row growth");
-    unsigned long long top = 0;
-    CK(cudaMemcpyAsync(&top, g->d_spare, sizeof(top), cudaMemcpyDeviceToHost, s), "row growth");
-    CK(cudaStreamSynchronize(s), "row growth");
-    if (fail) return dsssp::fail(DSSSP_E_CUDA, "row growth: twin index out of range (internal error)");
-    g->spare_top = (long long)top;
-    return DSSSP_OK;
 }
 
 // Kernel-node parameters of the batch kernels for the parameter block p.
@@ -1621,17 +1229,13 @@ int finish_batch(dsssp_graph* g, dsssp_stats* st) {
     CK(cudaStreamSynchronize(s), "batch");
     int repacks = 0;
     if (g->h_ctl->status == kStatusOverflowPending) {
-        // deletions are applied and the insertions that fit are placed.  The rows that ran
-        // out of slack drop their tombstones and are compacted in place or move to the spare
-        // region with room to grow; only when that region is used up is the whole adjacency
-        // repacked.  Then the update kernel runs.
-        int rc = grow_rows(g, g->h_ctl->ovf_count, s);
-        if (rc == kSpareExhausted) {
-            rc = repack(g, g->d_ovf, g->h_ctl->ovf_count, s);
-            repacks = 1;
-        }
+        // deletions are applied and the insertions that fit are placed; the rows that ran out of
+        // slack found no room in the spare region.  The whole adjacency is repacked, which
+        // folds their overflow in, and the update kernel runs again.
+        const int rc = repack(g, g->d_ovf, g->h_ctl->ovf_count, s);
         if (rc) return rc;
-        CK(cudaMemsetAsync(&g->dg.ctl->status, 0, sizeof(int), s), "status reset");
+        repacks = 1;
+        CK(cudaMemsetAsync(&g->dg.ctl->status, 0, offsetof(Ctl, inv_count) - offsetof(Ctl, status), s), "status reset");
         UpdParams p = make_params(g, g->pend_chg, g->pend_k, 0);
         // the front interval now spans the repack; the update interval is the resumed launch
         if (g->pend_events) CK(cudaEventRecord(g->ev[1], s), "event");
@@ -1640,14 +1244,32 @@ int finish_batch(dsssp_graph* g, dsssp_stats* st) {
         CK(cudaMemcpyAsync(g->h_ctl, g->dg.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s), "status read");
         CK(cudaStreamSynchronize(s), "batch");
     }
+    if (g->h_ctl->status < 0 && g->h_ctl->ovf_count > 0) {
+        // The update kernel gave up while rows were to grow.  Once every CTA had passed the
+        // growth's last phase but one, the last phase is run again; before that the rows stand as
+        // the insertions left them, and a repack takes their overflow in.
+        if (g->h_ctl->grow_done == (unsigned)g->coop_grid) {
+            CK(launch_grow_finish(make_params(g, g->pend_chg, g->pend_k, 0), g->num_sms, s), "row growth");
+        } else {
+            CK(cudaMemsetAsync(g->d_gidx, 0, sizeof(int) * (size_t)g->n, s), "row growth");
+            const int rc = repack(g, g->d_ovf, g->h_ctl->ovf_count, s);
+            if (rc) return rc;
+            repacks = 1;
+        }
+        CK(cudaStreamSynchronize(s), "row growth");
+    }
+    long long grow_dropped = 0;  // growth drops the tombstones of the rows that it compacts or moves
+    if (!repacks && g->h_ctl->spare_top) {
+        g->spare_top = (long long)g->h_ctl->spare_top;
+        grow_dropped = (long long)g->h_ctl->grow_dropped;
+    }
     fill_stats(g, *g->h_ctl, st, g->pend_events, g->pend_k, repacks);
     if (!repacks) {  // a repack counts the live entries itself
         const long long tombs = (long long)g->h_ctl->stat[ST_TOMBS];
         g->entries += 2 * (long long)g->h_ctl->stat[ST_LIVE_INS] - tombs;
-        g->dead += tombs - g->grow_dropped;  // row growth drops the tombstones of the rows it compacts
+        g->dead += tombs - grow_dropped;
         if (g->h_ctl->stat[ST_LIVE_INS] > 0) g->tails = true;  // insertions appended to row tails
     }
-    g->grow_dropped = 0;
     g->delta_ok = g->h_ctl->status == 0 && g->h_ctl->stat[ST_DIST_OVF] == 0;
     g->delta_empty = false;
     if (g->h_ctl->status == 0) g->last_rounds = (long long)g->h_ctl->stat[ST_ROUNDS];
@@ -1760,11 +1382,9 @@ void dsssp_graph_destroy(dsssp_graph* g) {
     dfree(d.state); dfree(d.rows); dfree(d.sorted_len); dfree(d.adj); dfree(d.inv_tag);
     dfree(d.push_tag); dfree(d.jm); dfree(d.invq); dfree(d.rt0); dfree(d.rt1); dfree(d.rc0); dfree(d.rc1);
     dfree(d.it); dfree(d.ic); dfree(d.ctl); dfree(d.far0); dfree(d.far1); dfree(d.far_tag); dfree(d.chg_tag);
-    dfree(g->d_chg); dfree(g->d_ins_state); dfree(g->d_ovf); dfree(g->d_hset); dfree(d.twin); dfree(g->s_twin);
+    dfree(g->d_chg); dfree(g->d_ovf); dfree(g->d_hset); dfree(d.twin); dfree(g->s_twin);
     dfree(g->d_par); dfree(g->d_dist); dfree(g->d_vtx); dfree(g->d_count); dfree(g->d_srcs); dfree(g->d_slot); dfree(g->d_seedq); dfree(g->d_spare);
-    dfree(g->d_need); dfree(g->d_gidx); dfree(g->d_grow_list); dfree(g->d_grow_count); dfree(g->d_old_start);
-    dfree(g->d_old_cap); dfree(g->d_fail);
-    dfree(g->d_gnew); dfree(g->d_gscr); dfree(g->d_glive); dfree(g->d_gsorted); dfree(g->d_gncap); dfree(g->d_gwords);
+    dfree(g->d_gidx); dfree(g->d_grow);
     dfree(g->s_state); dfree(g->s_rows); dfree(g->s_sorted); dfree(g->s_adj);
     if (g->bexec) cudaGraphExecDestroy(g->bexec);
     if (g->bgraph) cudaGraphDestroy(g->bgraph);
@@ -1850,8 +1470,6 @@ int dsssp_graph_create(int32_t n, int64_t m, const int32_t* u, const int32_t* v,
     if (!rc) rc = dalloc(&d.chg_tag, N, "change tags");
     if (!rc) rc = dalloc(&d.ctl, 1, "control block");
     if (!rc) rc = dalloc(&g->d_spare, 2, "spare region words");
-    if (!rc) rc = dalloc(&g->d_grow_count, 1, "row growth");
-    if (!rc) rc = dalloc(&g->d_fail, 1, "row growth");
     if (rc) { dsssp_graph_destroy(g); return rc; }
     cudaStream_t s = g->stream;
     cudaMemsetAsync(d.state, 0xFF, sizeof(unsigned long long) * N, s);
@@ -2287,6 +1905,7 @@ int dsssp_apply_batch_async(dsssp_graph* g, const dsssp_change* d_changes, int64
         return DSSSP_OK;
     }
     rc = ensure_batch(g, k);
+    if (!rc) rc = ensure_grow(g, s);
     if (!rc && g->copy_pending) CK(cudaStreamWaitEvent(s, g->ev_unpacked, 0), "apply_batch");  // a read's unpack
     if (!rc) rc = next_epoch(g, s);
     if (!rc) rc = enqueue_batch(g, (const int4*)d_changes, k, s);

@@ -11,11 +11,14 @@
 // The first four phases write only free slots, twin words and the work arrays: until the last
 // one (grow_finish) the rows stand as k_append left them, and grow_finish may be run again.
 //
-// A warp per chunk, not per row: rows of 10^5 entries grow in a stream on a skewed graph, and a warp
-// that walked one alone took up to 2 ms (RMAT scale 22, 10^6 changes a batch).  Inside k_update,
-// not as kernels of its own: with the host between them (status read, eight launches, three
-// synchronisations) a growth of a dozen rows took 0.11 ms.  A dozen rows are grown by one
-// CTA with block barriers.
+// Bound: random sectors (a moved entry reads its partner's place and writes its partner's twin
+// word) for many entries, a chain of dependent accesses and a barrier per phase for few.  A warp
+// per chunk, not per row: rows of 10^5 entries grow in a stream on a skewed graph, and a warp that
+// walked one alone took up to 2 ms.  Inside k_update, not as kernels with the host between them
+// (status read, eight launches, three synchronisations).  Per batch, growth included: 10,000
+// vertices and 1,000 changes 0.28 -> 0.21 ms, 300,000 and 12,345 changes 0.36 -> 0.29 ms, RMAT scale
+// 22 and 10^6 changes 1.66 -> 0.98 and 1.32 ms (a batch and its inverse, medians of a stream).
+// A handful of chunks is one CTA's work with block barriers: the grid's cost more than it.
 #pragma once
 
 // Chunks a row of `cap` slots is cut into (at least one: a row without slots grows too).
@@ -232,13 +235,17 @@ __device__ void grow_place(const UpdParams& p, const GrowTeam& t, unsigned novf)
         const int4 x = __ldcg(&p.ovf[o]);  // row, column, weight, 2 * record + side
         const unsigned s = (unsigned)x.w;
         const long long raw = __ldcg(&p.slot[s]), praw = __ldcg(&p.slot[s ^ 1u]);
-        const unsigned j = (unsigned)__ldcg(&q.gidx[x.x]) - 1u;
+        const int j = __ldcg(&q.gidx[x.x]) - 1, pj = __ldcg(&q.gidx[x.y]) - 1;
+        if (j < 0 || raw >= 0 || (praw < 0 && pj < 0)) {  // internal error: report, skip (the row is listed)
+            set_status(p.g.ctl, -4);
+            q.place[o] = make_uint2(kNoTwin, kNoTwin);
+            continue;
+        }
         const long long own = __ldcg(&q.fin[j]) + __ldcg(&q.live[j]) + (-1 - raw);
         if (!p.g.twin) {
             q.place[o] = make_uint2((unsigned)own, (unsigned)((unsigned long long)own >> 32));
             continue;
         }
-        const int pj = __ldcg(&q.gidx[x.y]) - 1;
         long long partner = praw;
         if (praw < 0) {
             partner = __ldcg(&q.fin[pj]) + __ldcg(&q.live[pj]) + (-1 - praw);
@@ -275,6 +282,7 @@ __device__ void grow_finish(const UpdParams& p, const GrowTeam& t, unsigned rows
         const int4 x = __ldcg(&p.ovf[o]);
         const uint2 s = __ldcg(&q.place[o]);
         const long long own = p.g.twin ? (long long)s.x : (long long)(((unsigned long long)s.y << 32) | s.x);
+        if (own >= p.g.cap_total) continue;  // reported by grow_place
         p.g.adj[own] = make_int2(x.y, x.z);
         if (p.g.twin) p.g.twin[own] = s.y;
     }

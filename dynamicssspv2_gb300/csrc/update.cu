@@ -293,6 +293,8 @@ __device__ __forceinline__ unsigned warp_incl_scan(unsigned x) {
     return x;
 }
 
+#include "grow.cuh"
+
 // Per-warp shared-memory buffer of pushed (vertex, degree, row start).  Entries are split into work
 // items when the buffer is nearly full (one list-counter atomic per warp for up to kBuf
 // vertices) and at the end of a phase (one atomic per CTA): the list counters are single
@@ -1384,23 +1386,6 @@ __device__ bool hash_contains(const UpdParams& p, unsigned long long pair, int w
     return false;
 }
 
-// Writes the entry (col, w) at position pos of row r, described by rd (read before the degree
-// bump).  Returns its slot, or -1 after listing it for the host-side row growth when the row
-// is full (record i).
-__device__ __forceinline__ long long place_entry(const UpdParams& p, const RowDesc& rd, int pos, int r, int col,
-                                                 int w, long long i, unsigned long long& ovf) {
-    if (pos < rd.cap) {
-        const long long at = rd.start + pos;
-        p.g.adj[at] = make_int2(col, w);
-        return at;
-    }
-    const int o = atomicAdd(&p.g.ctl->ovf_count, 1);
-    p.ovf[o] = make_int4(r, col, w, (int)i);
-    ovf++;
-    atomicCAS(&p.g.ctl->status, 0, kStatusOverflowPending);
-    return -1;
-}
-
 // Tombstones the reverse entry of slot j.  A twin word outside the adjacency is an internal
 // error: it is reported in the status word and the access is skipped.
 __device__ __forceinline__ void tombstone_twin(const UpdParams& p, long long j) {
@@ -1581,9 +1566,8 @@ __global__ void k_delete(UpdParams p) {
     block_add(&ctl->stat[ST_TOMBS], dead);
 }
 
-// Insertions that no deletion of the batch removes go into row slack, both directions.  An
-// entry that does not fit is written to the overflow list and the batch is deferred to a
-// host-side row growth (status 1).  Every surviving insertion then relaxes both of its ends
+// Insertions that no deletion of the batch removes go into row slack, both directions.  An end that
+// does not fit is listed with its row, and k_update grows the row first.  Every surviving insertion then relaxes both of its ends
 // (replaces insertEdge, gpuFunctions_undir.cuh:217-251); an improved end is claimed for the
 // first frontier and listed in seedq (k_update splits it into work items once every row has
 // its final degree) or, in near-far mode, put in the far list.  Doing this before the
@@ -1615,28 +1599,32 @@ __global__ void k_append(UpdParams p) {
         // probe; both degree bumps; both seed relaxations; both claims).
         int alive = 0;
         unsigned long long sa = kInfState, sb = kInfState;
+        RowDesc rx{0, 0, 0}, ry{0, 0, 0};
+        int pos0 = 0, pos1 = 0;
+        bool ov0 = false, ov1 = false;
         if (c.w == 1) {
             sa = __ldcg(&g.state[c.x]);
             sb = __ldcg(&g.state[c.y]);
-            const RowDesc rx = g.rows[c.x], ry = g.rows[c.y];  // start and cap are fixed in this kernel
+            rx = g.rows[c.x], ry = g.rows[c.y];  // start and cap are fixed in this kernel
             if (hash_contains(p, dpair_key((unsigned)c.x, (unsigned)c.y), c.z)) {
                 killed++;
             } else {
                 alive = 1;
                 live_ins++;
-                const int pos0 = atomicAdd(&g.rows[c.x].deg, 1);
-                const int pos1 = atomicAdd(&g.rows[c.y].deg, 1);
-                const long long at0 = place_entry(p, rx, pos0, c.x, c.y, c.z, i, ovf);
-                const long long at1 = place_entry(p, ry, pos1, c.y, c.x, c.z, i, ovf);
-                p.slot[2 * i] = at0;
-                p.slot[2 * i + 1] = at1;
+                pos0 = atomicAdd(&g.rows[c.x].deg, 1);
+                pos1 = atomicAdd(&g.rows[c.y].deg, 1);
+                ov0 = pos0 >= rx.cap;
+                ov1 = pos1 >= ry.cap;
+                if (!ov0) g.adj[rx.start + pos0] = make_int2(c.y, c.z);
+                if (!ov1) g.adj[ry.start + pos1] = make_int2(c.x, c.z);
                 if (g.twin) {  // an overflowed end is placed (and paired) by the row growth
-                    if (at0 >= 0) g.twin[at0] = at1 >= 0 ? (unsigned)at1 : kNoTwin;
-                    if (at1 >= 0) g.twin[at1] = at0 >= 0 ? (unsigned)at0 : kNoTwin;
+                    if (!ov0) g.twin[rx.start + pos0] = ov1 ? kNoTwin : (unsigned)(ry.start + pos1);
+                    if (!ov1) g.twin[ry.start + pos1] = ov0 ? kNoTwin : (unsigned)(rx.start + pos0);
                 }
+                ovf += (ov0 ? 1 : 0) + (ov1 ? 1 : 0);
             }
         }
-        if (i < p.k) p.ins_state[i] = alive;
+        list_overflow(p, i, c, rx, ry, pos0, pos1, ov0, ov1, rx.start + pos0, ry.start + pos1);
         // seed: relax both ends through the new edge
         bool pa = false, pbv = false;
         const unsigned long long ndb = (sa >> 32) + (unsigned)c.z, nda = (sb >> 32) + (unsigned)c.z;
@@ -1676,6 +1664,17 @@ __global__ void k_append(UpdParams p) {
     block_add(&ctl->stat[ST_LIVE_INS], live_ins);
     unsigned long long kk = warp_sum_u64(killed);
     if (lane_id() == 0 && kk) atomicAdd(&ctl->killed, (unsigned)kk);
+}
+
+// grid-wide; true when the kernel may go on
+__device__ __forceinline__ bool grow_rows(const UpdParams& p) { return __ldcg(&p.g.ctl->ovf_count) == 0 || grow(p); }
+
+// The last phase of a growth once more, for a batch whose update kernel gave up at a grid barrier
+// while that phase may have been running.
+__global__ void k_grow_finish(UpdParams p) {
+    const unsigned long long list = p.g.ctl->grow_list;
+    grow_finish(p, GrowTeam{blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x}, (unsigned)list,
+                (unsigned)(list >> 32), (unsigned)p.g.ctl->ovf_count);
 }
 
 template <bool kAgg>
@@ -1729,6 +1728,7 @@ __device__ void update_body(const UpdParams& p) {
     const bool leader = gtid == 0;
     uint4* pbuf = s_pbuf[threadIdx.x >> 5];
     LocalStats ls;
+    if (!grow_rows(p)) return;
     if (leader) ctl->ts[0] = globaltimer();
 
     unsigned rbase = __ldcg(&ctl->round_base);
@@ -1961,6 +1961,12 @@ cudaError_t launch_front(const UpdParams& p, int grid, cudaStream_t s, cudaEvent
     if (after_delete) cudaEventRecord(after_delete, s);
     k_append<<<g, 256, 0, s>>>(p);
     count_launch(3);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_grow_finish(const UpdParams& p, int grid, cudaStream_t s) {
+    k_grow_finish<<<(unsigned)grid, 256, 0, s>>>(p);
+    count_launch(1);
     return cudaGetLastError();
 }
 

@@ -139,7 +139,8 @@ typedef struct {
     double t_step1_ms;         /* insert + delete kernels (CUDA events) */
     double t_inval_ms;         /* subtree invalidation (device timestamps) */
     double t_relax_ms;         /* seeding + relaxation rounds (device timestamps) */
-    double t_update_ms;        /* the persistent update kernel (CUDA events) */
+    double t_update_ms;        /* the persistent update kernel, which first grows the rows that the
+                                  insertions overflowed (CUDA events) */
     double t_total_ms;         /* the whole batch on the device (CUDA events) */
     double bytes_alg;          /* algorithmic bytes of the batch (byte model of the engine) */
     double bytes_alg_update;   /* the update kernel's algorithmic bytes (per-unit byte model:
@@ -153,7 +154,7 @@ typedef struct {
                                    only the task byte model's units) */
     double t_delete_ms;        /* k_delete alone (CUDA events; batches at timing level 2) */
     double t_append_ms;        /* k_append alone, seeds included (CUDA events; batches at timing
-                                  level 2; with row growth it spans the growth too) */
+                                  level 2) */
     int64_t recovered_from;    /* DSSSP_W_RECOMPUTED: the code of the failure recovered from */
     double t_recompute_ms;     /* DSSSP_W_RECOMPUTED: the recomputation of the trees (CUDA events) */
     double t_seed_ms;          /* the seeding and pull phase alone (part of t_relax_ms) */

@@ -106,3 +106,37 @@ def test_invalid_options_are_refused():
         with pytest.raises(D.DsssspError) as e:
             g.set_opts(o)
         assert e.value.code == D.E_INVAL
+
+
+@pytest.mark.parametrize("recover", [1, 0])
+def test_timed_out_growth_keeps_the_whole_batch(recover):
+    """The barrier times out while rows are to grow (no slack: every insertion overflows): the
+    adjacency still takes in the whole batch, so a tree computed on it is the updated graph's,
+    and later batches are exact."""
+    n, m = 6000, 24000
+    u, v, w = D.gen_er(n, m, 1, 100, 81)
+    ch = D.gen_changes(n, u, v, w, 900, 900, seed=82)
+    with D.Graph(n, u, v, w, slack_pct=0, slack_min=0, spare_pct=100, recover=recover) as g:
+        g.tree_compute(0)
+        g.debug_set(D.DEBUG_SPIN_LIMIT, 4096)
+        g.debug_set(D.DEBUG_STALL_US, 200_000)
+        if recover:
+            assert g.apply_batch(ch).recovered_from == D.E_TIMEOUT
+        else:
+            with pytest.raises(D.DsssspError) as e:
+                g.apply_batch(ch)
+            assert e.value.code == D.E_TIMEOUT
+        g.debug_set(D.DEBUG_SPIN_LIMIT, 0)
+        g.debug_set(D.DEBUG_STALL_US, 0)
+        if not recover:
+            g.tree_compute(0)
+        p, d = g.tree_read()
+        check_against_oracle(n, u, v, w, ch, 0, p, d, "after a growth that timed out")
+        u, v, w = lines_after(n, u, v, w, ch)
+        for seed in (83, 84):
+            ch = D.gen_changes(n, u, v, w, 700, 700, seed=seed)
+            g.apply_batch(ch)
+            p, d = g.tree_read()
+            check_against_oracle(n, u, v, w, ch, 0, p, d, f"batch {seed}")
+            u, v, w = lines_after(n, u, v, w, ch)
+            assert g.health()["live"] == 2 * len(u) and g.validate()["violations"] == 0

@@ -5,7 +5,7 @@ import pytest
 
 import dynamicssspv2_gb300 as D
 from oracle import pyoracle as O
-from tests.common import case_arrays, check_against_oracle, golden_cases, tree_from_rows
+from tests.common import case_arrays, check_against_oracle, golden_cases, lines_after, tree_from_rows
 
 pytestmark = pytest.mark.gpu
 
@@ -812,3 +812,59 @@ def test_a_self_loop_deleted_by_many_records_is_counted_once():
             st = g.apply_batch(ch)
             assert st.tombstoned == 2 * len(loops)
             assert g.health()["live"] == 2 * (n - 1) and g.validate()["violations"] == 0
+@pytest.mark.parametrize("hub", [0, 255, 256, 257, 511, 513, 3000, 40000])
+def test_rows_grow_in_chunks(hub):
+    """Row growth at the edges of its chunks (256 slots): a hub row of that many slots without
+    slack, filled, half deleted (compacted in place next), filled again (moved), self-loops and
+    parallel edges among the insertions; beside it rows without any slot.  After every batch the
+    live count and the tree are exact, and a deletion of every inserted edge finds its entries
+    and their twins."""
+    rng = np.random.default_rng(hub)
+    n = hub + 300
+    u = np.concatenate([np.zeros(hub, np.int64), np.arange(hub, hub + 99)])
+    v = np.concatenate([1 + np.arange(hub), 1 + np.arange(hub, hub + 99)])
+    w = rng.integers(1, 50, len(u))
+    u, v, w = (np.ascontiguousarray(x, np.int32) for x in (u, v, w))
+
+    def insertions(k):
+        a = np.where(rng.random(k) < 0.7, 0, rng.integers(0, n, k))
+        b = np.where(rng.random(k) < 0.1, a, rng.integers(0, n, k))
+        return D.make_changes(a, b, rng.integers(1, 60, k), np.ones(k, np.int64))
+
+    with D.Graph(n, u, v, w, slack_pct=0, slack_min=0, spare_pct=400) as g:
+        g.tree_compute(0)
+        grown = 0
+        for step in range(7):
+            if step in (1, 4):  # half of the lines go
+                at = rng.choice(len(u), len(u) // 2, replace=False)
+                ch = D.make_changes(u[at], v[at], w[at], np.zeros(len(at), np.int64))
+            elif step == 6:  # every line goes
+                ch = D.make_changes(u, v, w, np.zeros(len(u), np.int64))
+            else:
+                ch = insertions(200 if hub < 3000 else hub // 4)
+            st = g.apply_batch(ch)
+            grown += st.overflow_entries
+            p, d = g.tree_read()
+            check_against_oracle(n, u, v, w, ch, 0, p, d, f"hub {hub} step {step}")
+            u, v, w = lines_after(n, u, v, w, ch)
+            assert g.health()["live"] == 2 * len(u), f"hub {hub} step {step}"
+            assert g.validate()["violations"] == 0
+        assert grown > 0 and len(u) == 0
+
+
+def test_growth_of_a_small_graph_under_larger_and_larger_batches():
+    """Batches that outgrow the buffers of the batches before them while the rows that can grow
+    stay the same few: the work arrays follow the batches as well as the rows."""
+    rng = np.random.default_rng(3)
+    n = 60
+    u, v, w = (np.ascontiguousarray(x, np.int32) for x in (np.arange(n - 1), np.arange(1, n), np.full(n - 1, 9)))
+    with D.Graph(n, u, v, w, slack_pct=0, slack_min=0, spare_pct=400) as g:
+        g.tree_compute(0)
+        for k in (5, 40, 300, 2000, 9000, 30, 12000):
+            ch = D.make_changes(rng.integers(0, n, k), rng.integers(0, n, k), rng.integers(1, 500, k), np.ones(k, np.int64))
+            st = g.apply_batch(ch)
+            p, d = g.tree_read()
+            check_against_oracle(n, u, v, w, ch, 0, p, d, f"{k} insertions")
+            u, v, w = lines_after(n, u, v, w, ch)
+            assert st.overflow_entries > 0 or k == 30
+            assert g.health()["live"] == 2 * len(u) and g.validate()["violations"] == 0
