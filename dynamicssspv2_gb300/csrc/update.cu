@@ -75,7 +75,7 @@ __shared__ unsigned s_ggen;        // group-barrier generation this CTA waits on
 __shared__ unsigned s_solo_cnt[3][2];
 __shared__ unsigned s_spin_limit;  // polls before a grid barrier gives up
 __shared__ uint4 s_pbuf[kMaxWarps][kBuf];  // (vertex, degree, row start) pushed, not yet expanded
-__shared__ unsigned s_stop;                // ... another CTA has ended the stretch
+__shared__ unsigned s_stop[2];             // ... another CTA has ended the stretch (seen in a step, read in the next)
 __shared__ unsigned s_qcnt[3];             // local stretches: items of the steps' queues, rotating
 __shared__ unsigned s_near[2];  // far_advance: the sizes of the near list
 __shared__ unsigned long long s_lstat[8];  // ... their counters, added to the kernel's at the end
@@ -966,13 +966,13 @@ __device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigne
     if (threadIdx.x == 0) {
         s_qcnt[0] = mine * parts;
         s_qcnt[1] = 0;
-        s_stop = 0;
+        s_stop[0] = s_stop[1] = 0;
     }
     __syncthreads();
     unsigned k = 0, n, cur = 0, nxt = 1, old = 2;  // the steps' counters rotate
     for (;; k++) {
         n = min(s_qcnt[cur], kQueue);
-        if (n == 0 || k >= steps_max || s_stop) break;
+        if (n == 0 || k >= steps_max || s_stop[k & 1]) break;
         if (n > limit && k > 0) {  // too much for this CTA: everybody's work is dealt out again
             if (threadIdx.x == 0) atomicExch(&ctl->rstop[slot], 1u);
             break;
@@ -983,7 +983,7 @@ __device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigne
             const unsigned i = b + (lane >> 2);
             st.visit(i < n ? queue_at(k & 1, i) : make_uint4(0, 0, 0, 0), (k + 1) & 1, &s_qcnt[nxt]);
         }
-        if (stop) s_stop = 1;
+        if (stop) s_stop[(k + 1) & 1] = 1;  // a slow warp may still read this step's word
         const unsigned t = old;
         old = cur;
         cur = nxt;
