@@ -61,10 +61,10 @@ constexpr unsigned kFarBuf = 64;           // per-warp staging of far-list pushe
 constexpr int kSpill = 64;                 // per-warp staging of vertices that leave a stretch
 constexpr unsigned kStretch = 256;         // steps of a local stretch at most
 static_assert(64 * (kLocalTe / 4) <= kQueue, "a CTA's first items must fit its queue");
-// a stretch keeps all of it in the push buffers: per warp kSpill entries pushed, then a share of
-// the two queues, then the far staging
-constexpr unsigned kShare = 2 * kQueue / kMaxWarps;
-static_assert(kSpill + kShare + kFarBuf / 4 <= kBuf && kSpill >= 2 * 32, "a stretch fits the push buffers");
+// a stretch keeps all of it in the push buffers: kSpill entries a warp for vertices that leave it,
+// the two queues, the far staging
+constexpr unsigned kQueueAt = kSpill * kMaxWarps, kFarAt = kQueueAt + 2 * kQueue;
+static_assert(kFarAt + kMaxWarps * kFarBuf / 4 <= kBuf * kMaxWarps && kSpill >= 2 * 32, "a stretch fits the push buffers");
 
 __shared__ unsigned s_nbar;        // grid barriers this CTA has passed
 __shared__ unsigned s_gen;         // barrier generation this CTA waits on next (ctl->bar_gen)
@@ -811,16 +811,19 @@ __device__ void run_items(Op& op, const UpdParams& p, const Item* tl, unsigned n
 // since (then that thread has pushed it).  The queue's pushes mark chg_tag, not push_tag, whose
 // tag says "claimed for the next list".
 //
-// Bound: the latency of the two accesses, 940 and 1,200-1,300 cycles of a step's 3,500-3,900 (clock
+// Bound: the latency of the two accesses, 1,000 and 1,200-1,400 cycles of a step's 3,300 (clock
 // counts on grids of 1.6M and 16.8M vertices), then the push, the block barrier and, per stretch,
-// a grid barrier with a new deal of the work.  A queue per CTA, not per warp: with one per warp a
-// step was 2.05 us instead of 2.7 (with its share of the deals), but a queue that grew past 32
-// entries took several steps a hop and the others waited for it (4096^2 grid, 100k changes: 21,476
-// steps, 46 ms a batch, against 12,310 and 36 ms).  A CTA whose queue passes one and a half passes
-// ends everybody's stretch (rstop), so the work is dealt out again when it is needed and not every
-// 16 or 64 steps (27.1 ms against 28.6 and 36).  Measured against rounds throughout: that batch
-// 95.0 -> 27.1 ms, a 1021 x 1543 grid with 9k changes 23.3 -> 7.8 ms, the tree of a 2048^2 grid
-// 38.0 -> 12.0 ms, ER graphs of 10k and 300k vertices 0.157 -> 0.130 and 0.264 -> 0.211 ms of k_update.
+// a grid barrier with a new deal of the work.  So the push is kept short (one shared atomic a
+// warp, no ranking bits unless a row takes two places), the fields of the parameter block are
+// held in registers and the pushed row is prefetched: 27.0 -> 23.7 ms on the 4096^2 grid below.
+// A queue per CTA, not per warp: with one per warp a step was shorter, but a queue that grew past
+// 32 entries took several steps a hop and the others waited for it (21,476 steps and 46 ms
+// against 12,310 and 36 ms).  A CTA whose queue passes one and a half passes ends everybody's
+// stretch (rstop), so the work is dealt out again when it is needed and not every 16 or 64 steps
+// (27.1 ms against 28.6 and 36).  Measured against rounds throughout: a 4096^2 grid with 100k
+// changes 95.0 -> 23.7 ms a batch, a 1021 x 1543 grid with 9k changes 23.3 -> 6.3 ms, the tree of
+// a 2048^2 grid 38.0 -> 9.7 ms, ER graphs of 10k and 300k vertices 0.157 -> 0.130 and 0.264 ->
+// 0.211 ms of k_update.
 // A round is a local stretch when it holds thread items only, no more than one pass of every CTA:
 // above that the grid is busy and the rounds' throughput counts.  (Half or a quarter of a pass:
 // the same on grids and ER graphs within 2 %, 64 pooled ER graphs 0.405 -> 0.410 and 0.424 ms.)
@@ -828,49 +831,61 @@ __device__ __forceinline__ bool local_step(const UpdParams& p, unsigned nt, unsi
     return nc == 0 && nt <= gridDim.x * (blockDim.x >> 2) && p.te <= kLocalTe && p.group_ctas == 0;
 }
 
-// Item i of queue q (0 or 1): (vertex, distance, slots, count), at most 4 slots each.
-__device__ __forceinline__ uint4& queue_at(unsigned q, unsigned i) {
-    const unsigned k = q * kQueue + i;
-    return s_pbuf[k / kShare][kSpill + k % kShare];
-}
-__device__ __forceinline__ unsigned* far_buf() {
-    return reinterpret_cast<unsigned*>(&s_pbuf[threadIdx.x >> 5][kSpill + kShare]);
-}
-
 __device__ __forceinline__ void keep_stats(const LocalStats& ls);
 
 struct Stretch {
     const UpdParams* p;
-    Out out;
-    Far far;
-    unsigned tag;
-    PushBuf pb;
-    unsigned nfar;
+    // fields of *p in registers: a function of its own reads them through memory
+    unsigned long long* state;
+    const int2* adj;
+    const RowDesc* rows;
+    unsigned* chg;
+    unsigned epoch, r, rbase, adv;  // list r is read, list r + 1 written; far list adv & 1
+    unsigned long long T;
+    int spilled;    // entries of the warp's spill staging
+    unsigned nfar;  // ... and of its far staging
     LocalStats ls;
 
+    __device__ __forceinline__ unsigned tag() const { return rbase + r + 2u; }
+    __device__ __forceinline__ PushBuf buf() const {
+        return PushBuf{&s_pbuf[0][0] + (threadIdx.x >> 5) * kSpill, spilled};
+    }
+    __device__ __forceinline__ Out out() const {
+        const DevGraph& g = p->g;
+        const bool odd = (r & 1) != 0;
+        const unsigned slot = (r + 1) % 3;
+        return Out{odd ? g.rt0 : g.rt1, &g.ctl->rcT[slot], g.tcap, odd ? g.rc0 : g.rc1, &g.ctl->rcC[slot], g.ccap};
+    }
+    __device__ __forceinline__ unsigned* lfar() const {
+        return reinterpret_cast<unsigned*>(&s_pbuf[0][0] + kFarAt) + (threadIdx.x >> 5) * kFarBuf;
+    }
+
     __device__ __forceinline__ void spill(bool pred, unsigned v, const RowDesc& rd) {
-        if (pb.count + 32 > kSpill) pb.expand_all(*p, out, ls);
+        PushBuf pb = buf();
+        if (spilled + 32 > kSpill) pb.expand_all(*p, out(), ls);
         pb.add(pred, v, rd);
+        spilled = pb.count;
         ls.frontier += pred ? 1 : 0;
     }
 
     __device__ __forceinline__ void flush_far() {
+        if (nfar == 0) return;
         __syncwarp();
-        const unsigned* lfar = far_buf();
+        const Far far{(adv & 1) ? p->g.far1 : p->g.far0, &p->g.ctl->fc[adv & 1], p->g.far_tag, rbase + adv,
+                      (unsigned)p->g.n, T};
         for (unsigned b = 0; b < nfar; b += 32)
-            far_push(*p, far, b + lane_id() < nfar, lfar[(b + lane_id()) & (kFarBuf - 1)]);
+            far_push(*p, far, b + lane_id() < nfar, lfar()[(b + lane_id()) & (kFarBuf - 1)]);
         nfar = 0;
         __syncwarp();
     }
 
-    // One item's entry per lane (warp-collective): x = the item (count 0: none), next = the
-    // number of the next step's queue, with its counter.
-    __device__ __forceinline__ void visit(const uint4& x, unsigned next, unsigned* next_cnt) {
+    // One item's entry per lane (warp-collective): x = the item, (vertex, distance, slots, count)
+    // of at most 4 entries (count 0: none), next = the next step's queue with its counter.
+    __device__ __forceinline__ void visit(const uint4& x, uint4* next, unsigned* next_cnt) {
         const unsigned lane = lane_id(), lt = (1u << lane) - 1u, sub = lane & 3u;
-        unsigned long long* const state = p->g.state;
         const bool act = sub < (x.w >> 8);
         const long long j = (long long)((unsigned long long)(x.w & 0xFFu) << 32 | x.z) + sub;
-        const int2 e = act ? ld_stream(&p->g.adj[j]) : make_int2(0, -1);
+        const int2 e = act ? ld_stream(&adj[j]) : make_int2(0, -1);
         const unsigned long long du = act ? __ldcg(&state[x.x]) >> 32 : kDistInf;
         const bool live = du < kDistInf && du >= x.y;  // below: improved since, and pushed again then
         const unsigned c = (unsigned)e.x;
@@ -878,31 +893,31 @@ struct Stretch {
         RowDesc rd{0, 0, 0};
         bool push = false;
         if (live && e.y >= 0) {
-            rd = p->g.rows[c];
+            rd = rows[c];
             if (e.y == 0) {
-                push = relax_to(p->g, p->epoch, c, nd, x.x, 0, __ldcg(&state[c]), ls);
+                push = relax_to(p->g, epoch, c, nd, x.x, 0, __ldcg(&state[c]), ls);
             } else if (nd < kDistInf) {
                 const unsigned long long cand = (nd << 32) | x.x;
                 const unsigned long long old = atomicMin(&state[c], cand);
                 push = (old >> 32) > nd;
                 if (push) ls.updates++;
-                else if (old > cand && p->g.chg_tag) p->g.chg_tag[c] = p->epoch;
+                else if (old > cand && chg) chg[c] = epoch;
             } else if (__ldcg(&state[c]) == kInfState) {
                 ls.dist_ovf++;
             }
         }
         ls.edges_relax += live ? 1 : 0;
         if (!__any_sync(kFull, push)) return;
-        const bool later = push && nd >= far.T;
+        const bool later = push && nd >= T;
         const bool near = push && !later && rd.deg > 0;
         // queue places: ceil(deg / 4) items a row, ranked in the warp by the bits of (items - 1)
         const bool shrt = near && rd.deg <= (int)kLocalDeg;
         const unsigned extra = shrt ? ((unsigned)rd.deg - 1u) >> 2 : 0u;
-        const unsigned m = __ballot_sync(kFull, shrt);
+        const unsigned m = __ballot_sync(kFull, shrt), mx = __ballot_sync(kFull, extra != 0);
         bool in = false;
         if (m) {
             unsigned rank = __popc(m & lt), total = __popc(m);
-            if (__any_sync(kFull, extra != 0)) {
+            if (mx) {
 #pragma unroll
                 for (int b = 0; b < 3; b++) {
                     const unsigned mb = __ballot_sync(kFull, extra & (1u << b));
@@ -910,30 +925,36 @@ struct Stretch {
                     total += __popc(mb) << b;
                 }
             }
-            unsigned base = 0;
-            if (lane == 0) base = atomicAdd(next_cnt, total);
-            const unsigned at = __shfl_sync(kFull, base, 0) + rank;
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(next_cnt, total);
+            at = __shfl_sync(kFull, at, 0) + rank;
             in = shrt && at + extra < kQueue;
             if (in) {
-                long long lo = rd.start;
-                for (unsigned k = 0; k <= extra; k++, lo += 4)
-                    queue_at(next, at + k) =
-                        make_uint4(c, (unsigned)nd, (unsigned)lo, (unsigned)((unsigned long long)lo >> 32) |
-                                                                      (min(4u, (unsigned)rd.deg - 4 * k) << 8));
-                if (p->g.chg_tag) p->g.chg_tag[c] = p->epoch;
+                const unsigned hi = (unsigned)((unsigned long long)rd.start >> 32);
+                if (extra == 0) {
+                    next[at] = make_uint4(c, (unsigned)nd, (unsigned)rd.start, hi | ((unsigned)rd.deg << 8));
+                } else {
+                    long long lo = rd.start;
+                    for (unsigned k = 0; k <= extra; k++, lo += 4)
+                        next[at + k] = make_uint4(c, (unsigned)nd, (unsigned)lo, (unsigned)((unsigned long long)lo >> 32) |
+                                                                                     (min(4u, (unsigned)rd.deg - 4 * k) << 8));
+                }
+                // the next step reads the row: on its way while this one ends
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(adj + rd.start));
+                if (chg) chg[c] = epoch;
                 ls.frontier++;
             } else if (shrt) {  // does not fit: its places stay empty
-                for (unsigned k = at; k < kQueue; k++) queue_at(next, k) = make_uint4(0, 0, 0, 0);
+                for (unsigned k = at; k < kQueue; k++) next[k] = make_uint4(0, 0, 0, 0);
             }
         }
         if (__any_sync(kFull, near && !in)) {
-            const bool won = near && !in && atomicExch(&p->g.push_tag[c], tag) != tag;
+            const bool won = near && !in && atomicExch(&p->g.push_tag[c], tag()) != tag();
             spill(won, c, rd);
         }
         const unsigned fmask = __ballot_sync(kFull, later);
         if (fmask) {
             if (nfar + __popc(fmask) > kFarBuf) flush_far();
-            if (later) far_buf()[nfar + __popc(fmask & lt)] = c;
+            if (later) lfar()[nfar + __popc(fmask & lt)] = c;
             nfar += __popc(fmask);
         }
     }
@@ -947,11 +968,11 @@ __device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigne
     const bool odd = (r & 1) != 0;
     const unsigned slot = (r + 1) % 3;
     const Item* const tl = odd ? p.g.rt1 : p.g.rt0;
-    const unsigned lane = lane_id(), per = blockDim.x >> 2, parts = (unsigned)p.te >> 2, limit = per + per / 2;
-    Stretch st{&p,
-               Out{odd ? p.g.rt0 : p.g.rt1, &ctl->rcT[slot], p.g.tcap, odd ? p.g.rc0 : p.g.rc1, &ctl->rcC[slot], p.g.ccap},
-               Far{(adv & 1) ? p.g.far1 : p.g.far0, &ctl->fc[adv & 1], p.g.far_tag, rbase + adv, (unsigned)p.g.n, T},
-               rbase + r + 2u, PushBuf{s_pbuf[threadIdx.x >> 5], 0}, 0, LocalStats{}};
+    const unsigned lane = lane_id();
+    const unsigned per = blockDim.x >> 2, parts = (unsigned)p.te >> 2, limit = per + per / 2;
+    uint4 *now = &s_pbuf[0][0] + kQueueAt, *next = now + kQueue;
+    Stretch st{&p, p.g.state, p.g.adj, p.g.rows, p.g.chg_tag, p.epoch, r, rbase, adv, T, 0, 0, LocalStats{}};
+    unsigned* const stopped = &ctl->rstop[slot];
     // items blockIdx, blockIdx + gridDim, ... of the list, at most `per` of them
     const unsigned mine = nt > blockIdx.x ? (nt - blockIdx.x - 1) / gridDim.x + 1 : 0u;
     for (unsigned i = threadIdx.x; i < mine; i += blockDim.x) {
@@ -959,7 +980,7 @@ __device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigne
         for (unsigned k = 0; k < parts; k++) {
             const long long lo = item_lo(it) + 4 * k;
             const unsigned cnt = it.w > 4 * k ? min(4u, it.w - 4 * k) : 0u;
-            queue_at(0, i * parts + k) =
+            now[i * parts + k] =
                 make_uint4(it.z, 0u, (unsigned)lo, (unsigned)((unsigned long long)lo >> 32) | (cnt << 8));
         }
     }
@@ -974,31 +995,34 @@ __device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigne
         n = min(s_qcnt[cur], kQueue);
         if (n == 0 || k >= steps_max || s_stop[k & 1]) break;
         if (n > limit && k > 0) {  // too much for this CTA: everybody's work is dealt out again
-            if (threadIdx.x == 0) atomicExch(&ctl->rstop[slot], 1u);
+            if (threadIdx.x == 0) atomicExch(stopped, 1u);
             break;
         }
         if (threadIdx.x == 0) s_qcnt[old] = 0;  // read by every thread before the last barrier
-        const unsigned stop = threadIdx.x == blockDim.x - 1 ? __ldcg(&ctl->rstop[slot]) : 0u;
+        const unsigned stop = threadIdx.x == blockDim.x - 1 ? __ldcg(stopped) : 0u;
         for (unsigned b = (threadIdx.x & ~31u) >> 2; b < n; b += per) {  // warp-uniform
             const unsigned i = b + (lane >> 2);
-            st.visit(i < n ? queue_at(k & 1, i) : make_uint4(0, 0, 0, 0), (k + 1) & 1, &s_qcnt[nxt]);
+            st.visit(i < n ? now[i] : make_uint4(0, 0, 0, 0), next, &s_qcnt[nxt]);
         }
         if (stop) s_stop[(k + 1) & 1] = 1;  // a slow warp may still read this step's word
         const unsigned t = old;
         old = cur;
         cur = nxt;
         nxt = t;
+        uint4* const q = now;
+        now = next;
+        next = q;
         __syncthreads();
     }
     st.flush_far();
     for (unsigned b = threadIdx.x & ~31u; b < n; b += blockDim.x) {
-        const uint4 x = b + lane < n ? queue_at(k & 1, b + lane) : make_uint4(0, 0, 0, 0);
+        const uint4 x = b + lane < n ? now[b + lane] : make_uint4(0, 0, 0, 0);
         const bool has = (x.w >> 8) != 0;
         RowDesc rd;
-        const bool won = claim_with_row(p, has, x.x, st.tag, rd);  // the whole row, once
+        const bool won = claim_with_row(p, has, x.x, st.tag(), rd);  // the whole row, once
         st.spill(won, x.x, rd);
     }
-    st.pb.flush_cta(p, st.out, st.ls);
+    st.buf().flush_cta(p, st.out(), st.ls);
     if (threadIdx.x == 0 && k) atomicMax(&ctl->rsteps[slot], k);
     keep_stats(st.ls);
 }
