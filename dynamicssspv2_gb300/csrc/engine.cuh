@@ -97,8 +97,9 @@ struct __align__(128) Ctl {
     unsigned long long scr_used;      // scratch slots taken from the free end of the spare region
     unsigned long long grow_dropped;  // tombstones dropped
     unsigned long long spare_top;     // the spare region's bump pointer after the growth (0: none)
+    unsigned tail_count;  // chunks of long row tails that k_delete left to k_append
     unsigned grow_done;   // CTAs past the growth's last phase but one (all: that phase has run or may)
-    unsigned pad1[17];
+    unsigned pad1[16];
     // line 2
     unsigned bar_count;
     unsigned pad2[31];
@@ -180,14 +181,15 @@ struct DevGrow {
     unsigned* row;         // the vertex
     unsigned* chunk0;      // its first chunk
     unsigned* done;        // chunks counted
-    int* live;             // live entries
-    int* lsorted;          // ... of them in the neighbour-sorted prefix
+    int* first;            // its entries from here on move (0, or the prefix stays)
+    int* live;             // the live ones of them
+    int* lsorted;          // neighbour-sorted prefix after the growth
     int* ndeg;             // degree and capacity after the growth
     int* ncap;
-    long long* fin;        // first slot after the growth
-    long long* scr;        // scratch of a row compacted in place, -1: the row moves
+    long long* fin;        // where they go
+    long long* scr;        // ... by way of scratch slots in place, -1: the row moves
     unsigned* chunk_row;   // per chunk: its row's place in the list
-    int* chunk_live;       // ... live entries, and those before it in its row
+    int* chunk_live;       // ... entries that move, and those before it in its row
     int* chunk_off;
     uint2* place;          // per overflowed end: its slot and its partner's (without twins: 64 bits)
     int* gidx;             // per vertex: 1 + its place in the list (0 = not growing)
@@ -204,6 +206,8 @@ struct UpdParams {
     unsigned long long hmask;
     int4* ovf;        // ends that did not fit their row: (row, col, wt, 2 * record + side)
     long long* slot;  // of their records, both directions: slot of the entry, -1 - k = the row's k-th overflow
+    uint4* tail_list; // chunks of long row tails to scan for a deletion: slots, length, column, weight
+    unsigned tail_cap;
     unsigned epoch;
     int te;           // edges per thread item
     int large_deg;    // rows above this become CTA items

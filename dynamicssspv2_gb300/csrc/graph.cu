@@ -486,6 +486,7 @@ struct dsssp_graph {
     long long grow_rows = 0, grow_chunks = 0, grow_ends = 0;  // what the work arrays hold
     unsigned long long s_spare[2] = {0, 0};  // spare words saved with the snapshot
     long long s_spare_lo = 0;                // and the first slot of its spare region
+    uint4* d_tails = nullptr;   // chunks of long row tails a batch's deletions search
     DelSlot* d_hset = nullptr;  // deletion set of the batch
     unsigned long long hcap = 0;
     Ctl* h_ctl = nullptr;  // pinned mirror of the control block
@@ -625,6 +626,9 @@ int ensure_work(dsssp_graph* g) {
     return rc;
 }
 
+// Places of the list of long row tails: what does not fit is scanned by the deletions' warps.
+long long tail_capacity(long long chg_cap) { return chg_cap < (1 << 18) ? chg_cap : (1 << 18); }
+
 int ensure_batch(dsssp_graph* g, long long k) {
     if (k <= g->chg_cap) return DSSSP_OK;
     long long cap = k + k / 4 + 1024;
@@ -633,6 +637,7 @@ int ensure_batch(dsssp_graph* g, long long k) {
     dfree(g->d_chg);
     dfree(g->d_ovf);
     dfree(g->d_hset);
+    dfree(g->d_tails);
     dfree(g->d_slot);
     dfree(g->d_seedq);
     g->chg_cap = 0;
@@ -640,6 +645,7 @@ int ensure_batch(dsssp_graph* g, long long k) {
     int rc = dalloc(&g->d_chg, (size_t)cap, "change buffer");
     if (!rc) rc = dalloc(&g->d_ovf, (size_t)cap * 2, "overflow buffer");
     if (!rc) rc = dalloc(&g->d_hset, (size_t)h, "deletion set");
+    if (!rc) rc = dalloc(&g->d_tails, (size_t)tail_capacity(cap), "tail list");
     if (!rc) rc = dalloc(&g->d_slot, (size_t)cap * 2, "slot buffer");
     const long long gl = 2 * cap < g->n ? 2 * cap : g->n;
     if (!rc) rc = dalloc(&g->d_seedq, (size_t)gl, "seed list");
@@ -665,7 +671,7 @@ int ensure_grow(dsssp_graph* g, cudaStream_t s) {
     dfree(g->d_grow);
     g->grow_rows = g->grow_chunks = g->grow_ends = 0;
     const size_t R = ((size_t)rows + 1) & ~(size_t)1, C = ((size_t)chunks + 1) & ~(size_t)1, E = (size_t)ends;
-    int rc = dalloc(&g->d_grow, R * (7 * 4 + 2 * 8) + C * 12 + E * 8, "row growth");
+    int rc = dalloc(&g->d_grow, R * (8 * 4 + 2 * 8) + C * 12 + E * 8, "row growth");
     if (rc) return rc;
     DevGrow& q = g->grow;
     unsigned char* at = g->d_grow;
@@ -679,6 +685,7 @@ int ensure_grow(dsssp_graph* g, cudaStream_t s) {
     carve(q.row, R);
     carve(q.chunk0, R);
     carve(q.done, R);
+    carve(q.first, R);
     carve(q.live, R);
     carve(q.lsorted, R);
     carve(q.ndeg, R);
@@ -879,6 +886,8 @@ UpdParams make_params(const dsssp_graph* g, const int4* chg, long long k, int mo
     p.hmask = g->hcap ? g->hcap - 1 : 0;
     p.ovf = g->d_ovf;
     p.slot = g->d_slot;
+    p.tail_list = g->d_tails;
+    p.tail_cap = (unsigned)tail_capacity(g->chg_cap);
     p.grow = g->grow;
     p.grow.slack_min = g->o.slack_min > 4 ? g->o.slack_min : 4;
     p.epoch = g->epoch;
@@ -1382,7 +1391,7 @@ void dsssp_graph_destroy(dsssp_graph* g) {
     dfree(d.state); dfree(d.rows); dfree(d.sorted_len); dfree(d.adj); dfree(d.inv_tag);
     dfree(d.push_tag); dfree(d.jm); dfree(d.invq); dfree(d.rt0); dfree(d.rt1); dfree(d.rc0); dfree(d.rc1);
     dfree(d.it); dfree(d.ic); dfree(d.ctl); dfree(d.far0); dfree(d.far1); dfree(d.far_tag); dfree(d.chg_tag);
-    dfree(g->d_chg); dfree(g->d_ovf); dfree(g->d_hset); dfree(d.twin); dfree(g->s_twin);
+    dfree(g->d_chg); dfree(g->d_ovf); dfree(g->d_hset); dfree(g->d_tails); dfree(d.twin); dfree(g->s_twin);
     dfree(g->d_par); dfree(g->d_dist); dfree(g->d_vtx); dfree(g->d_count); dfree(g->d_srcs); dfree(g->d_slot); dfree(g->d_seedq); dfree(g->d_spare);
     dfree(g->d_gidx); dfree(g->d_grow);
     dfree(g->s_state); dfree(g->s_rows); dfree(g->s_sorted); dfree(g->s_adj);

@@ -1445,13 +1445,6 @@ __device__ unsigned long long tombstone_prefix(const UpdParams& p, const RowDesc
     return probed;
 }
 
-__device__ unsigned long long tombstone_tail(const UpdParams& p, long long lo, long long hi, int col, int w,
-                                             bool with_twin, unsigned long long& dead) {
-    for (long long j = lo; j < hi; j++)
-        if (p.g.adj[j].x == col && p.g.adj[j].y == w) dead += tombstone_at(p, j, w, with_twin);
-    return (unsigned long long)(hi > lo ? hi - lo : 0);
-}
-
 // The whole row: the sorted prefix by binary search, the tail by this thread.
 __device__ unsigned long long tombstone_row(const UpdParams& p, const RowDesc& rd, int sorted_len, int col, int w,
                                             bool with_twin, unsigned long long& dead) {
@@ -1461,25 +1454,75 @@ __device__ unsigned long long tombstone_row(const UpdParams& p, const RowDesc& r
     unsigned long long probed = 1;
     for (; j < sl && adj[j].x == col; j++, probed++)
         if (adj[j].y == w) dead += tombstone_at(p, j, w, with_twin);
-    for (j = sl; j < end; j++, probed++)
-        if (adj[j].x == col && adj[j].y == w) dead += tombstone_at(p, j, w, with_twin);
+    probed += (unsigned long long)(end > sl ? end - sl : 0);
+    for (j = sl; j < end; j += 4) {  // four loads in flight
+        int2 e[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) e[k] = j + k < end ? adj[j + k] : make_int2(-1, -1);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (e[k].x == col && e[k].y == w) dead += tombstone_at(p, j + k, w, with_twin);
+    }
     return probed;
 }
 
-// Unsorted tails longer than this are scanned by the whole warp, 32 consecutive entries per
-// step, instead of by the deletion's own lane: under sustained insertion and deletion the tails
-// of hub rows grow to thousands of entries until the row is compacted or the adjacency is
-// repacked.  The deletion's lane lists such a tail in its warp's staging; the warp scans the
-// listed tails after its records (a lane whose warp's list is full scans its tail itself).
-constexpr long long kCoopTail = 64;
-constexpr int kTailList = 32;
-struct LongTail {
-    long long lo, hi;
-    int col, w;
-    bool twin;
-};
-__shared__ LongTail s_tails[kMaxWarps][kTailList];
-__shared__ unsigned s_ntails[kMaxWarps];
+// Unsorted tails of rows.  Under sustained insertion and deletion they grow until the row is compacted
+// or the adjacency is repacked, on hub rows to thousands of entries.  A deletion's lane scans up
+// to kShortTail of them itself (four loads in flight); the warp scans its 32 deletions' longer ones
+// together, their entries side by side, 128 in flight; a tail above kLongTail goes to the batch's
+// list in chunks, which k_append's warps scan (its appends lie behind every tail).  Bound: the
+// latency of the loads, so many are kept in flight, and the longest tail, so it is cut up.  RMAT
+// scale 22, a stream of 10^6 changes with 2.5 * 10^7 tail entries a batch: k_delete 0.36 -> 0.27 ms
+// against the tails of a warp one after the other, 32 entries at a time (0.14 without tails).
+// kShortTail 8 or 32: the same there, 64 pooled ER graphs 0.101 and 0.085 ms of the front kernels
+// against 0.085 at 16; 6 CTAs per SM (40 registers) against 4: 0.30 -> 0.27 ms.
+constexpr int kShortTail = 16;
+constexpr int kLongTail = 512;
+constexpr unsigned kTailChunk = 1024;
+constexpr unsigned kNoPair = 0x80000000u;  // in a tail's weight: leave the twins alone (weights are below 2^31)
+
+// One tail per lane (len 0: none), scanned by the warp; w carries kNoPair.  Returns the entries
+// this lane tombstoned.
+__device__ __forceinline__ unsigned scan_tails(const UpdParams& p, long long lo, unsigned len, int col, unsigned w) {
+    const unsigned lane = lane_id();
+    const unsigned incl = warp_incl_scan(len), total = __shfl_sync(kFull, incl, 31);
+    unsigned dead = 0;
+    for (unsigned b = 0; b < total; b += 128) {
+        long long j[4];
+        int2 e[4];
+        unsigned own[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const unsigned pos = b + 32 * k + lane;
+            unsigned o = 0;  // the first lane whose tails end behind pos
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1)
+                if (__shfl_sync(kFull, incl, o + s - 1) <= pos) o += s;
+            own[k] = o & 31u;
+            j[k] = __shfl_sync(kFull, lo, own[k]) + (pos - (__shfl_sync(kFull, incl, own[k]) - __shfl_sync(kFull, len, own[k])));
+            e[k] = pos < total ? p.g.adj[j[k]] : make_int2(-1, -1);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int c = __shfl_sync(kFull, col, own[k]);
+            const unsigned x = __shfl_sync(kFull, w, own[k]);
+            if (e[k].x == c && (unsigned)e[k].y == (x & ~kNoPair))
+                dead += tombstone_at(p, j[k], (int)(x & ~kNoPair), (x & kNoPair) == 0);
+        }
+    }
+    return dead;
+}
+
+// Lists a long tail in chunks; false when the list is full (its last places stay empty chunks).
+__device__ __forceinline__ bool list_tail(const UpdParams& p, long long lo, unsigned len, int col, unsigned w) {
+    const unsigned n = (len + kTailChunk - 1) / kTailChunk;
+    const unsigned at = atomicAdd(&p.g.ctl->tail_count, n);
+    const bool fits = at < p.tail_cap && n <= p.tail_cap - at;
+    for (unsigned k = 0; k < n && at < p.tail_cap && k < p.tail_cap - at; k++, lo += kTailChunk)
+        p.tail_list[at + k] = make_uint4((unsigned)lo, (unsigned)((unsigned long long)lo >> 32) |
+                                         (fits ? min(kTailChunk, len - k * kTailChunk) << 8 : 0u), (unsigned)col, w);
+    return fits;
+}
 
 }  // namespace
 
@@ -1507,27 +1550,26 @@ __global__ void k_prepare(UpdParams p) {
 
 // Deletions: cut off the child end of a deleted tree edge, tombstone every matching entry,
 // record the deletion in the batch's deletion set.
-// kTails: rows may hold unsorted tails (entries appended since the last layout), and long ones
-// are scanned warp-wide; without, every tail is scanned by its deletion's lane (the host picks
-// this form after a layout, a repack or a compaction, until a batch appends again: the long-tail
-// path alone costs the kernel a few percent).
+// kTails: rows may hold unsorted tails (entries appended since the last layout); without, every tail
+// is scanned by its deletion's lane (the host picks this form after a layout, a repack or a
+// compaction, until a batch appends again: the long-tail path alone costs the kernel a few
+// percent).
 template <bool kTails>
-__global__ void k_delete(UpdParams p) {
+__global__ void __launch_bounds__(256, 6) k_delete(UpdParams p) {
     Ctl* ctl = p.g.ctl;
     if (__ldcg(&ctl->status) != 0) return;  // set by k_prepare: same for every thread
     const long long nthreads = (long long)gridDim.x * blockDim.x;
     unsigned long long probed = 0, roots = 0, dead = 0;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
-    if constexpr (kTails) {
-        if (lane == 0) s_ntails[warp] = 0;
-        __syncwarp();
-    }
     WarpList roots_list{s_wlist[warp], kListRegion, 0};
     for (long long base = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; base < p.k; base += nthreads) {
         const long long i = base + lane;
         const int4 c = i < p.k ? p.chg[i] : make_int4(0, 0, 0, -1);
         bool cut = false;
         unsigned cutv = 0;
+        long long tlo = 0;  // this lane's tail for the warp to scan
+        unsigned tlen = 0, tw = 0;
+        int tcol = 0;
         if (c.w == 0) {
             const unsigned a = (unsigned)c.x, b = (unsigned)c.y;
             // gpuFunctions_undir.cuh:189-198: the child end is checked as b first, then as a.
@@ -1552,15 +1594,17 @@ __global__ void k_delete(UpdParams p) {
                 // a self-loop's two entries lie in the one row: the search meets both, each is
                 // counted by its own compare-and-swap (by the other's twin store as well, a loop
                 // deleted by two records of a batch was counted twice)
-                const bool tw = a != b;
-                if (!kTails || rs.deg - sl <= kCoopTail) {  // a short unsorted tail: this lane scans it too
-                    probed += tombstone_row(p, rs, sl, col, c.z, tw, dead);
-                } else {  // a long one goes to the warp's list (or, when that is full, to this lane)
-                    long long tlo, thi;
-                    probed += tombstone_prefix(p, rs, sl, col, c.z, tw, dead, tlo, thi);
-                    const unsigned at = atomicAdd(&s_ntails[warp], 1u);
-                    if (at < (unsigned)kTailList) s_tails[warp][at] = LongTail{tlo, thi, col, c.z, tw};
-                    else probed += tombstone_tail(p, tlo, thi, col, c.z, tw, dead);
+                const bool pair = a != b;
+                if (!kTails || rs.deg - sl <= kShortTail) {
+                    probed += tombstone_row(p, rs, sl, col, c.z, pair, dead);
+                } else {
+                    long long thi;
+                    probed += tombstone_prefix(p, rs, sl, col, c.z, pair, dead, tlo, thi);
+                    tcol = col;
+                    tw = (unsigned)c.z | (pair ? 0u : kNoPair);
+                    if (c.z >= 0) tlen = (unsigned)(thi - tlo);  // a negative weight matches nothing
+                    probed += tlen;
+                    if (tlen > (unsigned)kLongTail && list_tail(p, tlo, tlen, tcol, tw)) tlen = 0;
                 }
             } else {
                 probed += tombstone_row(p, ra, p.g.sorted_len[a], (int)b, c.z, false, dead);
@@ -1568,21 +1612,10 @@ __global__ void k_delete(UpdParams p) {
             }
             if (c.z >= 0 && !hash_insert(p, dpair_key(a, b), c.z)) set_status(ctl, -4 /* deletion set full */);
         }
+        if constexpr (kTails) dead += scan_tails(p, tlo, tlen, tcol, tw);
         roots_list.add(cut, cutv);
         roots += cut ? 1 : 0;
         roots_list.flush(p.g.invq, &ctl->inv_count, (unsigned)p.g.n, 32, ctl);
-    }
-    if constexpr (kTails) {  // the listed long tails, each by the whole warp (32 entries per step)
-        __syncwarp();
-        const unsigned nt = min(s_ntails[warp], (unsigned)kTailList);
-        for (unsigned t = 0; t < nt; t++) {
-            const LongTail lt = s_tails[warp][t];
-            for (long long j = lt.lo + lane; j < lt.hi; j += 32) {
-                const int2 e = p.g.adj[j];
-                if (e.x == lt.col && e.y == lt.w) dead += tombstone_at(p, j, lt.w, lt.twin);
-            }
-            if (lane == 0) probed += (unsigned long long)(lt.hi - lt.lo);
-        }
     }
     roots_list.flush_cta(p.g.invq, &ctl->inv_count, (unsigned)p.g.n, ctl);
     block_add(&ctl->stat[ST_ROOTS], roots);
@@ -1616,6 +1649,29 @@ __global__ void k_append(UpdParams p) {
     const unsigned seed_cap = (unsigned)min(2 * p.k, (long long)g.n);  // distinct claimed ends
     LocalStats ls;
     unsigned long long killed = 0, ovf = 0, live_ins = 0;
+    const unsigned tails = min(__ldcg(&ctl->tail_count), p.tail_cap);
+    if (tails) {  // the long tails that k_delete listed, a chunk per warp at a time
+        unsigned dead = 0;
+        for (unsigned c = (unsigned)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); c < tails;
+             c += (unsigned)(nthreads >> 5)) {
+            const uint4 x = __ldcg(&p.tail_list[c]);
+            const long long lo = (long long)((unsigned long long)(x.y & 0xFFu) << 32 | x.x);
+            const unsigned len = x.y >> 8;
+            for (unsigned b = 0; b < len; b += 256) {
+                int2 e[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const unsigned o = b + 32 * k + lane;
+                    e[k] = o < len ? ld_stream(&g.adj[lo + o]) : make_int2(-1, -1);
+                }
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (e[k].x == (int)x.z && (unsigned)e[k].y == (x.w & ~kNoPair))
+                        dead += tombstone_at(p, lo + b + 32 * k + lane, e[k].y, (x.w & kNoPair) == 0);
+            }
+        }
+        block_add(&ctl->stat[ST_TOMBS], dead);
+    }
     for (long long base = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; base < p.k; base += nthreads) {
         const long long i = base + lane;
         const int4 c = i < p.k ? p.chg[i] : make_int4(0, 0, 0, -1);

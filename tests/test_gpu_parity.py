@@ -868,3 +868,63 @@ def test_growth_of_a_small_graph_under_larger_and_larger_batches():
             u, v, w = lines_after(n, u, v, w, ch)
             assert st.overflow_entries > 0 or k == 30
             assert g.health()["live"] == 2 * len(u) and g.validate()["violations"] == 0
+
+
+@pytest.mark.parametrize("tail", [1, 7, 8, 9, 40, 511, 512, 513, 1025, 40000])
+def test_deletions_in_unsorted_tails(tail):
+    """Deletions whose rows are unsorted tails of that length: hubs 0 and 1 take their entries by
+    insertion, among them parallel edges between the two and self-loops, which one batch deletes
+    (tails at the edges of a lane's, a warp's and the list's share; with the longest, more chunks
+    than the list holds).  Live counts and trees are exact, and the tombstones are those of the
+    deleted lines only."""
+    rng = np.random.default_rng(tail)
+    k = min(300, tail + 1)  # parallel edges 0-1, distinct weights
+    n = tail + 10
+    u, v, w = (np.ascontiguousarray(x, np.int32) for x in (np.arange(n - 1), np.arange(1, n), np.full(n - 1, 700)))
+    spread = rng.permutation(np.arange(2, n))[: max(0, tail - k)]
+    a = np.concatenate([np.zeros(len(spread)), np.ones(len(spread)), np.zeros(k), [0, 1, 5]])
+    b = np.concatenate([spread, spread, np.ones(k), [0, 1, 5]])
+    x = np.concatenate([rng.integers(1, 600, 2 * len(spread)), 1000 + np.arange(k), [3, 4, 5]])
+    order = rng.permutation(len(a))
+    ins = D.make_changes(a[order], b[order], x[order], np.ones(len(a)))
+    gone = D.make_changes(np.concatenate([np.zeros(k), [0, 1]]), np.concatenate([np.ones(k), [0, 1]]),
+                          np.concatenate([1000 + np.arange(k), [3, 4]]), np.zeros(k + 2))
+    missing = D.make_changes([0, 1, 0], [1, 0, 0], [999, 5000, -1], np.zeros(3))
+    with D.Graph(n, u, v, w, slack_pct=0, slack_min=2, spare_pct=400) as g:
+        g.tree_compute(0)
+        for ch, dead in ((ins, 0), (np.concatenate([gone[::2], missing]), 2 * len(gone[::2])),
+                         (np.concatenate([gone[1::2], gone[1::4]]), 2 * len(gone[1::2])), (ins[:40], 0)):
+            st = g.apply_batch(ch)
+            assert st.tombstoned == dead
+            p, d = g.tree_read()
+            check_against_oracle(n, u, v, w, ch, 0, p, d, f"tail {tail}")
+            u, v, w = lines_after(n, u, v, w, ch)
+            assert g.health()["live"] == 2 * len(u) and g.validate()["violations"] == 0
+
+
+def test_a_row_that_closes_up_beside_one_that_gives_up_its_tail():
+    """In one batch hub 0 closes up wholly (tombstones in its sorted prefix) and hub 1 only its
+    tail (tombstones there): the edges between the two, which move in one row and stay in the
+    other, are still found from both sides afterwards."""
+    n = 70
+    leaves = np.arange(2, 62)
+    one = lambda h, ids, w, op: D.make_changes(np.full(len(ids), h), ids, np.full(len(ids), w), np.full(len(ids), op))
+    u = np.concatenate([np.zeros(60), np.ones(60), np.zeros(5)]).astype(np.int32)
+    v = np.concatenate([leaves, leaves, np.ones(5)]).astype(np.int32)
+    w = np.concatenate([np.full(120, 50), 7 + np.arange(5)]).astype(np.int32)
+    between = D.make_changes(np.zeros(5), np.ones(5), 7 + np.arange(5), np.zeros(5))
+    steps = [np.concatenate([one(0, leaves[:30], 50, 0), one(1, leaves[:14], 9, 1)]),
+             np.concatenate([one(1, leaves[:14], 9, 0), one(0, leaves[:16], 11, 1)]),
+             np.concatenate([one(1, leaves[20:26], 8, 1), one(0, leaves[30:33], 6, 1)]),  # both overflow
+             between[::2], between[1::2]]
+    with D.Graph(n, u, v, w, slack_pct=0, slack_min=16) as g:
+        g.tree_compute(0)
+        for i, ch in enumerate(steps):
+            st = g.apply_batch(ch)
+            assert st.overflow_entries == (7 if i == 2 else 0)
+            assert st.tombstoned == 2 * int((ch["op"] == 0).sum())
+            p, d = g.tree_read()
+            check_against_oracle(n, u, v, w, ch, 0, p, d, f"step {i}")
+            u, v, w = lines_after(n, u, v, w, ch)
+            assert g.health()["live"] == 2 * len(u) and g.validate()["violations"] == 0
+        assert g.health()["spare_used"] == 0  # neither row moved
