@@ -1,12 +1,13 @@
 // grow.cuh -- growth of the rows that a batch's insertions overflow, on the device.
 //
 // k_append lists the insertions that found their row full (ovf), and with the first of them the row
-// itself, cut into chunks of kGrowChunk slots.  k_update then starts with the growth: a growing
-// row keeps only its live entries, in their order, so the sorted prefix stays sorted and the
-// tombstones are gone.  When those entries and the overflow fit its own region with an eighth of
-// them (at least one slot) to spare, the row is compacted in place, through scratch slots at the
-// free end of the spare region; otherwise it moves to a region of 2 * (live + overflow) +
-// slack_min slots from the spare region (a bump allocator).  Every moved entry leaves its final
+// itself, cut into chunks of kGrowChunk slots.  k_update then starts with the growth.  A row makes
+// room in the cheapest way that leaves an eighth of its live entries (at least one slot) free
+// behind the overflow: its unsorted tail alone gives up its tombstones (links that come and go live
+// there; the sorted prefix keeps its own, as after any deletion); else all live entries close up
+// in place, in their order, so the prefix stays sorted; else they move to a region of
+// 2 * (live + overflow) + slack_min slots from the spare region (a bump allocator).  In place goes
+// through scratch slots at the free end of the spare region.  Every moved entry leaves its final
 // slot in its old twin word, through which its partner and the batch's recorded slots find it.
 // The first four phases write only free slots, twin words and the work arrays: until the last
 // one (grow_finish) the rows stand as k_append left them, and grow_finish may be run again.
@@ -15,10 +16,12 @@
 // word) for many entries, a chain of dependent accesses and a barrier per phase for few.  A warp
 // per chunk, not per row: rows of 10^5 entries grow in a stream on a skewed graph, and a warp that
 // walked one alone took up to 2 ms.  Inside k_update, not as kernels with the host between them
-// (status read, eight launches, three synchronisations).  Per batch, growth included: 10,000
-// vertices and 1,000 changes 0.28 -> 0.21 ms, 300,000 and 12,345 changes 0.36 -> 0.29 ms, RMAT scale
-// 22 and 10^6 changes 1.66 -> 0.98 and 1.32 ms (a batch and its inverse, medians of a stream).
-// A handful of chunks is one CTA's work with block barriers: the grid's cost more than it.
+// (status read, eight launches, three synchronisations).  The tail alone where that does: a batch of a
+// stream on a skewed graph otherwise moved a sixteenth of the adjacency.  k_update, growth included:
+// 10,000 vertices and 1,000 changes 0.28 -> 0.20 ms (the batch), 300,000 and 12,345 changes 0.36 ->
+// 0.28 ms, RMAT scale 20 with 10^5 insertions 0.31 -> 0.20 (all live entries) -> 0.15 ms, RMAT scale
+// 22 and 10^6 changes, of which the growth 1.16 -> 0.22 and 0.52 -> 0.17 and 0.10 ms (a batch and
+// its inverse).  A handful of chunks is one CTA's work with block barriers: the grid's cost more.
 #pragma once
 
 // Chunks a row of `cap` slots is cut into (at least one: a row without slots grows too).
@@ -31,7 +34,6 @@ __device__ __forceinline__ void grow_list_row(const UpdParams& p, unsigned j, un
     p.grow.row[j] = (unsigned)r;
     p.grow.chunk0[j] = c0;
     p.grow.done[j] = 0;
-    p.grow.lsorted[j] = 0;
     p.grow.gidx[r] = (int)j + 1;
     for (unsigned q = 0; q < chunks; q++) p.grow.chunk_row[c0 + q] = j;
 }
@@ -85,8 +87,8 @@ struct GrowTeam {
     __device__ __forceinline__ unsigned warps() const { return threads >> 5; }
 };
 
-// Phase 1: live entries of every chunk; the warp that counts a row's last chunk ranks them and
-// decides where the row goes.
+// Phase 1: live entries of every chunk (and those of the prefix); the warp that counts a row's last
+// chunk decides what moves and where, and ranks it.
 __device__ void grow_plan(const UpdParams& p, const GrowTeam& t, unsigned chunks) {
     const DevGrow& q = p.grow;
     const unsigned lane = lane_id();
@@ -108,38 +110,57 @@ __device__ void grow_plan(const UpdParams& p, const GrowTeam& t, unsigned chunks
         n = __reduce_add_sync(kFull, n);
         ns = __reduce_add_sync(kFull, ns);
         const unsigned parts = grow_chunks(rd.cap);
-        unsigned total = n;
-        if (lane == 0) q.chunk_live[c] = (int)n;
-        if (parts == 1) {
-            if (lane == 0) {
-                q.chunk_off[c] = 0;
-                q.lsorted[j] = (int)ns;
-            }
-        } else {
+        unsigned total = n, sorted = ns;
+        if (parts > 1) {
             unsigned d = 0;
             if (lane == 0) {
-                atomicAdd(&q.lsorted[j], (int)ns);
+                q.chunk_live[c] = (int)(n | ns << 16);
                 __threadfence();
                 d = atomicAdd(&q.done[j], 1u);
             }
             if (__shfl_sync(kFull, d, 0) != parts - 1) continue;
             __threadfence();
-            total = 0;
+            total = sorted = 0;
+            for (unsigned b = lane; b < parts; b += 32) {
+                const unsigned x = (unsigned)__ldcg(&q.chunk_live[c0 + b]);
+                total += x & 0xFFFFu;
+                sorted += x >> 16;
+            }
+            total = __reduce_add_sync(kFull, total);
+            sorted = __reduce_add_sync(kFull, sorted);
+        }
+        const long long need = rd.deg - rd.cap;
+        const long long room = total / 8 > 1 ? total / 8 : 1;  // free slots left in place
+        const bool tail = sl + (long long)(total - sorted) + need + room <= rd.cap;
+        const long long live = tail ? total - sorted : total;  // the entries that move
+        if (parts == 1) {
+            if (lane == 0) {
+                q.chunk_live[c] = (int)live;
+                q.chunk_off[c] = 0;
+            }
+        } else {  // the chunks' shares of them, ranked
+            unsigned before = 0;
             for (unsigned b = 0; b < parts; b += 32) {
-                const unsigned x = b + lane < parts ? (unsigned)__ldcg(&q.chunk_live[c0 + b + lane]) : 0u;
-                const unsigned incl = warp_incl_scan(x);
-                if (b + lane < parts) q.chunk_off[c0 + b + lane] = (int)(total + incl - x);
-                total += __shfl_sync(kFull, incl, 31);
+                const bool has = b + lane < parts;
+                const unsigned x = has ? (unsigned)__ldcg(&q.chunk_live[c0 + b + lane]) : 0u;
+                const unsigned mine = (x & 0xFFFFu) - (tail ? x >> 16 : 0u);
+                const unsigned incl = warp_incl_scan(mine);
+                if (has) {
+                    q.chunk_live[c0 + b + lane] = (int)mine;
+                    q.chunk_off[c0 + b + lane] = (int)(before + incl - mine);
+                }
+                before += __shfl_sync(kFull, incl, 31);
             }
         }
         if (lane != 0) continue;
-        const long long live = total, need = rd.deg - rd.cap;
-        const long long room = live / 8 > 1 ? live / 8 : 1;  // free slots left after an in-place compaction
-        dropped += (unsigned)(rd.cap - live);
+        const int first = tail ? sl : 0;  // entries from here on move
+        q.first[j] = first;
         q.live[j] = (int)live;
-        if (live + need + room <= rd.cap) {
+        q.lsorted[j] = tail ? sl : (int)sorted;
+        dropped += (unsigned)(rd.cap - first - live);
+        if (tail || live + need + room <= rd.cap) {
             const unsigned long long at = atomicAdd(&p.g.ctl->scr_used, (unsigned long long)live);
-            q.fin[j] = rd.start;
+            q.fin[j] = rd.start + first;
             q.scr[j] = (long long)(__ldcg(&q.spare[1]) - at - (unsigned long long)live);  // checked by grow()
             q.ncap[j] = rd.cap;
         } else {
@@ -149,7 +170,7 @@ __device__ void grow_plan(const UpdParams& p, const GrowTeam& t, unsigned chunks
             q.scr[j] = -1;
             q.ncap[j] = (int)(nc > 0x7FFFFFFFLL ? 0x7FFFFFFFLL : nc);
         }
-        q.ndeg[j] = (int)(live + need);
+        q.ndeg[j] = (int)(first + live + need);
     }
     if (lane == 0 && dropped) atomicAdd(&p.g.ctl->grow_dropped, (unsigned long long)dropped);
 }
@@ -162,7 +183,8 @@ __device__ void grow_out(const UpdParams& p, const GrowTeam& t, unsigned chunks)
     for (unsigned c = t.warp(); c < chunks; c += t.warps()) {
         const unsigned j = __ldcg(&q.chunk_row[c]);
         const RowDesc rd = ld_row(&p.g.rows[__ldcg(&q.row[j])]);
-        const int lo = (int)(c - __ldcg(&q.chunk0[j])) * kGrowChunk, hi = min(lo + kGrowChunk, rd.cap);
+        const int c0 = (int)(c - __ldcg(&q.chunk0[j])) * kGrowChunk, hi = min(c0 + kGrowChunk, rd.cap);
+        const int lo = max(c0, __ldcg(&q.first[j]));
         const long long off = __ldcg(&q.chunk_off[c]), fin = __ldcg(&q.fin[j]) + off, scr = __ldcg(&q.scr[j]);
         const long long dst = scr >= 0 ? scr + off : fin;
         int idx = 0;
@@ -194,7 +216,8 @@ __device__ void grow_out(const UpdParams& p, const GrowTeam& t, unsigned chunks)
 }
 
 // Phase 3: every moved entry takes its partner's final slot, from the partner's forwarding pointer
-// when the partner's row grows too; else the partner stays and gets this entry's final slot.
+// when the partner moves too (its row grows, and not by its tail alone with the partner in the
+// prefix); else the partner stays and gets this entry's final slot.
 __device__ void grow_relink(const UpdParams& p, const GrowTeam& t, unsigned chunks) {
     const DevGrow& q = p.grow;
     const unsigned lane = lane_id();
@@ -211,6 +234,7 @@ __device__ void grow_relink(const UpdParams& p, const GrowTeam& t, unsigned chun
                 const int e = b + 32 * k + (int)lane;
                 tw[k] = e < live ? __ldcg(&p.g.twin[at0 + e]) : kNoTwin;
                 gi[k] = e < live ? __ldcg(&q.gidx[__ldcg(&p.g.adj[at0 + e].x)]) : 0;
+                if (gi[k] && __ldcg(&q.first[gi[k] - 1]) > 0 && (long long)tw[k] < __ldcg(&q.fin[gi[k] - 1])) gi[k] = 0;
                 if (tw[k] != kNoTwin && (long long)tw[k] >= p.g.cap_total) {  // internal error: report, skip
                     set_status(p.g.ctl, -4);
                     tw[k] = kNoTwin;
@@ -289,7 +313,7 @@ __device__ void grow_finish(const UpdParams& p, const GrowTeam& t, unsigned rows
     for (unsigned j = t.thread; j < rows; j += t.threads) {
         const unsigned r = __ldcg(&q.row[j]);
         RowDesc nr;
-        nr.start = __ldcg(&q.fin[j]);
+        nr.start = __ldcg(&q.fin[j]) - __ldcg(&q.first[j]);
         nr.deg = __ldcg(&q.ndeg[j]);
         nr.cap = __ldcg(&q.ncap[j]);
         p.g.rows[r] = nr;
