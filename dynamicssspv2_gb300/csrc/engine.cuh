@@ -119,7 +119,10 @@ struct __align__(128) Ctl {
     unsigned pjC;
     unsigned pjf[3];
     unsigned fc[2];  // near-far: far-list counts (double buffer)
-    unsigned pad4[19];
+    unsigned lsteps[3];  // local stretches of the walk, as rsteps and rstop
+    unsigned lstop[3];
+    unsigned walk_done;  // their items, listed in rt1 for the pull
+    unsigned pad4[12];
     // line 4b: near-far threshold reduction
     unsigned long long fmin;
     // small steps run by CTA 0 alone hand their end state to the grid here
