@@ -315,6 +315,14 @@ struct PushBuf {
         __syncwarp();
     }
 
+    // the same with the ballot of pred at hand
+    __device__ __forceinline__ void add_mask(unsigned mask, bool pred, unsigned v, const RowDesc& rd) {
+        if (pred)
+            buf[count + __popc(mask & ((1u << lane_id()) - 1u))] =
+                make_uint4(v, (unsigned)rd.deg, (unsigned)rd.start, (unsigned)((unsigned long long)rd.start >> 32));
+        count += __popc(mask);
+    }
+
     // warp-collective: expands the buffer once it could not take another kAddsPerCheck
     __device__ __forceinline__ void flush(const UpdParams& p, const Out& o, LocalStats& ls) {
         if (count <= kBuf - kAddsPerCheck) return;
@@ -471,8 +479,12 @@ __device__ __forceinline__ void warp_agg_min(bool offer, unsigned c, unsigned lo
 }
 
 // ---- per-edge operations ---------------------------------------------------------------
-// visit4 handles up to four adjacency entries per lane and is called by all 32 lanes.
-
+// visit4 handles up to four adjacency entries per lane (a, a + stride, ... while below n; none for
+// n <= 0) and is called by all 32 lanes.  A busy round is bound by random accesses (a neighbour's
+// state per entry, 130-150 G/s against about 280 from the L2 with nothing else to do) and
+// instructions in equal parts; prefetching the next items' entries did not help (1.36 -> 1.40 ms for
+// the tree of RMAT scale 22), reading the next item early and leaving a visit in which no lane
+// improved anything did (1.39 -> 1.35 ms).
 template <bool kAgg>
 struct RelaxOp {
     const UpdParams* p;
@@ -494,12 +506,11 @@ struct RelaxOp {
     __device__ __forceinline__ void end_group(unsigned) {}
     __device__ __forceinline__ void finish() { pb.flush_cta(*p, out, *ls); }
 
-    __device__ __forceinline__ void visit4(unsigned u, unsigned long long du, const long long (&j)[4],
-                                           const bool (&ok)[4]) {
+    __device__ __forceinline__ void visit4(unsigned u, unsigned long long du, const int2* a, int n, int stride) {
         unsigned long long* state = p->g.state;
         int2 e[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) e[q] = ok[q] ? ld_stream(&p->g.adj[j[q]]) : make_int2(0, -1);
+        for (int q = 0; q < 4; q++) e[q] = q * stride < n ? ld_stream(a + q * stride) : make_int2(0, -1);
         unsigned long long cur[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) cur[q] = e[q].y >= 0 && !direct ? __ldcg(&state[e[q].x]) : kInfState;
@@ -567,6 +578,8 @@ struct RelaxOp {
                 later[q] = push[q] && (e[q].y == 0 ? du : nd) >= far.T;
             }
         }
+        if (live) ls->edges_relax += (unsigned)(n <= 0 ? 0 : min(4, (n + stride - 1) / stride));
+        if (!__any_sync(kFull, push[0] || push[1] || push[2] || push[3])) return;
         unsigned ftag[4], ctag[4];
         RowDesc rd[4];
 #pragma unroll
@@ -578,22 +591,25 @@ struct RelaxOp {
             ctag[q] = want ? atomicExch(&p->g.push_tag[c], tag) : tag;
         }
         bool fl[4], doit[4];
-        unsigned fc[4], nadd = 0;
+        unsigned fc[4], m[4], nadd = 0;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             fl[q] = later[q] && ftag[q] != far.gen;
             fc[q] = (unsigned)e[q].x;
             doit[q] = push[q] && !later[q] && ctag[q] != tag;
-            nadd += __popc(__ballot_sync(kFull, doit[q]));
+            m[q] = __ballot_sync(kFull, doit[q]);
+            nadd += __popc(m[q]);
         }
-        pb.reserve(nadd, *p, out, *ls);
+        if (nadd) {
+            pb.reserve(nadd, *p, out, *ls);
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            ls->frontier += doit[q] ? 1 : 0;
-            pb.add(doit[q], (unsigned)e[q].x, rd[q]);
-            ls->edges_relax += ok[q] && live ? 1 : 0;
+            for (int q = 0; q < 4; q++) {
+                ls->frontier += doit[q] ? 1 : 0;
+                pb.add_mask(m[q], doit[q], (unsigned)e[q].x, rd[q]);
+            }
+            __syncwarp();
         }
-        far_append4(*p, far, fl, fc);
+        if (far.T != ~0ull) far_append4(*p, far, fl, fc);
     }
 };
 
@@ -611,15 +627,19 @@ struct MarkOp {
     __device__ __forceinline__ void end_group(unsigned) {}
     __device__ __forceinline__ void finish() { pb.flush_cta(*p, out, *ls); }
 
-    __device__ __forceinline__ void visit4(unsigned x, unsigned long long, const long long (&j)[4],
-                                           const bool (&ok)[4]) {
+    __device__ __forceinline__ void visit4(unsigned x, unsigned long long, const int2* a, int n, int stride) {
         unsigned long long* state = p->g.state;
         int2 e[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) e[q] = ok[q] ? ld_stream(&p->g.adj[j[q]]) : make_int2(0, -1);
-        unsigned long long s[4];
+        for (int q = 0; q < 4; q++) e[q] = q * stride < n ? ld_stream(a + q * stride) : make_int2(0, -1);
+        unsigned par[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) s[q] = e[q].y >= 0 ? __ldcg(&state[e[q].x]) : kInfState;
+        for (int q = 0; q < 4; q++)
+            par[q] = e[q].y >= 0 ? __ldcg(reinterpret_cast<const unsigned*>(&state[e[q].x])) : kNone;  // low word
+        ls->edges_inv += (unsigned)(n <= 0 ? 0 : min(4, (n + stride - 1) / stride));
+        bool child[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) child[q] = e[q].y >= 0 && par[q] == x;
         // a child is cut off even when already tagged: a root that an insertion of this batch
         // re-parented onto a vertex of a cut-off subtree must lose that distance.  The four
         // tag exchanges and degree loads go out before any result is used.
@@ -628,22 +648,24 @@ struct MarkOp {
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const unsigned c = (unsigned)e[q].x;
-            const bool child = e[q].y >= 0 && (unsigned)s[q] == x;
-            if (child) state[c] = kInfState;
-            old[q] = child ? atomicExch(&p->g.inv_tag[c], p->epoch) : p->epoch;
-            rd[q] = row_if(*p, child, c);
+            if (child[q]) state[c] = kInfState;
+            old[q] = child[q] ? atomicExch(&p->g.inv_tag[c], p->epoch) : p->epoch;
+            rd[q] = row_if(*p, child[q], c);
         }
-        unsigned nadd = 0;
+        unsigned m[4], nadd = 0;
 #pragma unroll
-        for (int q = 0; q < 4; q++) nadd += __popc(__ballot_sync(kFull, old[q] != p->epoch));
+        for (int q = 0; q < 4; q++) {
+            m[q] = __ballot_sync(kFull, old[q] != p->epoch);
+            nadd += __popc(m[q]);
+        }
         pb.reserve(nadd, *p, out, *ls);
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             const bool mark = old[q] != p->epoch;
             ls->marked += mark ? 1 : 0;
-            pb.add(mark, (unsigned)e[q].x, rd[q]);
-            ls->edges_inv += ok[q] ? 1 : 0;
+            pb.add_mask(m[q], mark, (unsigned)e[q].x, rd[q]);
         }
+        __syncwarp();
     }
 };
 
@@ -675,18 +697,17 @@ struct PullOp {
     __device__ __forceinline__ void begin_group(unsigned) { best = kInfState; need = false; }
     __device__ __forceinline__ void finish() { pb.flush_cta(*p, out, *ls); }
 
-    __device__ __forceinline__ void visit4(unsigned x, unsigned long long, const long long (&j)[4],
-                                           const bool (&ok)[4]) {
+    __device__ __forceinline__ void visit4(unsigned x, unsigned long long, const int2* a, int n, int stride) {
         unsigned long long* state = p->g.state;
         int2 e[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) e[q] = ok[q] ? ld_stream(&p->g.adj[j[q]]) : make_int2(0, -1);
+        for (int q = 0; q < 4; q++) e[q] = q * stride < n ? ld_stream(a + q * stride) : make_int2(0, -1);
         unsigned long long s[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) s[q] = e[q].y >= 0 ? __ldcg(&state[e[q].x]) : kInfState;
+        ls->edges_pull += (unsigned)(n <= 0 ? 0 : min(4, (n + stride - 1) / stride));
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            ls->edges_pull += ok[q] ? 1 : 0;
             if (e[q].y < 0 || s[q] == kInfState) continue;
             const unsigned long long nd = (s[q] >> 32) + (unsigned)e[q].y;
             if (nd >= kDistInf) {
@@ -755,44 +776,40 @@ __device__ void run_items(Op& op, const UpdParams& p, const Item* tl, unsigned n
     const unsigned lane = lane_id();
     const unsigned gtid = cta * blockDim.x + threadIdx.x;
     const unsigned nthreads = ncta * blockDim.x;
-    for (unsigned t = cta; t < nc; t += ncta) {
-        const Item it = __ldcg(&cl[t]);
+    // CTA items, split further while they are too few for the CTAs (a hub's row alone: 93 items of
+    // 1,024 edges, all of which push, took 39 us on as many CTAs, in quarters 20 us)
+    const unsigned parts = nc * 4 <= ncta ? 4u : nc * 2 <= ncta ? 2u : 1u;
+    for (unsigned t = cta; t < nc * parts; t += ncta) {
+        Item it = __ldcg(&cl[t / parts]);
         const unsigned long long du = __shfl_sync(kFull, op.prep(it.z), 0);
         if (op.skip(du)) continue;
+        if (parts > 1) {
+            const unsigned len = (it.w + parts - 1) / parts, from = min(it.w, len * (t % parts));
+            it = make_item(it.z, item_lo(it) + from, min(len, it.w - from));
+        }
         const long long lo = item_lo(it), hi = lo + (long long)it.w;
         op.begin_group(it.z);
-        for (long long b = lo; b < hi; b += 4LL * blockDim.x) {
-            long long j[4];
-            bool ok[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                j[q] = b + (long long)q * blockDim.x + threadIdx.x;
-                ok[q] = j[q] < hi;
-            }
-            op.visit4(it.z, du, j, ok);
-        }
+        for (long long b = lo; b < hi; b += 4LL * blockDim.x)
+            op.visit4(it.z, du, p.g.adj + b + threadIdx.x, (int)(hi - b) - (int)threadIdx.x, (int)blockDim.x);
         op.end_group(it.z);
     }
     // thread items: the item names its slots, so the adjacency loads go out alongside the
     // load of the vertex's own state (prep)
+    auto load = [&](unsigned i) {
+        return i < nt + nt2 ? __ldcg(i < nt ? &tl[i] : &tl2[i - nt]) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    Item ahead = load(gtid);
     for (unsigned base = gtid - lane; base < nt + nt2; base += nthreads) {
         const unsigned i = base + lane;
         const bool has = i < nt + nt2;
-        const Item it = has ? __ldcg(i < nt ? &tl[i] : &tl2[i - nt]) : make_uint4(0u, 0u, 0u, 0u);
+        const Item it = ahead;
+        ahead = load(i + nthreads);
         const unsigned long long du = has ? op.prep(it.z) : kDistInf;
         const long long lo = item_lo(it);
         const int cnt = (int)it.w;
         op.begin_lane(it.z);
-        for (int b = 0; b < p.te; b += 4) {  // warp-uniform trip count (visit4 is warp-collective)
-            long long j[4];
-            bool ok[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                ok[q] = b + q < cnt;
-                j[q] = lo + b + q;
-            }
-            op.visit4(it.z, du, j, ok);
-        }
+        for (int b = 0; b < p.te; b += 4)  // warp-uniform trip count (visit4 is warp-collective)
+            op.visit4(it.z, du, p.g.adj + lo + b, cnt - b, 1);
         op.end_lane(it.z, has && !op.skip(du));
     }
     op.finish();
