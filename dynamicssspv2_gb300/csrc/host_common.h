@@ -6,7 +6,12 @@
 #include <string>
 #include <vector>
 
+struct dsssp_graph;
+
 namespace dsssp {
+
+// dsssp_tree_read_range with parent ids less `shift` (a pooled graph's own ids).
+int tree_read_shifted(dsssp_graph* g, int32_t first, int32_t count, int32_t shift, int32_t* parent, int64_t* dist);
 
 void set_error(const char* fmt, ...);
 int fail(int code, const char* fmt, ...);

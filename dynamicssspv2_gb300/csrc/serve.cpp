@@ -390,11 +390,7 @@ int dsssp_pool_tree_read(dsssp_pool* p, int32_t graph, int32_t* parent, int64_t*
     if (!p || graph < 0 || graph >= p->count() || !parent || !dist) return fail(DSSSP_E_INVAL, "pool_tree_read: bad arguments");
     if (p->size(graph) == 0) return fail(DSSSP_E_INVAL, "pool_tree_read: graph %d was removed", graph);
     const int32_t a = (int32_t)p->first[(size_t)graph], nn = p->size(graph);
-    const int rc = dsssp_tree_read_range(p->g, a, nn, parent, dist);
-    if (rc) return rc;
-    for (int32_t x = 0; x < nn; x++)
-        if (parent[x] >= 0) parent[x] -= a;
-    return DSSSP_OK;
+    return dsssp::tree_read_shifted(p->g, a, nn, a, parent, dist);
 }
 
 int dsssp_pool_add_graph(dsssp_pool* p, int32_t n, int64_t m, const int32_t* u, const int32_t* v, const int32_t* w,

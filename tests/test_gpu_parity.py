@@ -928,3 +928,38 @@ def test_a_row_that_closes_up_beside_one_that_gives_up_its_tail():
             u, v, w = lines_after(n, u, v, w, ch)
             assert g.health()["live"] == 2 * len(u) and g.validate()["violations"] == 0
         assert g.health()["spare_used"] == 0  # neither row moved
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 1021, 1024, 5000])
+def test_tree_reads_into_pinned_and_pageable_memory(n):
+    """Every read of the tree gives the same into pageable memory (staged copies), pinned memory
+    (written by the kernel), pinned memory off a 16-byte boundary and a mix; nothing behind the
+    arrays is written."""
+    torch = pytest.importorskip("torch")
+    m = 2 * n if n > 8 else max(0, n - 1)
+    u, v, w = D.gen_er(n, m, 1, 100, n) if n > 8 else (np.arange(m, dtype=np.int32), np.arange(1, m + 1, dtype=np.int32),
+                                                        np.full(m, 5, np.int32))
+
+    def pinned(dtype, off):
+        t = torch.full((n + 9,), 77, dtype=torch.int32 if dtype != np.int64 else torch.int64).pin_memory()
+        return t.numpy().view(dtype)[off: off + n + 1]
+
+    with D.Graph(n, u, v, w) as g:
+        g.tree_compute(0)
+        want = g.tree_read()
+        want32 = g.tree_read32()
+        for off in (0, 1, 2, 3):
+            for par, dist in ((pinned(np.int32, off), pinned(np.int64, off)), (pinned(np.int32, off), np.full(n + 1, 77)),
+                              (np.full(n + 1, 77, np.int32), pinned(np.int64, off))):
+                g.tree_read(par[:n], dist[:n])
+                assert np.array_equal(par[:n], want[0]) and np.array_equal(dist[:n], want[1]) and par[n] == dist[n] == 77
+            par, dist = pinned(np.int32, off), pinned(np.uint32, off)
+            g.tree_read32(par[:n], dist[:n])
+            assert np.array_equal(par[:n], want32[0]) and np.array_equal(dist[:n], want32[1]) and par[n] == dist[n] == 77
+            only = pinned(np.uint32, off)
+            D._check(D._lib.dsssp_tree_read32(g.handle, None, only[:n].ctypes.data), "tree_read32")
+            assert np.array_equal(only[:n], want32[1]) and only[n] == 77
+            a, c = n // 3, n - n // 3  # a range that starts anywhere
+            par, dist = pinned(np.int32, off), pinned(np.int64, off)
+            D._check(D._lib.dsssp_tree_read_range(g.handle, a, c, par.ctypes.data, dist.ctypes.data), "tree_read_range")
+            assert np.array_equal(par[:c], want[0][a:]) and np.array_equal(dist[:c], want[1][a:]) and par[c] == dist[c] == 77
