@@ -196,7 +196,8 @@ struct DevGrow {
     int* chunk_off;
     uint2* place;          // per overflowed end: its slot and its partner's (without twins: 64 bits)
     int* gidx;             // per vertex: 1 + its place in the list (0 = not growing)
-    unsigned long long* spare;  // {top, end} of the spare region
+    unsigned long long* spare;      // {top, end} of the spare region
+    unsigned long long spare_from;  // its top before the batch: slots from here on are free
     int slack_min;
 };
 

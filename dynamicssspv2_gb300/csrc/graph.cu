@@ -908,6 +908,7 @@ UpdParams make_params(const dsssp_graph* g, const int4* chg, long long k, int mo
     p.tail_list = g->d_tails;
     p.tail_cap = (unsigned)tail_capacity(g->chg_cap);
     p.grow = g->grow;
+    p.grow.spare_from = (unsigned long long)g->spare_top;
     p.grow.slack_min = g->o.slack_min > 4 ? g->o.slack_min : 4;
     p.epoch = g->epoch;
     p.te = g->o.small_deg;

@@ -9,7 +9,7 @@
 // 2 * (live + overflow) + slack_min slots from the spare region (a bump allocator).  In place goes
 // through scratch slots at the free end of the spare region.  Every moved entry leaves its final
 // slot in its old twin word, through which its partner and the batch's recorded slots find it.
-// The first four phases write only free slots, twin words and the work arrays: until the last
+// The phases before the last write only free slots, twin words and the work arrays: until the last
 // one (grow_finish) the rows stand as k_append left them, and grow_finish may be run again.
 //
 // Bound: random sectors (a moved entry reads its partner's place and writes its partner's twin
@@ -87,8 +87,42 @@ struct GrowTeam {
     __device__ __forceinline__ unsigned warps() const { return threads >> 5; }
 };
 
+// The live entries of a chunk (slots [lo, hi) of the row at `start`) to dst, with a forwarding pointer
+// (their place from fin on) in each one's old twin word.  Warp-collective.
+__device__ __forceinline__ void grow_out_chunk(const UpdParams& p, long long start, int lo, int hi, long long dst,
+                                               long long fin) {
+    const unsigned lane = lane_id(), lt = (1u << lane) - 1u;
+    int idx = 0;
+    for (int b = lo; b < hi; b += 128) {
+        int2 x[4];
+        unsigned tw[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int e = b + 32 * k + (int)lane;
+            x[k] = e < hi ? __ldcg(&p.g.adj[start + e]) : make_int2(0, -1);
+            tw[k] = p.g.twin && e < hi ? __ldcg(&p.g.twin[start + e]) : kNoTwin;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const bool live = x[k].y >= 0;
+            const unsigned m = __ballot_sync(kFull, live);
+            if (live) {
+                const int at = idx + __popc(m & lt);
+                p.g.adj[dst + at] = x[k];
+                if (p.g.twin) {
+                    p.g.twin[dst + at] = tw[k];  // the partner's old slot, re-linked by the next phase
+                    p.g.twin[start + b + 32 * k + (int)lane] = (unsigned)(fin + at);
+                }
+            }
+            idx += __popc(m);
+        }
+    }
+}
+
 // Phase 1: live entries of every chunk (and those of the prefix); the warp that counts a row's last
-// chunk decides what moves and where, and ranks it.
+// chunk decides what moves and where, and ranks it.  A row of one chunk moves at once, if its slots
+// lie in the spare region (whether all do is known after the phase; what it writes is free until
+// then).
 __device__ void grow_plan(const UpdParams& p, const GrowTeam& t, unsigned chunks) {
     const DevGrow& q = p.grow;
     const unsigned lane = lane_id();
@@ -152,66 +186,48 @@ __device__ void grow_plan(const UpdParams& p, const GrowTeam& t, unsigned chunks
                 before += __shfl_sync(kFull, incl, 31);
             }
         }
-        if (lane != 0) continue;
         const int first = tail ? sl : 0;  // entries from here on move
-        q.first[j] = first;
-        q.live[j] = (int)live;
-        q.lsorted[j] = tail ? sl : (int)sorted;
-        dropped += (unsigned)(rd.cap - first - live);
-        if (tail || live + need + room <= rd.cap) {
-            const unsigned long long at = atomicAdd(&p.g.ctl->scr_used, (unsigned long long)live);
-            q.fin[j] = rd.start + first;
-            q.scr[j] = (long long)(__ldcg(&q.spare[1]) - at - (unsigned long long)live);  // checked by grow()
-            q.ncap[j] = rd.cap;
-        } else {
-            const long long nc = 2 * (live + need) + q.slack_min;
-            if (nc > 0x7FFFFFFFLL) atomicExch(&p.g.ctl->grow_fail, 1u);
-            q.fin[j] = (long long)atomicAdd(&q.spare[0], (unsigned long long)nc);
-            q.scr[j] = -1;
+        long long fin = rd.start + first, scr = -1;
+        if (lane == 0) {
+            q.first[j] = first;
+            q.live[j] = (int)live;
+            q.lsorted[j] = tail ? sl : (int)sorted;
+            q.ndeg[j] = (int)(first + live + need);
+            dropped += (unsigned)(rd.cap - first - live);
+            long long nc = rd.cap;
+            if (tail || live + need + room <= rd.cap) {
+                const unsigned long long at = atomicAdd(&p.g.ctl->scr_used, (unsigned long long)live);
+                scr = (long long)(__ldcg(&q.spare[1]) - at - (unsigned long long)live);  // checked by grow()
+            } else {
+                nc = 2 * (live + need) + q.slack_min;
+                if (nc > 0x7FFFFFFFLL) atomicExch(&p.g.ctl->grow_fail, 1u);
+                fin = (long long)atomicAdd(&q.spare[0], (unsigned long long)nc);
+            }
+            q.fin[j] = fin;
+            q.scr[j] = scr;
             q.ncap[j] = (int)(nc > 0x7FFFFFFFLL ? 0x7FFFFFFFLL : nc);
         }
-        q.ndeg[j] = (int)(first + live + need);
+        if (parts > 1) continue;
+        fin = __shfl_sync(kFull, fin, 0);
+        scr = __shfl_sync(kFull, scr, 0);
+        const long long dst = scr != -1 ? scr : fin;
+        if (dst >= (long long)q.spare_from && dst + live <= (long long)__ldcg(&q.spare[1]))
+            grow_out_chunk(p, rd.start, first, rd.cap, dst, fin);
     }
     if (lane == 0 && dropped) atomicAdd(&p.g.ctl->grow_dropped, (unsigned long long)dropped);
 }
 
-// Phase 2: the live entries to where their row goes (or its scratch), a forwarding pointer in
-// each one's old twin word.
+// Phase 2 (rows of several chunks): the live entries to where their row goes (or its scratch).
 __device__ void grow_out(const UpdParams& p, const GrowTeam& t, unsigned chunks) {
     const DevGrow& q = p.grow;
-    const unsigned lane = lane_id(), lt = (1u << lane) - 1u;
     for (unsigned c = t.warp(); c < chunks; c += t.warps()) {
         const unsigned j = __ldcg(&q.chunk_row[c]);
         const RowDesc rd = ld_row(&p.g.rows[__ldcg(&q.row[j])]);
+        if (grow_chunks(rd.cap) == 1) continue;  // moved by phase 1
         const int c0 = (int)(c - __ldcg(&q.chunk0[j])) * kGrowChunk, hi = min(c0 + kGrowChunk, rd.cap);
         const int lo = max(c0, __ldcg(&q.first[j]));
         const long long off = __ldcg(&q.chunk_off[c]), fin = __ldcg(&q.fin[j]) + off, scr = __ldcg(&q.scr[j]);
-        const long long dst = scr >= 0 ? scr + off : fin;
-        int idx = 0;
-        for (int b = lo; b < hi; b += 128) {
-            int2 x[4];
-            unsigned tw[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int e = b + 32 * k + (int)lane;
-                x[k] = e < hi ? __ldcg(&p.g.adj[rd.start + e]) : make_int2(0, -1);
-                tw[k] = p.g.twin && e < hi ? __ldcg(&p.g.twin[rd.start + e]) : kNoTwin;
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const bool live = x[k].y >= 0;
-                const unsigned m = __ballot_sync(kFull, live);
-                if (live) {
-                    const int at = idx + __popc(m & lt);
-                    p.g.adj[dst + at] = x[k];
-                    if (p.g.twin) {
-                        p.g.twin[dst + at] = tw[k];  // the partner's old slot, re-linked by the next phase
-                        p.g.twin[rd.start + b + 32 * k + (int)lane] = (unsigned)(fin + at);
-                    }
-                }
-                idx += __popc(m);
-            }
-        }
+        grow_out_chunk(p, rd.start, lo, hi, scr >= 0 ? scr + off : fin, fin);
     }
 }
 
@@ -251,8 +267,7 @@ __device__ void grow_relink(const UpdParams& p, const GrowTeam& t, unsigned chun
     }
 }
 
-// Phase 4: the final slot of every overflowed end and of its partner, which is told at once when
-// it did fit (it lies where phase 2 left it).
+// Beside it: the final slots of every overflowed end and of its partner.
 __device__ void grow_place(const UpdParams& p, const GrowTeam& t, unsigned novf) {
     const DevGrow& q = p.grow;
     for (unsigned o = t.thread; o < novf; o += t.threads) {
@@ -270,25 +285,15 @@ __device__ void grow_place(const UpdParams& p, const GrowTeam& t, unsigned novf)
             q.place[o] = make_uint2((unsigned)own, (unsigned)((unsigned long long)own >> 32));
             continue;
         }
-        long long partner = praw;
-        if (praw < 0) {
-            partner = __ldcg(&q.fin[pj]) + __ldcg(&q.live[pj]) + (-1 - praw);
-        } else {
-            long long cur = praw;
-            if (pj >= 0) {
-                const long long fin = __ldcg(&q.fin[pj]), scr = __ldcg(&q.scr[pj]);
-                partner = __ldcg(&p.g.twin[praw]);
-                cur = scr >= 0 ? scr + (partner - fin) : partner;
-            }
-            if (cur >= 0 && cur < p.g.cap_total) p.g.twin[cur] = (unsigned)own;
-            else set_status(p.g.ctl, -4);  // internal error
-        }
+        long long partner = praw;  // it fitted: where it is, or where its row's growth puts it
+        if (praw < 0) partner = __ldcg(&q.fin[pj]) + __ldcg(&q.live[pj]) + (-1 - praw);
+        else if (pj >= 0) partner = __ldcg(&p.g.twin[praw]);
         q.place[o] = make_uint2((unsigned)own, (unsigned)partner);
     }
 }
 
-// Phase 5: compacted rows back from their scratch, the overflowed ends behind the live entries, the
-// new descriptors.  Reads only what the phases before it wrote, so it may run again.
+// Phase 4: compacted rows back from their scratch, the overflowed ends behind the live entries with
+// their partners told (whose twin words say kNoTwin until then), the new descriptors.  Reads only what the phases before it wrote, so it may run again.
 __device__ void grow_finish(const UpdParams& p, const GrowTeam& t, unsigned rows, unsigned chunks, unsigned novf) {
     const DevGrow& q = p.grow;
     const unsigned lane = lane_id();
@@ -299,7 +304,9 @@ __device__ void grow_finish(const UpdParams& p, const GrowTeam& t, unsigned rows
         const int live = __ldcg(&q.chunk_live[c]);
         for (int e = (int)lane; e < live; e += 32) {
             p.g.adj[fin + e] = __ldcg(&p.g.adj[scr + off + e]);
-            if (p.g.twin) p.g.twin[fin + e] = __ldcg(&p.g.twin[scr + off + e]);
+            if (!p.g.twin) continue;
+            const unsigned tw = __ldcg(&p.g.twin[scr + off + e]);
+            if (tw != kNoTwin) p.g.twin[fin + e] = tw;  // else told below
         }
     }
     for (unsigned o = t.thread; o < novf; o += t.threads) {
@@ -308,7 +315,9 @@ __device__ void grow_finish(const UpdParams& p, const GrowTeam& t, unsigned rows
         const long long own = p.g.twin ? (long long)s.x : (long long)(((unsigned long long)s.y << 32) | s.x);
         if (own >= p.g.cap_total) continue;  // reported by grow_place
         p.g.adj[own] = make_int2(x.y, x.z);
-        if (p.g.twin) p.g.twin[own] = s.y;
+        if (!p.g.twin || (long long)s.y >= p.g.cap_total) continue;
+        p.g.twin[own] = s.y;
+        p.g.twin[s.y] = s.x;
     }
     for (unsigned j = t.thread; j < rows; j += t.threads) {
         const unsigned r = __ldcg(&q.row[j]);
@@ -322,8 +331,8 @@ __device__ void grow_finish(const UpdParams& p, const GrowTeam& t, unsigned rows
     }
 }
 
-// The spare region cannot take the moves and the scratch: nothing has been written, the host
-// repacks (which folds the overflow list in).
+// If the spare region cannot take the moves and the scratch, only slots that were free before the
+// batch have been written: the host repacks (which folds the overflow list in).
 __device__ __forceinline__ bool grow_fits(const UpdParams& p) {
     return __ldcg(&p.g.ctl->grow_fail) == 0 &&
            __ldcg(&p.grow.spare[0]) + __ldcg(&p.g.ctl->scr_used) <= __ldcg(&p.grow.spare[1]);
@@ -347,12 +356,10 @@ __device__ __noinline__ bool grow(const UpdParams& p) {
             __threadfence();
             __syncthreads();
             if (grow_fits(p)) {
-                grow_out(p, t, chunks);
+                if (chunks != rows) grow_out(p, t, chunks);
                 __threadfence();
                 __syncthreads();
                 if (p.g.twin) grow_relink(p, t, chunks);
-                __threadfence();
-                __syncthreads();
                 grow_place(p, t, novf);
                 __threadfence();
                 __syncthreads();
@@ -374,10 +381,11 @@ __device__ __noinline__ bool grow(const UpdParams& p) {
         grow_give_up(p, t, rows);
         return false;
     }
-    grow_out(p, t, chunks);
-    if (!grid_sync(ctl)) return false;
+    if (chunks != rows) {  // some row has several
+        grow_out(p, t, chunks);
+        if (!grid_sync(ctl)) return false;
+    }
     if (p.g.twin) grow_relink(p, t, chunks);
-    if (!grid_sync(ctl)) return false;
     grow_place(p, t, novf);
     __syncthreads();
     if (threadIdx.x == 0) {
