@@ -33,6 +33,7 @@ constexpr unsigned long long kDistInf = 0xFFFFFFFFull;
 constexpr unsigned kTagOk = 0xFFFFFFFFu;   // pointer jumping: reaches the root untouched
 constexpr unsigned kTagInv = 0xFFFFFFFEu;  // pointer jumping: below a cut-off vertex
 constexpr int kStatusOverflowPending = 1;  // internal: the spare region cannot take the growing rows
+constexpr unsigned kRefusedWeight = 1, kRefusedVertex = 2;  // why k_prepare refused a batch
 constexpr int kGrowChunk = 256;            // slots of a growing row that one warp handles
 constexpr unsigned kNoTwin = 0xFFFFFFFFu;   // twin not known yet (the other end overflowed)
 constexpr unsigned long long kHashEmpty = 0xFFFFFFFFFFFFFFFFull;
@@ -74,10 +75,12 @@ enum StatIdx {
     ST_SEED_UPD,    // k_append: distance-lowering seed relaxations
     ST_SEED_FRONT,  // k_append: ends claimed for the first frontier (or the far list)
     ST_EDGES_PULL,  // adjacency entries scanned by the pulls of cut-off vertices
+    ST_KILLED,      // insertions removed by a deletion of the same batch
     ST_COUNT
 };
 
-// Device control block.  Everything from line 1 on is cleared before every batch.
+// Device control block.  Everything from line 1 on is cleared before every computation, by k_prepare
+// for a batch.
 struct __align__(128) Ctl {
     // line 0 (persistent)
     unsigned bar_gen;
@@ -85,12 +88,13 @@ struct __align__(128) Ctl {
     unsigned spin_limit;  // grid-barrier poll limit (0 = default); persistent, set by the host
     unsigned stall_us;    // test hook: the last CTA of k_update waits this long before its first barrier
     unsigned grp_gen;     // generation of the group barrier (the first group_ctas CTAs)
-    unsigned pad0[27];
+    unsigned pad0a;
+    unsigned long long refused;  // (epoch << 32) | why, of the last batch that k_prepare refused
+    unsigned pad0[24];
     // line 1
     int status;
     int ovf_count;       // ends of insertions that found their row full
     unsigned inv_count;  // roots appended by k_delete
-    unsigned killed;     // insertions removed by a deletion of the same batch
     unsigned seed_count;  // vertices k_append seeded into the first frontier
     unsigned grow_fail;   // row growth: a row of more than 2^31 slots
     unsigned long long grow_list;     // growing rows (low word) and their chunks (high word)
@@ -139,6 +143,8 @@ struct __align__(128) Ctl {
     unsigned long long ts[8];
     unsigned long long pad6[8];
 };
+
+static_assert(sizeof(Ctl) % 128 == 0, "the control block is whole lines");
 
 // A work item: adjacency slots [lo, lo + cnt) of vertex v's row, as {lo low word, lo high
 // word, v, cnt} (one 16-byte load).
@@ -204,7 +210,8 @@ struct DevGrow {
 struct UpdParams {
     DevGraph g;
     DevGrow grow;
-    const int4* chg;  // (u, v, w, op) records
+    int4* chg;        // (u, v, w, op) records
+    const int4* chg_src;  // where they come from in pinned host memory (nullptr: they are in chg)
     long long k;
     DelSlot* hset;    // deletion set: endpoint pair -> weight (open addressing)
     unsigned long long hmask;

@@ -516,7 +516,7 @@ struct dsssp_graph {
     // the batch launch sequence as an instantiated CUDA graph (opts.launch_graph)
     cudaGraph_t bgraph = nullptr;
     cudaGraphExec_t bexec = nullptr;
-    cudaGraphNode_t bn_hash = nullptr, bn_kern[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaGraphNode_t bn_kern[4] = {nullptr, nullptr, nullptr, nullptr};
     int bgraph_timing = 0;  // the timing level the instantiated graph records
     int bgraph_agg = 0;     // the update kernel it launches (opts.warp_agg)
     int bgraph_tails = 0;   // the deletion kernel it launches (tails)
@@ -899,7 +899,8 @@ UpdParams make_params(const dsssp_graph* g, const int4* chg, long long k, int mo
     p.g.n = g->n;
     p.g.src = g->src;
     p.g.cap_total = g->cap_total;
-    p.chg = chg;
+    p.chg = const_cast<int4*>(chg);  // written only when the records come from the host (chg_src)
+    p.chg_src = nullptr;
     p.k = k;
     p.hset = g->d_hset;
     p.hmask = g->hcap ? g->hcap - 1 : 0;
@@ -939,6 +940,7 @@ int next_epoch(dsssp_graph* g, cudaStream_t s) {
     if (g->epoch >= 0xFFFFFFF0u) {
         CK(cudaMemsetAsync(g->dg.inv_tag, 0, sizeof(unsigned) * (size_t)g->n, s), "tag reset");
         CK(cudaMemsetAsync(g->dg.chg_tag, 0, sizeof(unsigned) * (size_t)g->n, s), "tag reset");
+        CK(cudaMemsetAsync(&g->dg.ctl->refused, 0, sizeof(g->dg.ctl->refused), s), "tag reset");
         g->epoch = 0;
     }
     g->epoch++;
@@ -1007,7 +1009,7 @@ void fill_stats(const dsssp_graph* g, const Ctl& c, dsssp_stats* st, bool events
             if (cudaEventElapsedTime(&ap, g->ev[5], g->ev[1]) == cudaSuccess) st->t_append_ms = ap;
         }
     }
-    st->n_killed = (int64_t)c.killed;
+    st->n_killed = (int64_t)c.stat[ST_KILLED];
     st->work_items = (int64_t)c.stat[ST_ITEMS];
     st->advances = (int64_t)c.stat[ST_ADVANCES];
     st->tombstoned = (int64_t)c.stat[ST_TOMBS];
@@ -1048,10 +1050,9 @@ struct BatchNodes {
     UpdParams p;
     void* args[1];
     cudaKernelNodeParams kp[4];
-    cudaMemsetParams hash;
 };
 
-void batch_nodes(const dsssp_graph* g, const UpdParams& p, unsigned long long h, BatchNodes& b) {
+void batch_nodes(const dsssp_graph* g, const UpdParams& p, BatchNodes& b) {
     const void* fns[4];
     batch_kernels(fns);
     fns[1] = delete_kernel(p.tails != 0);
@@ -1070,13 +1071,6 @@ void batch_nodes(const dsssp_graph* g, const UpdParams& p, unsigned long long h,
         k.kernelParams = b.args;
         k.extra = nullptr;
     }
-    memset(&b.hash, 0, sizeof(b.hash));
-    b.hash.dst = g->d_hset;
-    b.hash.value = 0xFF;
-    b.hash.elementSize = 1;
-    b.hash.width = sizeof(DelSlot) * (size_t)h;
-    b.hash.height = 1;
-    b.hash.pitch = 0;
 }
 
 void drop_batch_graph(dsssp_graph* g) {
@@ -1086,8 +1080,7 @@ void drop_batch_graph(dsssp_graph* g) {
     g->bgraph = nullptr;
 }
 
-// Builds and instantiates the batch graph: [event 0] control-block reset, deletion-set reset,
-// k_prepare, [event 4], k_delete, [event 5], k_append, [event 1] k_update (cooperative),
+// Builds and instantiates the batch graph: [event 0] k_prepare, [event 4], k_delete, [event 5], k_append, [event 1] k_update (cooperative),
 // [event 2] status read.  Events 0-2 are recorded at timing level 1, events 4-5 at level 2.
 cudaError_t build_batch_graph(dsssp_graph* g, const BatchNodes& b, int timing) {
     drop_batch_graph(g);
@@ -1098,21 +1091,6 @@ cudaError_t build_batch_graph(dsssp_graph* g, const BatchNodes& b, int timing) {
     cudaGraphNode_t prev = nullptr, n = nullptr;
     auto dep = [&]() { return prev ? 1 : 0; };
     if (timing && (e = cudaGraphAddEventRecordNode(&n, gr, &prev, dep(), g->ev[0])) == cudaSuccess) prev = n;
-    if (e == cudaSuccess) {
-        cudaMemsetParams c;
-        memset(&c, 0, sizeof(c));
-        const size_t off = offsetof(Ctl, status);  // line 1 onwards, as clear_ctl
-        c.dst = (char*)g->dg.ctl + off;
-        c.value = 0;
-        c.elementSize = 1;
-        c.width = sizeof(Ctl) - off;
-        c.height = 1;
-        if ((e = cudaGraphAddMemsetNode(&n, gr, &prev, dep(), &c)) == cudaSuccess) prev = n;
-    }
-    if (e == cudaSuccess && (e = cudaGraphAddMemsetNode(&n, gr, &prev, dep(), &b.hash)) == cudaSuccess) {
-        prev = n;
-        g->bn_hash = n;
-    }
     for (int i = 0; i < 4 && e == cudaSuccess; i++) {
         if (i == 3 && timing && (e = cudaGraphAddEventRecordNode(&n, gr, &prev, dep(), g->ev[1])) == cudaSuccess)
             prev = n;
@@ -1149,16 +1127,15 @@ cudaError_t build_batch_graph(dsssp_graph* g, const BatchNodes& b, int timing) {
 }
 
 // Replays the batch graph with this batch's parameters; false = use plain launches.
-bool launch_batch_graph(dsssp_graph* g, const UpdParams& p, unsigned long long h, cudaStream_t s) {
+bool launch_batch_graph(dsssp_graph* g, const UpdParams& p, cudaStream_t s) {
     if (!g->o.launch_graph || g->bgraph_failed || p.k <= 0) return false;
     BatchNodes b;
-    batch_nodes(g, p, h, b);
+    batch_nodes(g, p, b);
     const int timing = g->o.timing;
     cudaError_t e = cudaSuccess;
     if (!g->bexec || g->bgraph_timing != timing || g->bgraph_agg != p.warp_agg || g->bgraph_tails != p.tails) {
         e = build_batch_graph(g, b, timing);
     } else {
-        e = cudaGraphExecMemsetNodeSetParams(g->bexec, g->bn_hash, &b.hash);
         for (int i = 0; i < 4 && e == cudaSuccess; i++) e = cudaGraphExecKernelNodeSetParams(g->bexec, g->bn_kern[i], &b.kp[i]);
     }
     if (e == cudaSuccess) e = cudaGraphLaunch(g->bexec, s);
@@ -1172,8 +1149,8 @@ bool launch_batch_graph(dsssp_graph* g, const UpdParams& p, unsigned long long h
     return true;
 }
 
-// Enqueues one batch (records already on the device).
-int enqueue_batch(dsssp_graph* g, const int4* d_chg, long long k, cudaStream_t s) {
+// Enqueues one batch (records on the device, or in pinned host memory at src and bound for d_chg).
+int enqueue_batch(dsssp_graph* g, const int4* d_chg, const int4* src, long long k, cudaStream_t s) {
     // k_append already claims frontier tags: restart the tag sequence before it could wrap
     // (the mirror holds the round base the last kernel left)
     if (g->h_ctl->round_base > 0xF0000000u) reset_tags(g, g->stream);
@@ -1186,14 +1163,12 @@ int enqueue_batch(dsssp_graph* g, const int4* d_chg, long long k, cudaStream_t s
     while (h < hb) h <<= 1;  // this batch uses the first h slots of the deletion set
     UpdParams p = make_params(g, d_chg, k, 0);
     p.hmask = h - 1;
+    p.chg_src = src;
     g->pend_rb0 = g->h_ctl->round_base;  // the device reads the same value (mirror)
-    g->pend_graph = launch_batch_graph(g, p, h, s);
+    g->pend_graph = launch_batch_graph(g, p, s);
     if (g->pend_graph) return DSSSP_OK;
     const bool ev = g->o.timing != 0;
     if (ev) CK(cudaEventRecord(g->ev[0], s), "event");
-    int rc = clear_ctl(g, s);
-    if (rc) return rc;
-    CK(cudaMemsetAsync(g->d_hset, 0xFF, sizeof(DelSlot) * h, s), "deletion set reset");
     const bool fev = g->o.timing >= 2;
     CK(launch_front(p, g->num_sms * 8, s, fev ? g->ev[4] : nullptr, fev ? g->ev[5] : nullptr), "insert/delete kernels");
     if (ev) CK(cudaEventRecord(g->ev[1], s), "event");
@@ -1944,8 +1919,8 @@ int dsssp_tree_validate(dsssp_graph* g, int64_t* violations, int64_t* roots, int
     return DSSSP_OK;
 }
 
-int dsssp_apply_batch_async(dsssp_graph* g, const dsssp_change* d_changes, int64_t k, void* stream) {
-    if (!g || k < 0 || (k > 0 && !d_changes)) return fail(DSSSP_E_INVAL, "apply_batch: bad arguments");
+// d_changes: the records' place on the device; src: pinned host memory that they come from, or nullptr
+static int apply_impl(dsssp_graph* g, const int4* d_changes, const int4* src, int64_t k, void* stream) {
     int rc = set_device(g);
     if (rc) return rc;
     if (g->pending) return fail(DSSSP_E_INVAL, "apply_batch: previous batch not finished");
@@ -1960,14 +1935,19 @@ int dsssp_apply_batch_async(dsssp_graph* g, const dsssp_change* d_changes, int64
     if (!rc) rc = ensure_grow(g, s);
     if (!rc && g->copy_pending) CK(cudaStreamWaitEvent(s, g->ev_unpacked, 0), "apply_batch");  // a read's unpack
     if (!rc) rc = next_epoch(g, s);
-    if (!rc) rc = enqueue_batch(g, (const int4*)d_changes, k, s);
+    if (!rc) rc = enqueue_batch(g, d_changes, src, k, s);
     if (rc) return rc;
     g->pending = true;
     g->pend_k = k;
-    g->pend_chg = (const int4*)d_changes;
+    g->pend_chg = d_changes;
     g->pend_stream = s;
     g->pend_events = g->o.timing != 0;
     return DSSSP_OK;
+}
+
+int dsssp_apply_batch_async(dsssp_graph* g, const dsssp_change* d_changes, int64_t k, void* stream) {
+    if (!g || k < 0 || (k > 0 && !d_changes)) return fail(DSSSP_E_INVAL, "apply_batch: bad arguments");
+    return apply_impl(g, (const int4*)d_changes, nullptr, k, stream);
 }
 
 int dsssp_batch_finish(dsssp_graph* g, dsssp_stats* st) {
@@ -1986,8 +1966,11 @@ int dsssp_apply_batch_host_async(dsssp_graph* g, const dsssp_change* changes, in
     rc = ensure_batch(g, k);
     if (rc) return rc;
     cudaStream_t s = stream ? (cudaStream_t)stream : g->stream;
-    CK(cudaMemcpyAsync(g->d_chg, changes, sizeof(int4) * (size_t)k, cudaMemcpyHostToDevice, s), "batch upload");
-    return dsssp_apply_batch_async(g, (const dsssp_change*)g->d_chg, k, s);
+    // pinned records are read by the first kernel itself; others take a copy
+    const int4* src = (const int4*)pinned_view(const_cast<dsssp_change*>(changes), sizeof(int4) * (size_t)k);
+    if ((uintptr_t)src & 15) src = nullptr;
+    if (!src) CK(cudaMemcpyAsync(g->d_chg, changes, sizeof(int4) * (size_t)k, cudaMemcpyHostToDevice, s), "batch upload");
+    return apply_impl(g, g->d_chg, src, k, s);
 }
 
 int dsssp_apply_batch(dsssp_graph* g, const dsssp_change* changes, int64_t k, void* stream, dsssp_stats* st) {

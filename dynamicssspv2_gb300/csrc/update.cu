@@ -1,7 +1,8 @@
 // update.cu -- the batch-update kernels of the dynamic SSSP engine (sm_103a).
 //
 // One batch (replaces SSSPmainForUndirected.cu:196-281) is four launches on one stream:
-//   k_prepare   validate and count the change records
+//   k_prepare   clear the control block and the deletion set, bring the records from pinned host
+//               memory and validate them
 //   k_delete    the child end of a deleted tree edge is cut off and every adjacency entry
 //               matching a deletion is tombstoned (binary search in the sorted row prefix +
 //               scan of older appended entries); deletions also go into a device hash set
@@ -1461,15 +1462,21 @@ __device__ void flush_stats(Ctl* ctl, const LocalStats& ls) {
     if (threadIdx.x < 8 && s_lstat[threadIdx.x]) atomicAdd(&ctl->stat[idx[threadIdx.x]], s_lstat[threadIdx.x]);
 }
 
-__device__ void block_add(unsigned long long* dst, unsigned long long x) {
-    __shared__ unsigned long long s_sum;
+// Adds a CTA's sums of N counters to stat[idx[0]], stat[idx[1]], ..., one atomic each.
+template <int N>
+__device__ void block_add(Ctl* ctl, const int (&idx)[N], const unsigned long long (&x)[N]) {
+    __shared__ unsigned long long s_sum[N];
+    if (threadIdx.x < N) s_sum[threadIdx.x] = 0;
     __syncthreads();
-    if (threadIdx.x == 0) s_sum = 0;
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+        const unsigned long long t = warp_sum_u64(x[q]);
+        if (lane_id() == 0 && t) atomicAdd(&s_sum[q], t);
+    }
     __syncthreads();
-    x = warp_sum_u64(x);
-    if (lane_id() == 0 && x) atomicAdd(&s_sum, x);
-    __syncthreads();
-    if (threadIdx.x == 0 && s_sum) atomicAdd(dst, s_sum);
+#pragma unroll
+    for (int q = 0; q < N; q++)
+        if (threadIdx.x == q && s_sum[q]) atomicAdd(&ctl->stat[idx[q]], s_sum[q]);
 }
 
 // Per-warp staging of appends to a plain u32 list.  A warp writes its region of shared memory
@@ -1686,24 +1693,33 @@ __device__ __forceinline__ bool list_tail(const UpdParams& p, long long lo, unsi
 
 // ---- kernels -----------------------------------------------------------------------------
 
+// Clears the control block and the batch's deletion set and validates the records, which it brings
+// from pinned host memory if they lie there (a copy and two memset nodes before it cost a batch of 17
+// changes 8 us; for 16 MB the link is the bound either way).  A refusal is told under the batch's epoch (line 0 of the control block), so
+// that no word needs clearing before any of this.
 __global__ void k_prepare(UpdParams p) {
     Ctl* ctl = p.g.ctl;
-    unsigned long long ins = 0, del = 0, ign = 0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.k;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int4 c = p.chg[i];
+    if (blockIdx.x == 0) {  // line 1 on
+        unsigned* w = reinterpret_cast<unsigned*>(&ctl->status);
+        const unsigned words = (unsigned)((sizeof(Ctl) - offsetof(Ctl, status)) / sizeof(unsigned));
+        for (unsigned i = threadIdx.x; i < words; i += blockDim.x) w[i] = 0;
+    }
+    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long nthreads = (long long)gridDim.x * blockDim.x;
+    static_assert(sizeof(DelSlot) == sizeof(uint4), "a deletion-set slot is one store");
+    uint4* const set = reinterpret_cast<uint4*>(p.hset);
+    for (unsigned long long i = (unsigned long long)tid; i <= p.hmask; i += (unsigned long long)nthreads)
+        set[i] = make_uint4(kNone, kNone, kNone, kNone);
+    unsigned refused = 0;
+    for (long long i = tid; i < p.k; i += nthreads) {
+        const int4 c = p.chg_src ? __ldcs(&p.chg_src[i]) : p.chg[i];
+        if (p.chg_src) p.chg[i] = c;
         if (c.w == 1 || c.w == 0) {
-            if (c.x < 0 || c.x >= p.g.n || c.y < 0 || c.y >= p.g.n) set_status(ctl, -3 /* BAD_VERTEX */);
-            else if (c.w == 1 && c.z < 0) set_status(ctl, -10 /* BAD_WEIGHT */);
-            if (c.w == 1) ins++;
-            else del++;
-        } else {
-            ign++;
+            if (c.x < 0 || c.x >= p.g.n || c.y < 0 || c.y >= p.g.n) refused = kRefusedVertex;
+            else if (c.w == 1 && c.z < 0) refused = max(refused, kRefusedWeight);
         }
     }
-    block_add(&ctl->stat[ST_INS], ins);
-    block_add(&ctl->stat[ST_DEL], del);
-    block_add(&ctl->stat[ST_IGN], ign);
+    if (refused) atomicMax(&ctl->refused, ((unsigned long long)p.epoch << 32) | refused);
 }
 
 // Deletions: cut off the child end of a deleted tree edge, tombstone every matching entry,
@@ -1715,7 +1731,12 @@ __global__ void k_prepare(UpdParams p) {
 template <bool kTails>
 __global__ void __launch_bounds__(256, 6) k_delete(UpdParams p) {
     Ctl* ctl = p.g.ctl;
-    if (__ldcg(&ctl->status) != 0) return;  // set by k_prepare: same for every thread
+    const unsigned long long refused = __ldcg(&ctl->refused);  // by k_prepare: same for every thread
+    if (refused >> 32 == p.epoch) {
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            set_status(ctl, (unsigned)refused == kRefusedVertex ? -3 /* BAD_VERTEX */ : -10 /* BAD_WEIGHT */);
+        return;
+    }
     const long long nthreads = (long long)gridDim.x * blockDim.x;
     unsigned long long probed = 0, roots = 0, dead = 0;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
@@ -1776,9 +1797,7 @@ __global__ void __launch_bounds__(256, 6) k_delete(UpdParams p) {
         roots_list.flush(p.g.invq, &ctl->inv_count, (unsigned)p.g.n, 32, ctl);
     }
     roots_list.flush_cta(p.g.invq, &ctl->inv_count, (unsigned)p.g.n, ctl);
-    block_add(&ctl->stat[ST_ROOTS], roots);
-    block_add(&ctl->stat[ST_DEL_PROBED], probed);
-    block_add(&ctl->stat[ST_TOMBS], dead);
+    block_add<3>(ctl, {ST_ROOTS, ST_DEL_PROBED, ST_TOMBS}, {roots, probed, dead});
 }
 
 // Insertions that no deletion of the batch removes go into row slack, both directions.  An end that
@@ -1790,12 +1809,24 @@ __global__ void __launch_bounds__(256, 6) k_delete(UpdParams p) {
 // infinite, so nothing relaxes from them), an end relaxed from a vertex that the walk later
 // cuts off takes that vertex as its parent and is cut off with it, and every other relaxed
 // distance is the length of a live path.
-__global__ void k_append(UpdParams p) {
+// 5 CTAs per SM (48 registers) against 4: 0.146 -> 0.141 ms on RMAT scale 22 with 10^6 changes.
+__global__ void __launch_bounds__(256, 5) k_append(UpdParams p) {
     Ctl* ctl = p.g.ctl;
-    if (__ldcg(&ctl->status) < 0) return;  // same for every thread
     DevGraph& g = p.g;
     const unsigned lane = lane_id();
     const long long nthreads = (long long)gridDim.x * blockDim.x;
+    unsigned long long n_del = 0, n_ign = 0;
+    if (__ldcg(&ctl->status) < 0) {  // refused (same for every thread): only counted
+        unsigned long long n_ins = 0;
+        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.k; i += nthreads) {
+            const int op = p.chg[i].w;
+            n_ins += op == 1 ? 1 : 0;
+            n_del += op == 0 ? 1 : 0;
+            n_ign += op != 0 && op != 1 ? 1 : 0;
+        }
+        block_add<3>(ctl, {ST_INS, ST_DEL, ST_IGN}, {n_ins, n_del, n_ign});
+        return;
+    }
     const unsigned rbase = __ldcg(&ctl->round_base);
     const unsigned tag0 = rbase + 1;
     // near-far: a batch starts with threshold 0, so every seed waits in the far list
@@ -1828,11 +1859,13 @@ __global__ void k_append(UpdParams p) {
                         dead += tombstone_at(p, lo + b + 32 * k + lane, e[k].y, (x.w & kNoPair) == 0);
             }
         }
-        block_add(&ctl->stat[ST_TOMBS], dead);
+        block_add<1>(ctl, {ST_TOMBS}, {dead});
     }
     for (long long base = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; base < p.k; base += nthreads) {
         const long long i = base + lane;
         const int4 c = i < p.k ? p.chg[i] : make_int4(0, 0, 0, -1);
+        n_del += i < p.k && c.w == 0 ? 1 : 0;
+        n_ign += i < p.k && c.w != 0 && c.w != 1 ? 1 : 0;
         // Independent accesses of one record go out together (states, rows and the deletion-set
         // probe; both degree bumps; both seed relaxations; both claims).
         int alive = 0;
@@ -1895,13 +1928,9 @@ __global__ void k_append(UpdParams p) {
     }
     near_list.flush_cta(p.seedq, &ctl->seed_count, seed_cap, ctl);
     far_list.flush_cta(g.far0, &ctl->fc[0], (unsigned)g.n, ctl);
-    block_add(&ctl->stat[ST_SEED_UPD], ls.updates);  // kept apart from k_update's counters
-    block_add(&ctl->stat[ST_SEED_FRONT], ls.frontier);
-    block_add(&ctl->stat[ST_DIST_OVF], ls.dist_ovf);
-    block_add(&ctl->stat[ST_OVF], ovf);
-    block_add(&ctl->stat[ST_LIVE_INS], live_ins);
-    unsigned long long kk = warp_sum_u64(killed);
-    if (lane_id() == 0 && kk) atomicAdd(&ctl->killed, (unsigned)kk);
+    // the seeds' counters are kept apart from k_update's
+    block_add<9>(ctl, {ST_SEED_UPD, ST_SEED_FRONT, ST_DIST_OVF, ST_OVF, ST_LIVE_INS, ST_KILLED, ST_INS, ST_DEL, ST_IGN},
+                 {ls.updates, ls.frontier, ls.dist_ovf, ovf, live_ins, killed, live_ins + killed, n_del, n_ign});
 }
 
 // grid-wide; true when the kernel may go on

@@ -88,10 +88,9 @@ typedef struct {
                              the last batch or tree computation needed more than auto_rounds
                              rounds, plain rounds otherwise.  Costs 12 bytes per vertex, allocated when
                              first used. */
-    int32_t launch_graph; /* 1 = a batch's launch sequence (control-block reset, deletion-set
-                             reset, the four kernels, the status read) is replayed from an
-                             instantiated CUDA graph whose node parameters are updated per
-                             batch; 0 = plain stream launches.  Falls back to plain launches
+    int32_t launch_graph; /* 1 = a batch's launch sequence (the four kernels, the status read) is
+                             replayed from an instantiated CUDA graph whose node parameters are
+                             updated per batch; 0 = plain stream launches.  Falls back to plain launches
                              if the graph cannot be built. */
     int32_t recover;      /* 1 (the default) = a batch whose update kernel fails after its edits
                              reached the adjacency recomputes the trees from the roots and returns
