@@ -34,6 +34,7 @@ constexpr unsigned kTagOk = 0xFFFFFFFFu;   // pointer jumping: reaches the root 
 constexpr unsigned kTagInv = 0xFFFFFFFEu;  // pointer jumping: below a cut-off vertex
 constexpr int kStatusOverflowPending = 1;  // internal: the spare region cannot take the growing rows
 constexpr unsigned kRefusedWeight = 1, kRefusedVertex = 2;  // why k_prepare refused a batch
+constexpr int kLocalDeg = 32;  // rows above this leave a local stretch through the lists
 constexpr int kGrowChunk = 256;            // slots of a growing row that one warp handles
 constexpr unsigned kNoTwin = 0xFFFFFFFFu;   // twin not known yet (the other end overflowed)
 constexpr unsigned long long kHashEmpty = 0xFFFFFFFFFFFFFFFFull;
@@ -88,7 +89,7 @@ struct __align__(128) Ctl {
     unsigned spin_limit;  // grid-barrier poll limit (0 = default); persistent, set by the host
     unsigned stall_us;    // test hook: the last CTA of k_update waits this long before its first barrier
     unsigned grp_gen;     // generation of the group barrier (the first group_ctas CTAs)
-    unsigned pad0a;
+    unsigned long_rows;   // rows above kLocalDeg entries as of the last layout
     unsigned long long refused;  // (epoch << 32) | why, of the last batch that k_prepare refused
     unsigned pad0[24];
     // line 1

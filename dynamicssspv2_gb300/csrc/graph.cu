@@ -122,8 +122,10 @@ __global__ void k_row_ids(const long long* poff, int n, unsigned* ids) {
 }
 
 __global__ void k_rows_init(const long long* start, const long long* deg, const long long* cap, int n,
-                            RowDesc* rows, int* sorted_len) {
+                            RowDesc* rows, int* sorted_len, unsigned* long_rows) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned lng = __ballot_sync(0xFFFFFFFFu, v < n && deg[v] > kLocalDeg);
+    if ((threadIdx.x & 31) == 0 && lng) atomicAdd(long_rows, (unsigned)__popc(lng));
     if (v >= n) return;
     RowDesc r;
     r.start = start[v];
@@ -815,7 +817,9 @@ int layout_rows(dsssp_graph* g, unsigned long long* keys_in, long long total, co
             count_launch(1);
         }
         if (n > 0) {
-            k_rows_init<<<blocks_for(n), kThreads, 0, s>>>(start, deg64, cap, n, g->dg.rows, g->dg.sorted_len);
+            cudaMemsetAsync(&g->dg.ctl->long_rows, 0, sizeof(unsigned), s);
+            k_rows_init<<<blocks_for(n), kThreads, 0, s>>>(start, deg64, cap, n, g->dg.rows, g->dg.sorted_len,
+                                                           &g->dg.ctl->long_rows);
             count_launch(1);
         }
         cudaError_t e = cudaGetLastError();

@@ -56,7 +56,6 @@ constexpr int kAddsPerCheck = 32;          // entries a warp may add between two
 static_assert(kBuf > kAddsPerCheck, "a push buffer must take one visit's adds after a check");
 constexpr int kSoloSteps = 256;            // consecutive solo steps before the grid re-syncs
 constexpr unsigned kQueue = 256;           // items of a CTA's queue in a local stretch (two queues)
-constexpr unsigned kLocalDeg = 32;         // rows above this leave a local stretch through the lists
 constexpr int kLocalTe = 16;               // thread items of more edges than this keep to the rounds
 constexpr unsigned kFarBuf = 64;           // per-warp staging of far-list pushes
 constexpr int kSpill = 64;                 // per-warp staging of vertices that leave a stretch
@@ -853,13 +852,20 @@ __device__ __forceinline__ bool local_step(const UpdParams& p, unsigned nt, unsi
 
 __device__ __forceinline__ void keep_stats(const LocalStats& ls);
 
+// A graph of whose rows nearly all fit a stretch's queue.  On others (RMAT: one row in ten above
+// kLocalDeg) a stretch soon leaves through the lists, and the phases before it are better kept
+// apart: seeds, pulls and the first rounds of an RMAT-20 insertion batch 0.071 ms apart, 0.083 in one.
+__device__ __forceinline__ bool short_rows(const UpdParams& p) {
+    return 64ull * __ldcg(&p.g.ctl->long_rows) <= (unsigned long long)p.g.n;
+}
+
 // Pushes c (want), whose row rd has entries, into a CTA's queue: ceil(deg / 4) items, ranked in the
 // warp by the bits of (items - 1).  False for rows above kLocalDeg and where the queue is full (its
 // last places stay empty).  Warp-collective.
 __device__ __forceinline__ bool queue_push(bool want, unsigned c, unsigned nd, const RowDesc& rd, uint4* queue,
                                            unsigned* count) {
     const unsigned lane = lane_id(), lt = (1u << lane) - 1u;
-    const bool shrt = want && rd.deg <= (int)kLocalDeg;
+    const bool shrt = want && rd.deg <= kLocalDeg;
     const unsigned extra = shrt ? ((unsigned)rd.deg - 1u) >> 2 : 0u;
     const unsigned m = __ballot_sync(kFull, shrt), mx = __ballot_sync(kFull, extra != 0);
     if (m == 0) return false;
@@ -938,6 +944,57 @@ struct Stretch {
         __syncwarp();
     }
 
+    // v (pred) into the queue, or to the lists
+    __device__ __forceinline__ void begin(bool pred, unsigned v, unsigned d, uint4* queue, unsigned* count) {
+        const RowDesc rd = row_if(*p, pred, v);
+        pred = pred && rd.deg > 0;
+        const bool in = queue_push(pred, v, d, rd, queue, count);
+        ls.frontier += in ? 1 : 0;
+        if (__any_sync(kFull, pred && !in)) {
+            const bool won = pred && !in && atomicExch(&p->g.push_tag[v], tag()) != tag();
+            spill(won, v, rd);
+        }
+    }
+
+    __device__ __forceinline__ void begin_seed(unsigned i, unsigned ns, uint4* queue, unsigned* count) {
+        const unsigned v = i < ns ? __ldcg(&p->seedq[i]) : 0u;
+        begin(i < ns, v, 0u, queue, count);  // distance 0: whatever the state says
+    }
+
+    // item i of a cut-off vertex: its best live neighbour, as PullOp
+    __device__ __forceinline__ void begin_pull(unsigned i, unsigned nt, unsigned nd, uint4* queue, unsigned* count) {
+        const bool has = i < nt + nd;
+        const Item it = has ? __ldcg(i < nt ? &p->g.it[i] : &p->g.rt1[i - nt]) : make_uint4(0u, 0u, 0u, 0u);
+        const int2* a = adj + item_lo(it);
+        int2 e[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) e[q] = q < (int)it.w ? ld_stream(a + q) : make_int2(0, -1);
+        unsigned long long s[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) s[q] = e[q].y >= 0 ? __ldcg(&state[e[q].x]) : kInfState;
+        ls.edges_pull += min(4u, it.w);
+        unsigned long long best = kInfState;
+        bool push = false;
+        unsigned d = 0;  // of a push through a zero weight: whatever the state says
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (e[q].y < 0 || s[q] == kInfState) continue;
+            const unsigned long long nd = (s[q] >> 32) + (unsigned)e[q].y;
+            if (nd >= kDistInf) ls.dist_ovf++;
+            else if (e[q].y > 0) best = min(best, (nd << 32) | (unsigned)e[q].x);
+            else if (relax_to(p->g, epoch, it.z, nd, (unsigned)e[q].x, 0, __ldcg(&state[it.z]), ls)) push = true;
+        }
+        if (best != kInfState) {
+            const unsigned long long old = atomicMin(&state[it.z], best);
+            if ((old >> 32) > (best >> 32)) {
+                if (!push) d = (unsigned)(best >> 32);
+                push = true;
+                ls.updates++;
+            }
+        }
+        if (__any_sync(kFull, push)) begin(push, it.z, d, queue, count);
+    }
+
     // One item's entry per lane (warp-collective): x = the item, (vertex, distance, slots, count)
     // of at most 4 entries (count 0: none), next = the next step's queue with its counter.
     __device__ __forceinline__ void visit(const uint4& x, uint4* next, unsigned* next_cnt) {
@@ -989,21 +1046,29 @@ struct Stretch {
     }
 };
 
-// CTA-collective; reads list r (nt thread items) and appends to list r + 1.  A function of its
-// own, with its own counters, so that the rounds keep their registers.
+// CTA-collective; reads list r (nt thread items) and appends to list r + 1.  With `pull` the
+// stretch begins at the seeds of k_append (ns of them) and the cut-off vertices' items (nt in `it`,
+// nd in rt1) instead: each of these pulls the vertex's best live neighbour, and what improves is
+// relaxed on at once, while other CTAs still pull.  That is exact: a neighbour that a pull reads too
+// early is pushed by whoever lowers it.  A function of its own, with its own counters, so that
+// the rounds keep their registers.
 __device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigned nt, unsigned steps_max,
-                                         unsigned rbase, unsigned adv, unsigned long long T) {
+                                         unsigned rbase, unsigned adv, unsigned long long T, bool pull, unsigned nd,
+                                         unsigned ns) {
     Ctl* const ctl = p.g.ctl;
     const bool odd = (r & 1) != 0;
     const unsigned slot = (r + 1) % 3;
     const Item* const tl = odd ? p.g.rt1 : p.g.rt0;
     const unsigned lane = lane_id();
-    const unsigned per = blockDim.x >> 2, parts = (unsigned)p.te >> 2, limit = per + per / 2;
+    const unsigned per = blockDim.x >> 2, parts = (unsigned)p.te >> 2;
+    // near-far frontiers are steady, and a CTA that falls behind holds up the others; a plain one grows
+    // and shrinks again (3 passes against 1.5: 300,000 vertices 0.049 -> 0.043 ms, the grid 27 -> 32 ms)
+    const unsigned limit = T == ~0ull ? 3 * per : per + per / 2;
     uint4 *now = &s_pbuf[0][0] + kQueueAt, *next = now + kQueue;
     Stretch st{&p, p.g.state, p.g.adj, p.g.rows, p.g.chg_tag, p.epoch, r, rbase, adv, T, 0, 0, LocalStats{}};
     unsigned* const stopped = &ctl->rstop[slot];
     // items blockIdx, blockIdx + gridDim, ... of the list, at most `per` of them
-    const unsigned mine = nt > blockIdx.x ? (nt - blockIdx.x - 1) / gridDim.x + 1 : 0u;
+    const unsigned mine = !pull && nt > blockIdx.x ? (nt - blockIdx.x - 1) / gridDim.x + 1 : 0u;
     for (unsigned i = threadIdx.x; i < mine; i += blockDim.x) {
         const Item it = __ldcg(&tl[blockIdx.x + (unsigned long long)i * gridDim.x]);
         for (unsigned k = 0; k < parts; k++) {
@@ -1019,6 +1084,13 @@ __device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigne
         s_stop[0] = s_stop[1] = 0;
     }
     __syncthreads();
+    if (pull) {
+        for (unsigned i0 = (threadIdx.x & ~31u); blockIdx.x + i0 * gridDim.x < ns; i0 += blockDim.x)
+            st.begin_seed(blockIdx.x + (i0 + lane) * gridDim.x, ns, now, &s_qcnt[0]);
+        for (unsigned i0 = (threadIdx.x & ~31u); blockIdx.x + i0 * gridDim.x < nt + nd; i0 += blockDim.x)
+            st.begin_pull(blockIdx.x + (i0 + lane) * gridDim.x, nt, nd, now, &s_qcnt[0]);
+        __syncthreads();
+    }
     unsigned k = 0, n, cur = 0, nxt = 1, old = 2;  // the steps' counters rotate
     for (;; k++) {
         n = min(s_qcnt[cur], kQueue);
@@ -1059,13 +1131,14 @@ __device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigne
 // The same for levels of the subtree walk: list entries [lo, lo + nt) of `it` are this stretch's first
 // items, hiT and hiC where the grid's lists end.  The items of the vertices that the stretch cuts
 // off and walks on from go to `done` (rt1, free during the walk), for their pull; those it does
-// not reach go behind hiT, as the next level's.  Three accesses a step: the entry, the neighbour's
+// not reach go behind hiT, as the next level's.  With `roots` > 0 the stretch begins at the roots
+// instead (at most half a pass of every CTA), without a list of them.  Three accesses a step: the entry, the neighbour's
 // parent word, and for a child its tag beside its row descriptor.  A step is a level.
 // Against levels on the grid and on CTA 0, the walk of ER graphs of 10k, 300k vertices and of 64
 // pooled ones: 0.088 -> 0.073, 0.140 -> 0.106 and 0.166 -> 0.145 ms; a 1021 x 1543 grid's 48 levels and
 // pointer jumping 0.52 -> 0.31 ms; RMAT, whose levels hold hub rows, unchanged.
 __device__ __noinline__ void walk_local(const UpdParams& p, unsigned li, unsigned lo, unsigned nt, unsigned hiT,
-                                        unsigned hiC, unsigned steps_max) {
+                                        unsigned hiC, unsigned steps_max, unsigned roots) {
     Ctl* const ctl = p.g.ctl;
     const DevGraph& g = p.g;
     unsigned long long* const state = g.state;
@@ -1087,6 +1160,18 @@ __device__ __noinline__ void walk_local(const UpdParams& p, unsigned li, unsigne
         s_stop[0] = s_stop[1] = 0;
     }
     __syncthreads();
+    if (roots) {
+        const unsigned share = roots > blockIdx.x ? (roots - blockIdx.x - 1) / gridDim.x + 1 : 0u;
+        for (unsigned b = threadIdx.x & ~31u; b < share; b += blockDim.x) {
+            const bool has = b + lane < share;
+            const unsigned v = has ? __ldcg(&g.invq[blockIdx.x + (b + lane) * gridDim.x]) : 0u;
+            const RowDesc rd = row_if(p, has, v);
+            const bool in = queue_push(has && rd.deg > 0, v, 0u, rd, now, &s_qcnt[0]);
+            if (pb.count + 32 > kSpill) pb.expand_all(p, out, ls);
+            pb.add(has && !in, v, rd);
+        }
+        __syncthreads();
+    }
     // writes n items of a queue to a list from place `at` on (thread items of at most 4 entries)
     auto keep = [&](const uint4* q, unsigned n, Item* list, long long at, long long cap) {
         if (at + n > cap) {
@@ -1111,7 +1196,7 @@ __device__ __noinline__ void walk_local(const UpdParams& p, unsigned li, unsigne
         unsigned at = 0;
         if (threadIdx.x == 0) {
             s_qcnt[old] = 0;
-            if (k > 0) at = atomicAdd(&ctl->walk_done, n);  // the first step's items are in `it` already
+            if (k > 0 || roots) at = atomicAdd(&ctl->walk_done, n);  // a list's items are in `it` already
         }
         const unsigned stop = threadIdx.x == blockDim.x - 1 ? __ldcg(stopped) : 0u;
         for (unsigned b = warp0; b < n; b += per) {  // warp-uniform
@@ -1141,7 +1226,7 @@ __device__ __noinline__ void walk_local(const UpdParams& p, unsigned li, unsigne
         }
         if (stop) s_stop[(k + 1) & 1] = 1;  // a slow warp may still read this step's word
         if (threadIdx.x == 0) s_done[k & 1] = at;
-        if (k > 0) nprev = n;
+        if (k > 0 || roots) nprev = n;
         unsigned t = old;
         old = cur;
         cur = nxt;
@@ -1258,7 +1343,18 @@ __device__ __forceinline__ unsigned long long walk(const UpdParams& p) {
     // so far, so every CTA derives the same bounds while faster CTAs already append.  Small
     // levels are walked in CTA queues, several to a list.
     const unsigned nroots = __ldcg(&ctl->inv_count);  // written by k_delete
-    {
+    unsigned loT = 0, loC = 0, hiT = 0, hiC = 0;
+    int level = 0;
+    unsigned li = 0;
+    if (nroots == 0) return 0;
+    if (leader) ls.marked += nroots;
+    if (p.te == 4 && p.group_ctas == 0 && nroots <= gridDim.x * min(4u, blockDim.x >> 3) && short_rows(p)) {
+        unsigned used;
+        walk_local(p, li, 0, 0, 0, 0, (unsigned)p.bfs_levels, nroots);
+        if (!grid_sync(ctl, &ctl->ltT[1], &ctl->ltC[1], hiT, hiC, &ctl->lsteps[1], used)) return ~0ull;
+        level = (int)used;
+        li = 1;
+    } else {
         const Out lvl0{g.it, &ctl->ltT[0], g.tcap, g.ic, &ctl->ltC[0], g.ccap};
         PushBuf pb{pbuf, 0};
         for (unsigned base = gtid - lane; base < nroots; base += nthreads) {
@@ -1268,12 +1364,8 @@ __device__ __forceinline__ unsigned long long walk(const UpdParams& p) {
             pb.flush(p, lvl0, ls);
         }
         pb.flush_cta(p, lvl0, ls);
+        if (!grid_sync(ctl, &ctl->ltT[0], &ctl->ltC[0], hiT, hiC)) return ~0ull;
     }
-    if (leader) ls.marked += nroots;
-    unsigned loT = 0, loC = 0, hiT, hiC;
-    if (!grid_sync(ctl, &ctl->ltT[0], &ctl->ltC[0], hiT, hiC)) return ~0ull;
-    int level = 0;
-    unsigned li = 0;
     bool need_pj = false;
     for (;;) {
         if (loT >= hiT && loC >= hiC) break;
@@ -1288,7 +1380,7 @@ __device__ __forceinline__ unsigned long long walk(const UpdParams& p) {
                 ctl->lsteps[(li + 2) % 3] = 0;
                 ctl->lstop[(li + 2) % 3] = 0;
             }
-            walk_local(p, li, loT, hiT - loT, hiT, hiC, (unsigned)(p.bfs_levels - level));
+            walk_local(p, li, loT, hiT - loT, hiT, hiC, (unsigned)(p.bfs_levels - level), 0);
             unsigned addT, addC, used;
             if (!grid_sync(ctl, &ctl->ltT[(li + 1) % 3], &ctl->ltC[(li + 1) % 3], addT, addC, &ctl->lsteps[(li + 1) % 3], used))
                 return ~0ull;
@@ -1597,7 +1689,7 @@ __device__ __forceinline__ unsigned tombstone_at(const UpdParams& p, long long j
 // out, which the caller scans.  With the twin index the reverse entries are tombstoned too.
 // Returns the number of entries examined; `dead` counts the entries tombstoned.
 __device__ unsigned long long tombstone_prefix(const UpdParams& p, const RowDesc& rd, int sorted_len, int col, int w,
-                                               bool with_twin, unsigned long long& dead, long long& tlo,
+                                               bool with_twin, unsigned& dead, long long& tlo,
                                                long long& thi) {
     const int2* adj = p.g.adj;
     const long long sl = rd.start + sorted_len;
@@ -1612,7 +1704,7 @@ __device__ unsigned long long tombstone_prefix(const UpdParams& p, const RowDesc
 
 // The whole row: the sorted prefix by binary search, the tail by this thread.
 __device__ unsigned long long tombstone_row(const UpdParams& p, const RowDesc& rd, int sorted_len, int col, int w,
-                                            bool with_twin, unsigned long long& dead) {
+                                            bool with_twin, unsigned& dead) {
     const int2* adj = p.g.adj;
     const long long sl = rd.start + sorted_len, end = rd.start + rd.deg;
     long long j = lower_col(adj, rd.start, sl, col);
@@ -1738,7 +1830,8 @@ __global__ void __launch_bounds__(256, 6) k_delete(UpdParams p) {
         return;
     }
     const long long nthreads = (long long)gridDim.x * blockDim.x;
-    unsigned long long probed = 0, roots = 0, dead = 0;
+    unsigned long long probed = 0;
+    unsigned roots = 0, dead = 0;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     WarpList roots_list{s_wlist[warp], kListRegion, 0};
     for (long long base = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; base < p.k; base += nthreads) {
@@ -2023,6 +2116,9 @@ __device__ void update_body(const UpdParams& p) {
     };
 
     unsigned nT = 0, nC = 0;  // the sizes of the next relaxation round's lists
+    // r counts the lists (a round or a local stretch each), hops the rounds and the steps of
+    // the stretches: the depth of the dependent relaxations
+    unsigned r = 0, hops = 0;
     if (p.mode == 1) {
         PushBuf pb{pbuf, 0};
         for (unsigned base = gtid - lane; base < (unsigned)p.nsrc; base += nthreads) {
@@ -2043,15 +2139,23 @@ __device__ void update_body(const UpdParams& p) {
         hiC = (unsigned)(ends >> 32);
         if (leader) ctl->ts[1] = globaltimer();
 
-        seed_and_pull(p, hiT, hiC, rbase, T);
-        if (!grid_sync(ctl, &ctl->rcT[0], &ctl->rcC[0], nT, nC)) return;
+        const unsigned ns = __ldcg(&ctl->seed_count), nd = __ldcg(&ctl->walk_done);
+        if (!kAgg && !nf && p.te == 4 && p.max_rounds > 0 && local_step(p, ns + hiT + nd, hiC) && short_rows(p)) {
+            // few enough for one stretch: its list is number 2 (rt0; rt1 holds items of the walk)
+            if (leader) ctl->ts[2] = ctl->ts[1];
+            relax_local(p, 1, hiT, p.max_rounds < (long long)kStretch ? (unsigned)p.max_rounds : kStretch, rbase, 0, T,
+                        true, nd, ns);
+            if (!grid_sync(ctl, &ctl->rcT[2], &ctl->rcC[2], nT, nC, &ctl->rsteps[2], hops)) return;
+            r = 2;
+        } else {
+            seed_and_pull(p, hiT, hiC, rbase, T);
+            if (!grid_sync(ctl, &ctl->rcT[0], &ctl->rcC[0], nT, nC)) return;
+            if (leader) ctl->ts[2] = globaltimer();
+        }
     }
-    if (leader) ctl->ts[2] = globaltimer();
+    if (leader && p.mode == 1) ctl->ts[2] = globaltimer();
 
     // ---- C. relaxation rounds ---------------------------------------------------------------
-    // r counts the lists (a round or a local stretch each), hops the rounds and the steps of
-    // the stretches: the depth of the dependent relaxations
-    unsigned r = 0, hops = 0;
     for (;; r++) {
         // nT, nC: the sizes of round r's lists (read at the barrier before)
         if (nT == 0 && nC == 0) {
@@ -2084,7 +2188,7 @@ __device__ void update_body(const UpdParams& p) {
                 ctl->rstop[(r + 2) % 3] = 0;
             }
             const long long left = p.max_rounds - hops;
-            relax_local(p, r, nT, left < (long long)kStretch ? (unsigned)left : kStretch, rbase, adv, T);
+            relax_local(p, r, nT, left < (long long)kStretch ? (unsigned)left : kStretch, rbase, adv, T, false, 0, 0);
             unsigned t2, used;
             if (!grid_sync(ctl, &ctl->rcT[(r + 1) % 3], &ctl->rcC[(r + 1) % 3], t2, nC, &ctl->rsteps[(r + 1) % 3], used))
                 break;
