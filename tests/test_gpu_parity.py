@@ -796,6 +796,32 @@ def test_local_stretches_around_their_widest_round(leaves):
     check_against_oracle(n, u, v, w, None, 0, p, d, f"{leaves} leaves")
 
 
+@pytest.mark.parametrize("first", [1, 2, 3, 4])
+def test_local_stretch_pushes_more_than_its_queue_holds(first):
+    """Trees of rows with four entries: a step's pushes end below, at and beyond the places that are
+    left in the CTA's queue (162 items push 486 vertices, 108 push 324, 81 push 243)."""
+    level, u, v, n = np.arange(1, 1 + first), [np.zeros(first, np.int64)], [np.arange(1, 1 + first)], 1 + first
+    for _ in range(8):
+        kids = n + np.arange(3 * len(level))
+        u.append(np.repeat(level, 3))
+        v.append(kids)
+        n += len(kids)
+        level = kids
+    u, v = np.concatenate(u), np.concatenate(v)
+    w = 1 + (np.arange(len(u)) * 2654435761 % 53)
+    u, v, w = (np.ascontiguousarray(x, np.int32) for x in (u, v, w))
+    ch = np.concatenate([D.make_changes(u[:first], v[:first], w[:first], np.zeros(first)),
+                         D.make_changes(u[:first], v[:first], w[:first] + 7, np.ones(first))])
+    for opts in ({}, {"delta": 60}):
+        with D.Graph(n, u, v, w, **opts) as g:
+            g.tree_compute(0)
+            p, d = g.tree_read()
+            check_against_oracle(n, u, v, w, None, 0, p, d, f"tree, {first} children, {opts}")
+            g.apply_batch(ch)
+            p, d = g.tree_read()
+            check_against_oracle(n, u, v, w, ch, 0, p, d, f"batch, {first} children, {opts}")
+
+
 def test_a_self_loop_deleted_by_many_records_is_counted_once():
     """Self-loops among which many are one line repeated, each deleted by many records of one
     batch: the live count afterwards is exact (every entry is tombstoned and counted once)."""
