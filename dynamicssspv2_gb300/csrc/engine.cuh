@@ -106,7 +106,7 @@ struct __align__(128) Ctl {
     unsigned grow_done;   // CTAs past the growth's last phase but one (all: that phase has run or may)
     unsigned pad1[16];
     // line 2
-    unsigned bar_count;
+    unsigned bar_count;  // arrivals at the grid barrier since the launch of k_update, which finds 0 here
     unsigned pad2[31];
     // line 2b: arrivals at the group barrier (its own line: the grid's CTAs poll bar_gen meanwhile)
     unsigned grp_count;
@@ -246,8 +246,18 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
     return v;
 }
 
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ void st_relaxed(unsigned* p, unsigned v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 __device__ __forceinline__ unsigned long long globaltimer() {

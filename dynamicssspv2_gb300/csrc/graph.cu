@@ -1244,6 +1244,7 @@ int finish_batch(dsssp_graph* g, dsssp_stats* st) {
         if (rc) return rc;
         repacks = 1;
         CK(cudaMemsetAsync(&g->dg.ctl->status, 0, offsetof(Ctl, inv_count) - offsetof(Ctl, status), s), "status reset");
+        CK(cudaMemsetAsync(&g->dg.ctl->bar_count, 0, sizeof(g->dg.ctl->bar_count), s), "status reset");
         UpdParams p = make_params(g, g->pend_chg, g->pend_k, 0);
         // the front interval now spans the repack; the update interval is the resumed launch
         if (g->pend_events) CK(cudaEventRecord(g->ev[1], s), "event");
