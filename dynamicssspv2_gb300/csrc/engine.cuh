@@ -123,17 +123,17 @@ struct __align__(128) Ctl {
     unsigned pjT;
     unsigned pjC;
     unsigned pjf[3];
-    unsigned fc[2];  // near-far: far-list counts (double buffer)
+    unsigned fc[3];  // near-far: far-list counts, of advance adv's list in slot adv % 3
     unsigned lsteps[3];  // local stretches of the walk, as rsteps and rstop
     unsigned lstop[3];
     unsigned walk_done;  // their items, listed in rt1 for the pull
-    unsigned pad4[12];
+    unsigned pad4[11];
     // line 4b: near-far threshold reduction
-    unsigned long long fmin;
+    unsigned long long fmin[2];  // by the parity of the advances
     // small steps run by CTA 0 alone hand their end state to the grid here
     unsigned long long solo[4];
     unsigned solo_n[2];  // list sizes of the first round after solo relaxation rounds
-    unsigned pad4b[20];
+    unsigned pad4b[18];
     // line 5: barrier diagnostics (first timed-out barrier, arrivals then, CTAs that timed
     // out, max barrier count at exit, 0xFFFFFFFF - min barrier count at exit)
     unsigned diag[8];

@@ -822,6 +822,29 @@ def test_local_stretch_pushes_more_than_its_queue_holds(first):
             check_against_oracle(n, u, v, w, ch, 0, p, d, f"batch, {first} children, {opts}")
 
 
+@pytest.mark.parametrize("leaves", [300, 116735, 116736, 116737])
+@pytest.mark.parametrize("opts", [{}, {"warp_agg": 1}, {"small_deg": 16}], ids=str)
+def test_far_lists_around_one_pass_of_the_grid(leaves, opts):
+    """A star whose leaves all wait in the far list, on in chains of three: the list is one vertex
+    below, at and above what a local stretch takes whole (above, and with aggregated offers, it
+    is split by the grid).  No leaf lies within one width of the first threshold."""
+    hub = np.zeros(leaves, np.int64)
+    a = 1 + np.arange(leaves)
+    u = np.concatenate([hub, a, a + leaves])
+    v = np.concatenate([a, a + leaves, a + 2 * leaves])
+    n = 1 + 3 * leaves
+    w = 25 + (np.arange(len(u)) * 2654435761 % 73)
+    u, v, w = (np.ascontiguousarray(x, np.int32) for x in (u, v, w))
+    ch = D.gen_changes(n, u, v, w, 60, 60, seed=leaves)
+    with D.Graph(n, u, v, w, delta=10, **opts) as g:
+        assert g.tree_compute(0).advances > 0
+        p, d = g.tree_read()
+        check_against_oracle(n, u, v, w, None, 0, p, d, f"{leaves} leaves")
+        g.apply_batch(ch)
+        p, d = g.tree_read()
+        check_against_oracle(n, u, v, w, ch, 0, p, d, f"{leaves} leaves, batch")
+
+
 def test_a_self_loop_deleted_by_many_records_is_counted_once():
     """Self-loops among which many are one line repeated, each deleted by many records of one
     batch: the live count afterwards is exact (every entry is tombstoned and counted once)."""
