@@ -227,6 +227,8 @@ struct UpdParams {
     int bfs_levels;
     int mode;         // 0 = batch update, 1 = from scratch (state already reset)
     unsigned long long delta;  // near-far bucket width; 0 = plain frontier relaxation
+    unsigned long long late_delta;  // ... of a plain computation's rounds past late_after; 0 = all are plain
+    unsigned late_after;
     unsigned* seedq;  // vertices seeded by k_append (claimed, expanded by k_update)
     const int* srcs;  // mode 1: the sources (every root is its own parent)
     int nsrc;

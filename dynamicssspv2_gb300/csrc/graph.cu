@@ -607,20 +607,30 @@ int ensure_far(dsssp_graph* g) {
     return DSSSP_OK;
 }
 
+// The automatic bucket width.  Wide buckets: a round costs a dependent chain and a grid barrier
+// whatever its size, so fewer rounds beat fewer relaxations (the 4096^2 grid: 103 ms at 8x, 87 ms
+// at 32x, 83 ms at 64-96x with 4-6x the relaxations).
+unsigned long long auto_delta(const dsssp_graph* g) {
+    const double d = 32.0 * g->mean_w;
+    return d < 1.0 ? 1ull : (unsigned long long)(d + 0.5);
+}
+
 // Near-far bucket width of the next batch or tree computation.  delta > 0 is used as given;
 // delta < 0 (automatic) turns near-far rounds on with 32 times the mean edge weight once the
 // last batch or tree computation needed more than opts.auto_rounds rounds (a high-diameter graph);
 // 0 keeps plain rounds.
 unsigned long long effective_delta(const dsssp_graph* g) {
     if (g->o.delta > 0) return (unsigned long long)g->o.delta;
-    if (g->o.delta < 0 && g->last_rounds > (long long)g->o.auto_rounds) {
-        // wide buckets: a round costs a dependent chain and a grid barrier whatever its size,
-        // so fewer rounds beat fewer relaxations (the 4096^2 grid: 103 ms at 8x, 87 ms at 32x,
-        // 83 ms at 64-96x with 4-6x the relaxations)
-        const double d = 32.0 * g->mean_w;
-        return d < 1.0 ? 1ull : (unsigned long long)(d + 0.5);
-    }
+    if (g->o.delta < 0 && g->last_rounds > (long long)g->o.auto_rounds) return auto_delta(g);
     return 0;
+}
+
+// Whether a plain computation may go on near-far past opts.auto_rounds rounds (late_delta): on graphs
+// large and sparse enough to be deep, whose lists are allocated with the graph.  The first tree of
+// grids of 1024^2, 2048^2, 4096^2 vertices 13.4 -> 4.3, 61 -> 9.2 and 469 -> 20.2 ms, of 724^2 7.2 -> 3.0
+// ms; of 512^2 2.4 -> 2.1 ms, against 0.1 ms for the lists, and the same below.
+bool may_run_deep(const dsssp_graph* g) {
+    return g->o.delta < 0 && g->n >= (1 << 19) && g->entries <= 8 * (long long)g->n;
 }
 
 int ensure_work(dsssp_graph* g) {
@@ -922,6 +932,8 @@ UpdParams make_params(const dsssp_graph* g, const int4* chg, long long k, int mo
     p.bfs_levels = g->o.bfs_levels;
     p.mode = mode;
     p.delta = g->dg.far_tag ? effective_delta(g) : 0ull;  // the caller ensured the lists
+    p.late_delta = !p.delta && g->dg.far_tag && g->o.delta < 0 ? auto_delta(g) : 0ull;
+    p.late_after = (unsigned)g->o.auto_rounds;
     p.seedq = g->d_seedq;
     p.srcs = g->d_srcs;
     p.nsrc = 0;
@@ -1600,6 +1612,9 @@ int dsssp_graph_create(int32_t n, int64_t m, const int32_t* u, const int32_t* v,
     if (!rc) rc = layout_rows(g, keys, 2 * m, deg64, poff, s);
     dfree(deg); dfree(cursor); dfree(deg64); dfree(poff); dfree(keys);
     if (rc) { dsssp_graph_destroy(g); return rc; }
+    size_t room = 0, total = 0;
+    if (may_run_deep(g) && cudaMemGetInfo(&room, &total) == cudaSuccess && room > total / 4)
+        (void)ensure_far(g);  // without them all rounds of the first computation are plain
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { dsssp_graph_destroy(g); return cuda_fail(e, "graph build"); }
     *out = g;

@@ -1320,7 +1320,8 @@ __device__ __forceinline__ void keep_stats(const LocalStats& ls) {
 // and a barrier.  0 when nothing waits or the kernel must stop.
 __device__ __forceinline__ unsigned long long next_threshold(const UpdParams& p, unsigned nfar, unsigned adv,
                                                           unsigned long long T, bool least) {
-    if (!least) return T + p.delta;
+    const unsigned long long width = p.delta ? p.delta : p.late_delta;
+    if (!least) return T + width;
     Ctl* const ctl = p.g.ctl;
     const DevGraph& g = p.g;
     const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
@@ -1333,7 +1334,7 @@ __device__ __forceinline__ unsigned long long next_threshold(const UpdParams& p,
     block_max(&ctl->fmin[adv & 1], ~mn);  // max of ~d = min of d; 0 = nothing waits
     if (!grid_sync(ctl)) return 0;
     const unsigned long long fm = __ldcg(&ctl->fmin[adv & 1]);
-    return fm ? ~fm + p.delta : 0;
+    return fm ? ~fm + width : 0;
 }
 
 // A far list of at most one pass of the grid goes straight into a local stretch: every CTA takes its
@@ -2191,7 +2192,7 @@ __device__ void update_body(const UpdParams& p) {
     // from scratch starts with the sources (distance 0) near and T = delta.  Far generations
     // of this call are rbase, rbase + 1, ... (at most one per round, so below the next
     // call's round base).
-    const bool nf = p.delta != 0 && g.far0 != nullptr && g.far1 != nullptr && g.far_tag != nullptr;
+    bool nf = p.delta != 0 && g.far0 != nullptr && g.far1 != nullptr && g.far_tag != nullptr;
     unsigned long long T = nf ? (p.mode == 1 ? p.delta : 0ull) : ~0ull;
     unsigned adv = 0;     // advances: far list adv & 1 takes this near phase's far pushes, generation rbase + adv
     bool sparse = false;  // an advance by one width has found nothing
@@ -2242,6 +2243,13 @@ __device__ void update_body(const UpdParams& p) {
     // ---- C. relaxation rounds ---------------------------------------------------------------
     for (;; r++) {
         // nT, nC: the sizes of round r's lists (read at the barrier before)
+        if (!nf && p.late_delta != 0 && hops >= p.late_after) {
+            // A plain computation has turned out deep: what it pushes from here on waits, and the
+            // first advance picks a threshold.  (Switching after 256, 512, 1024, 2048 rounds, the first
+            // tree of a 2048^2 grid: 9.2, 9.2, 11.7, 27.6 ms; never: 61 ms.)
+            nf = true;
+            T = 0;
+        }
         Begin kind = kList;
         bool least = true;
         unsigned nfar = 0;

@@ -710,6 +710,31 @@ def test_automatic_near_far_on_a_deep_graph():
         assert st.advances == 0
 
 
+@pytest.mark.parametrize("auto_rounds", [256, 700])
+def test_a_deep_computation_goes_on_near_far(auto_rounds):
+    """Plain rounds past opts.auto_rounds go on near-far on a large sparse graph: the first tree of a
+    725 x 725 grid, and a first batch on a loaded tree that cuts half of it, give the tree of
+    plain rounds (positive weights: one tree)."""
+    a = 725
+    n = a * a
+    u, v, w = D.gen_grid(a, a, 0.0, 0, 1, 100, seed=31)
+    cut = np.flatnonzero((u % a < 60) & (v % a < 60) & (np.minimum(u, v) < 60 * a) & (u // a + u % a == 60))
+    ch = D.make_changes(u[cut], v[cut], w[cut], np.zeros(len(cut)))
+    got = []
+    for opts in ({"auto_rounds": auto_rounds}, {"delta": 0}):
+        with D.Graph(n, u, v, w, **opts) as g:
+            st = g.tree_compute(0)
+            assert (st.advances > 0) == ("auto_rounds" in opts) and st.rounds > 1000
+            tree = g.tree_read()
+        with D.Graph(n, u, v, w, **opts) as g:
+            g.tree_load(*tree)
+            st = g.apply_batch(ch)
+            assert (st.advances > 0) == ("auto_rounds" in opts and st.rounds > auto_rounds)
+            assert g.validate()["violations"] == 0
+            got.append((*tree, *g.tree_read()))
+    assert all(np.array_equal(x, y) for x, y in zip(*got))
+
+
 def test_create_with_null_opts_and_edgeless_graph():
     """dsssp_graph_create with NULL options takes the defaults; an edgeless graph keeps the
     options it is given."""
