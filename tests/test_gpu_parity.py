@@ -870,6 +870,34 @@ def test_far_lists_around_one_pass_of_the_grid(leaves, opts):
         check_against_oracle(n, u, v, w, ch, 0, p, d, f"{leaves} leaves, batch")
 
 
+@pytest.mark.parametrize("width", [1, 2, 3, 4, 5, 7, 8, 9, 13, 40])
+def test_deletions_at_every_place_of_a_sorted_row(width):
+    """Rows of `width` neighbours joined by one to six parallel lines each: deletions of one weight
+    per pair (each twice in the batch), of several weights of one pair, and of lines that are not
+    there, at the edges of the search's last four entries; every other row end lies in the row
+    of a hub, so both choices of the shorter row occur."""
+    rng = np.random.default_rng(width)
+    rows, u, v, w = 60, [], [], []
+    n = 1 + rows + width
+    for r in range(rows):
+        u.append(0), v.append(1 + r), w.append(200 + r)  # the hub keeps every row reachable
+        for k in range(width):
+            for _ in range(1 + (r + k) % 6):
+                u.append(1 + r), v.append(1 + rows + k), w.append(int(rng.integers(1, 9)))
+    u, v, w = (np.ascontiguousarray(x, np.int32) for x in (u, v, w))
+    pick = np.flatnonzero((u != 0) & (rng.random(len(u)) < 0.5))
+    pick = np.concatenate([pick, pick[::2]])
+    ch = np.concatenate([D.make_changes(u[pick], v[pick], w[pick], np.zeros(len(pick))),
+                         D.make_changes(v[pick], u[pick], w[pick] + 50, np.zeros(len(pick)))])
+    u1, v1, w1 = lines_after(n, u, v, w, ch)
+    with D.Graph(n, u, v, w) as g:
+        g.tree_compute(0)
+        st = g.apply_batch(ch)
+        assert st.tombstoned == 2 * (len(u) - len(u1)) and g.health()["live"] == 2 * len(u1)
+        p, d = g.tree_read()
+        check_against_oracle(n, u, v, w, ch, 0, p, d, f"width {width}")
+
+
 def test_a_self_loop_deleted_by_many_records_is_counted_once():
     """Self-loops among which many are one line repeated, each deleted by many records of one
     batch: the live count afterwards is exact (every entry is tombstoned and counted once)."""
