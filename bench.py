@@ -346,8 +346,8 @@ def pipelined_e2e(D, g, ch, h_ch, h_dist32_after, reset, sptr, pairs: int = 5) -
     copy overlapping the next batch's upload and kernels.  Checked: after B the distances are
     those of B alone (the e2e leg's last read), after B and its inverse those of the start.
     Every batch adds 2 x 500k adjacency entries while its deletions only tombstone theirs, so
-    rows outgrow their slack and, within about ten steps, the spare region: the repack that
-    follows (a full compaction) is part of the timed stream.  apply_ms shows each step.
+    rows outgrow their slack: their growth, and a repack should the spare region be used up, is
+    part of the timed stream.  apply_ms shows each step.
     Returns a dict (see its keys)."""
     import ctypes as C
 

@@ -14,6 +14,7 @@
 //               Each surviving insertion then relaxes both ends and seeds the first frontier
 //               (replaces insertEdge, gpuFunctions_undir.cuh:217-251)
 //   k_update    one persistent cooperative kernel with a bounded grid barrier:
+//               0. rows that the insertions overflow grow (grow.cuh)
 //               A. cut-off subtrees are walked level by level from the roots (replaces
 //                  filterAffectedNodes + updateNeighbors_del and its host loop,
 //                  gpuFunctions_undir.cuh:125-144, 312-349, MAIN:219-239); after bfs_levels
@@ -27,8 +28,8 @@
 //                  gpuFunctions_undir.cuh:162-174, 370-433, MAIN:263-281).  With a bucket
 //                  width delta > 0 the rounds are near-far ordered: a vertex whose new
 //                  distance is at or above the threshold T waits in a de-duplicated far list;
-//                  when the near frontier runs dry, T moves to (least far distance) + delta
-//                  and the far list is split again.  High-diameter graphs then settle most
+//                  when the near frontier runs dry, T moves on and the far list is split
+//                  again.  Small levels and rounds run as local stretches in the CTAs' queues.  High-diameter graphs then settle most
 //                  vertices once instead of once per improving wave.  The result is the same
 //                  fixpoint: exact distances, the same parents.
 // Load balance: a vertex entering a frontier is split by degree into work items -- rows of
@@ -840,14 +841,15 @@ __device__ void run_items(Op& op, const UpdParams& p, const Item* tl, unsigned n
 // counts on grids of 1.6M and 16.8M vertices), then the push, the block barrier and, per stretch,
 // a grid barrier with a new deal of the work.  So the push is kept short (one shared atomic a
 // warp, no ranking bits unless a row takes two places), the fields of the parameter block are
-// held in registers and the pushed row is prefetched: 27.0 -> 23.7 ms on the 4096^2 grid below.
+// held in registers and the pushed row is prefetched: 27.0 -> 23.7 ms on the 4096^2 grid below; with
+// the shorter usual push, barrier and advances 22.8 ms.
 // A queue per CTA, not per warp: with one per warp a step was shorter, but a queue that grew past
 // 32 entries took several steps a hop and the others waited for it (21,476 steps and 46 ms
 // against 12,310 and 36 ms).  A CTA whose queue passes one and a half passes ends everybody's
 // stretch (rstop), so the work is dealt out again when it is needed and not every 16 or 64 steps
 // (27.1 ms against 28.6 and 36).  Measured against rounds throughout: a 4096^2 grid with 100k
-// changes 95.0 -> 23.7 ms a batch, a 1021 x 1543 grid with 9k changes 23.3 -> 6.3 ms, the tree of
-// a 2048^2 grid 38.0 -> 9.7 ms, ER graphs of 10k and 300k vertices 0.157 -> 0.130 and 0.264 ->
+// changes 95.0 -> 22.8 ms a batch, a 1021 x 1543 grid with 9k changes 23.3 -> 5.7 ms, the tree of
+// a 2048^2 grid 38.0 -> 9.1 ms, ER graphs of 10k and 300k vertices 0.157 -> 0.130 and 0.264 ->
 // 0.211 ms of k_update.
 // A round is a local stretch when it holds thread items only, no more than one pass of every CTA:
 // above that the grid is busy and the rounds' throughput counts.  (Half or a quarter of a pass:
@@ -2135,7 +2137,8 @@ __global__ void k_grow_finish(UpdParams p) {
 template <bool kAgg>
 __device__ void update_body(const UpdParams& p);
 
-// 3 CTAs of 256 threads per SM: 80 registers a thread without spills.  Every walk level and
+// 3 CTAs of 256 threads per SM: 80 registers a thread (2 CTAs: the tree of RMAT-22 1.354 -> 1.749 ms;
+// 4: 1.430 ms, a grid batch 6.1 -> 7.3 ms).  Every walk level and
 // relaxation round waits on its slowest CTA's chain of dependent accesses, so shorter chains
 // and fewer CTAs at each barrier beat more resident warps here (4 CTAs per SM with 64
 // registers and spills was slower on every workload but the throughput-bound 256-graph batch).

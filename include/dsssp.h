@@ -82,12 +82,15 @@ typedef struct {
     int32_t delta;        /* near-far bucket width of the relaxation rounds: 0 = plain frontier
                              rounds; > 0 = a round relaxes only vertices whose distance is below
                              a threshold T, the others wait until the near frontier is empty and
-                             T moves to (least waiting distance) + delta.  Same results; far
-                             fewer rounds and relaxations on high-diameter graphs.  -1 (the
-                             default) = automatic: near-far with 32 x the mean edge weight once
-                             the last batch or tree computation needed more than auto_rounds
-                             rounds, plain rounds otherwise.  Costs 12 bytes per vertex, allocated when
-                             first used. */
+                             T moves on by delta (over a gap, to the least waiting distance + delta).
+                             Same results; far fewer rounds and relaxations on high-diameter graphs.
+                             -1 (the default) = automatic: near-far with 32 x the mean edge weight
+                             once the last batch or tree computation needed more than auto_rounds
+                             rounds, plain rounds otherwise; on graphs of at least 2^19 vertices
+                             with at most 8 adjacency entries each a plain computation that passes
+                             auto_rounds rounds goes on near-far.  Costs 12 bytes per vertex,
+                             allocated when first used, on such graphs with the graph (if a quarter
+                             of the device's memory is free). */
     int32_t launch_graph; /* 1 = a batch's launch sequence (the four kernels, the status read) is
                              replayed from an instantiated CUDA graph whose node parameters are
                              updated per batch; 0 = plain stream launches.  Falls back to plain launches
@@ -105,7 +108,8 @@ typedef struct {
                              work items runs on one CTA with block barriers instead of the whole
                              grid (0..64; 0 = never; default 2) */
     int32_t auto_rounds;  /* delta = -1: near-far rounds start once the last batch or tree
-                             computation needed more than this many rounds (default 256) */
+                             computation needed more than this many rounds, on large sparse graphs
+                             (see delta) after this many in the computation itself (default 256) */
     int32_t group_ctas;   /* a relaxation round too large for one CTA (solo_waves) but at most
                              group_waves CTA-waves on group_ctas CTAs runs on the first group_ctas
                              CTAs with a barrier of their own while the other CTAs wait: a shorter
