@@ -515,6 +515,7 @@ struct dsssp_graph {
     cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     unsigned epoch = 0;
     int coop_grid = 0;
+    int pend_grid = 0;         // CTAs of the pending batch's update kernel
     // the batch launch sequence as an instantiated CUDA graph (opts.launch_graph)
     cudaGraph_t bgraph = nullptr;
     cudaGraphExec_t bexec = nullptr;
@@ -1068,6 +1069,16 @@ struct BatchNodes {
     cudaKernelNodeParams kp[4];
 };
 
+// CTAs of a batch's update kernel: one per SM where graph and batch are small, which then waits for
+// fewer at its barriers.  Batch and inverse, update kernel: ER of 10,000 vertices with 100, 1,000 and
+// 4,000 changes 0.101 -> 0.096, 0.154 -> 0.148 and 0.194 -> 0.185 ms (10,000 changes: 0.284 -> 0.297),
+// of 1,000 vertices with 20 0.085 -> 0.080; RMAT-13 with 200 and 4,000 0.100 -> 0.089 and 0.274 -> 0.260;
+// grids of up to 181^2 the same within 2 % and of 256^2 1.57 -> 1.65 ms, hence the line at 2^15 vertices.
+// Trees from scratch have wider rounds (ER of 10,000: 0.088 -> 0.097 ms) and keep the full grid.
+int update_grid(const dsssp_graph* g, long long k) {
+    return g->o.ctas_per_sm == 0 && g->n <= (1 << 15) && k <= 4096 ? g->num_sms : g->coop_grid;
+}
+
 void batch_nodes(const dsssp_graph* g, const UpdParams& p, BatchNodes& b) {
     const void* fns[4];
     batch_kernels(fns);
@@ -1081,7 +1092,7 @@ void batch_nodes(const dsssp_graph* g, const UpdParams& p, BatchNodes& b) {
         cudaKernelNodeParams& k = b.kp[i];
         k = cudaKernelNodeParams{};
         k.func = const_cast<void*>(fns[i]);
-        k.gridDim = dim3(i < 3 ? front : (unsigned)g->coop_grid);
+        k.gridDim = dim3(i < 3 ? front : (unsigned)g->pend_grid);
         k.blockDim = dim3(i < 3 ? 256u : (unsigned)g->o.block);
         k.sharedMemBytes = 0;
         k.kernelParams = b.args;
@@ -1181,6 +1192,7 @@ int enqueue_batch(dsssp_graph* g, const int4* d_chg, const int4* src, long long 
     p.hmask = h - 1;
     p.chg_src = src;
     g->pend_rb0 = g->h_ctl->round_base;  // the device reads the same value (mirror)
+    g->pend_grid = update_grid(g, k);
     g->pend_graph = launch_batch_graph(g, p, s);
     if (g->pend_graph) return DSSSP_OK;
     const bool ev = g->o.timing != 0;
@@ -1188,7 +1200,7 @@ int enqueue_batch(dsssp_graph* g, const int4* d_chg, const int4* src, long long 
     const bool fev = g->o.timing >= 2;
     CK(launch_front(p, g->num_sms * 8, s, fev ? g->ev[4] : nullptr, fev ? g->ev[5] : nullptr), "insert/delete kernels");
     if (ev) CK(cudaEventRecord(g->ev[1], s), "event");
-    CK(launch_update(p, g->coop_grid, g->o.block, s), "update kernel");
+    CK(launch_update(p, g->pend_grid, g->o.block, s), "update kernel");
     if (ev) CK(cudaEventRecord(g->ev[2], s), "event");
     CK(cudaMemcpyAsync(g->h_ctl, g->dg.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s), "status read");
     return DSSSP_OK;
@@ -1260,7 +1272,7 @@ int finish_batch(dsssp_graph* g, dsssp_stats* st) {
         UpdParams p = make_params(g, g->pend_chg, g->pend_k, 0);
         // the front interval now spans the repack; the update interval is the resumed launch
         if (g->pend_events) CK(cudaEventRecord(g->ev[1], s), "event");
-        CK(launch_update(p, g->coop_grid, g->o.block, s), "update kernel");
+        CK(launch_update(p, g->pend_grid, g->o.block, s), "update kernel");
         if (g->pend_events) CK(cudaEventRecord(g->ev[2], s), "event");
         CK(cudaMemcpyAsync(g->h_ctl, g->dg.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s), "status read");
         CK(cudaStreamSynchronize(s), "batch");
@@ -1269,7 +1281,7 @@ int finish_batch(dsssp_graph* g, dsssp_stats* st) {
         // The update kernel gave up while rows were to grow.  Once every CTA had passed the
         // growth's last phase but one, the last phase is run again; before that the rows stand as
         // the insertions left them, and a repack takes their overflow in.
-        if (g->h_ctl->grow_done == (unsigned)g->coop_grid) {
+        if (g->h_ctl->grow_done == (unsigned)g->pend_grid) {
             CK(launch_grow_finish(make_params(g, g->pend_chg, g->pend_k, 0), g->num_sms, s), "row growth");
         } else {
             CK(cudaMemsetAsync(g->d_gidx, 0, sizeof(int) * (size_t)g->n, s), "row growth");
@@ -1306,7 +1318,7 @@ int finish_batch(dsssp_graph* g, dsssp_stats* st) {
         rc = fail(DSSSP_E_TIMEOUT,
                   "grid barrier #%u timed out with %u of %d CTAs arrived; %u CTAs timed out; "
                   "CTA barrier counts at exit: min %u max %u",
-                  d[0], d[1], g->coop_grid, d[2], 0xFFFFFFFFu - d[4], d[3]);
+                  d[0], d[1], g->pend_grid, d[2], 0xFFFFFFFFu - d[4], d[3]);
     } else {
         rc = status_code(dev_status);
     }

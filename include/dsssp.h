@@ -71,7 +71,8 @@ typedef struct {
     int32_t chunk;        /* edges per CTA work item */
     int32_t bfs_levels;   /* subtree walk levels before switching to pointer jumping */
     int32_t block;        /* threads per CTA of the update kernel (multiple of 32) */
-    int32_t ctas_per_sm;  /* resident CTAs per SM of the update kernel; 0 = occupancy max */
+    int32_t ctas_per_sm;  /* resident CTAs per SM of the update kernel; 0 = occupancy max, one for
+                             batches of at most 4096 changes on graphs of at most 2^15 vertices */
     int32_t timing;       /* 1 = record CUDA events and phase timestamps into the stats; 2 = also
                              events between the batch front kernels (t_delete_ms, t_append_ms),
                              which costs a batch a few microseconds */

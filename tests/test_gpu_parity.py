@@ -898,6 +898,22 @@ def test_deletions_at_every_place_of_a_sorted_row(width):
         check_against_oracle(n, u, v, w, ch, 0, p, d, f"width {width}")
 
 
+@pytest.mark.parametrize("n", [32767, 32768, 32769])
+def test_small_batches_around_the_one_cta_grid(n):
+    """Streams of batches just below, at and above the sizes (2^15 vertices, 4,096 changes) up to
+    which the update kernel runs with one CTA per SM, changing over within one graph, rows growing."""
+    u, v, w = D.gen_er(n, 4 * n, 1, 100, 91)
+    with D.Graph(n, u, v, w, slack_pct=0, slack_min=1, spare_pct=60) as g:
+        g.tree_compute(0)
+        for seed, k in ((92, 4095), (93, 4096), (94, 4097), (95, 20000), (96, 1), (97, 4096)):
+            ch = D.gen_changes(n, u, v, w, k - k // 2, k // 2, seed=seed)
+            g.apply_batch(ch)
+            p, d = g.tree_read()
+            check_against_oracle(n, u, v, w, ch, 0, p, d, f"{k} changes")
+            u, v, w = lines_after(n, u, v, w, ch)
+            assert g.health()["live"] == 2 * len(u) and g.validate()["violations"] == 0
+
+
 def test_a_self_loop_deleted_by_many_records_is_counted_once():
     """Self-loops among which many are one line repeated, each deleted by many records of one
     batch: the live count afterwards is exact (every entry is tombstoned and counted once)."""
