@@ -908,6 +908,17 @@ int repack(dsssp_graph* g, const int4* d_ovf, int n_ovf, cudaStream_t s) {
     return rc;
 }
 
+// A tree from scratch on a large graph of whose rows more than one in 64 is above kLocalDeg entries goes
+// by items of twice the default's size: its rounds are wide, and an item costs 16 bytes to write and
+// read and a load of its vertex's state.  RMAT of scale 22 with 16, 32 and 64 million edges 0.90 ->
+// 0.83, 1.39 -> 1.34 and 2.67 -> 2.30 ms, of scale 20 with 8 million 0.465 -> 0.443, ER of 2^20 vertices
+// with 16 and 32 edges each 1.68 -> 1.61 and 2.60 -> 2.41 ms; RMAT-18 the same, RMAT-16 0.157 -> 0.165, and
+// on shorter rows (ER with 4 edges each) 0.57 -> 0.64 ms.  Options that were set stay.
+bool wide_items(const dsssp_graph* g) {
+    return g->o.small_deg == 4 && g->o.large_deg == 256 && g->n >= (1 << 18) &&
+           64ull * g->h_ctl->long_rows > (unsigned long long)g->n;
+}
+
 UpdParams make_params(const dsssp_graph* g, const int4* chg, long long k, int mode) {
     UpdParams p;
     p.g = g->dg;
@@ -927,8 +938,9 @@ UpdParams make_params(const dsssp_graph* g, const int4* chg, long long k, int mo
     p.grow.spare_from = (unsigned long long)g->spare_top;
     p.grow.slack_min = g->o.slack_min > 4 ? g->o.slack_min : 4;
     p.epoch = g->epoch;
-    p.te = g->o.small_deg;
-    p.large_deg = g->o.large_deg;
+    const bool wide = mode == 1 && wide_items(g);
+    p.te = wide ? 8 : g->o.small_deg;
+    p.large_deg = wide ? 512 : g->o.large_deg;
     p.chunk = g->o.chunk;
     p.bfs_levels = g->o.bfs_levels;
     p.mode = mode;
@@ -1627,6 +1639,7 @@ int dsssp_graph_create(int32_t n, int64_t m, const int32_t* u, const int32_t* v,
     size_t room = 0, total = 0;
     if (may_run_deep(g) && cudaMemGetInfo(&room, &total) == cudaSuccess && room > total / 4)
         (void)ensure_far(g);  // without them all rounds of the first computation are plain
+    cudaMemcpyAsync(&g->h_ctl->long_rows, &d.ctl->long_rows, sizeof(d.ctl->long_rows), cudaMemcpyDeviceToHost, s);
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { dsssp_graph_destroy(g); return cuda_fail(e, "graph build"); }
     *out = g;

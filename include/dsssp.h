@@ -67,7 +67,9 @@ typedef struct {
     int32_t small_deg;    /* edges per thread work item (multiple of 4, 4..64): a frontier
                              vertex of degree d <= small_deg is one thread's item, a longer row
                              up to large_deg is split into ceil(d/small_deg) thread items */
-    int32_t large_deg;    /* rows above this degree are split into CTA items of `chunk` edges */
+    int32_t large_deg;    /* rows above this degree are split into CTA items of `chunk` edges (with
+                             small_deg 4 and large_deg 256, the defaults, a tree from scratch on a
+                             large graph of long rows takes 8 and 512) */
     int32_t chunk;        /* edges per CTA work item */
     int32_t bfs_levels;   /* subtree walk levels before switching to pointer jumping */
     int32_t block;        /* threads per CTA of the update kernel (multiple of 32) */

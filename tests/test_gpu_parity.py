@@ -914,6 +914,30 @@ def test_small_batches_around_the_one_cta_grid(n):
             assert g.health()["live"] == 2 * len(u) and g.validate()["violations"] == 0
 
 
+@pytest.mark.parametrize("scale,factor", [(17, 16), (18, 16), (18, 1)])
+def test_trees_from_scratch_by_wide_items(scale, factor):
+    """RMAT graphs around the line from which a tree from scratch goes by wide items (2^18 vertices,
+    one row in 64 above 32 entries): the first tree, one from another source and one after a batch are
+    those of narrow items."""
+    n = 1 << scale
+    u, v, w = D.gen_rmat(scale, factor << scale, seed=17)
+    hub = int(np.bincount(np.concatenate([u, v]), minlength=n).argmax())
+    ch = D.gen_changes(n, u, v, w, 3000, 3000, seed=18)
+    got = []
+    for opts in ({}, {"large_deg": 257}):
+        with D.Graph(n, u, v, w, **opts) as g:
+            g.tree_compute(hub)
+            trees = [g.tree_read()]
+            g.tree_compute(int(u[0]))
+            trees.append(g.tree_read())
+            g.apply_batch(ch)
+            g.tree_compute(hub)
+            assert g.validate()["violations"] == 0
+            got.append(trees + [g.tree_read()])
+    for x, y in zip(*got):
+        assert np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1])
+
+
 def test_a_self_loop_deleted_by_many_records_is_counted_once():
     """Self-loops among which many are one line repeated, each deleted by many records of one
     batch: the live count afterwards is exact (every entry is tombstoned and counted once)."""
