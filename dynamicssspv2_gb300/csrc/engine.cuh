@@ -232,7 +232,8 @@ struct UpdParams {
     unsigned* seedq;  // vertices seeded by k_append (claimed, expanded by k_update)
     const int* srcs;  // mode 1: the sources (every root is its own parent)
     int nsrc;
-    long long max_rounds;
+    long long max_rounds;  // of lists: a round or a local stretch each
+    int capped;       // 1 = that is the caller's own cap and may bind: rounds alone, which it counts
     unsigned solo_waves;  // steps of at most this many CTA-waves of items run on CTA 0 alone
     unsigned group_ctas;  // mid-size steps run on CTAs [0, group_ctas) with a group barrier (0 = off)
     unsigned group_waves; // ... a step is mid-size up to group_ctas * group_waves CTA-waves of items

@@ -945,12 +945,15 @@ UpdParams make_params(const dsssp_graph* g, const int4* chg, long long k, int mo
     p.bfs_levels = g->o.bfs_levels;
     p.mode = mode;
     p.delta = g->dg.far_tag ? effective_delta(g) : 0ull;  // the caller ensured the lists
-    p.late_delta = !p.delta && g->dg.far_tag && g->o.delta < 0 ? auto_delta(g) : 0ull;
+    // a cap that plain rounds cannot pass is none; under another one the rounds stay what it counts
+    const long long enough = 2LL * g->n + 16;
+    p.max_rounds = g->o.max_rounds > 0 ? g->o.max_rounds : enough;
+    p.capped = p.max_rounds < enough;
+    p.late_delta = !p.delta && !p.capped && g->dg.far_tag && g->o.delta < 0 ? auto_delta(g) : 0ull;
     p.late_after = (unsigned)g->o.auto_rounds;
     p.seedq = g->d_seedq;
     p.srcs = g->d_srcs;
     p.nsrc = 0;
-    p.max_rounds = g->o.max_rounds > 0 ? g->o.max_rounds : 2LL * g->n + 16;
     p.solo_waves = (unsigned)g->o.solo_waves;
     p.group_ctas = (unsigned)g->o.group_ctas;
     p.group_waves = (unsigned)g->o.group_waves;
@@ -1243,9 +1246,9 @@ int recover_after_failure(dsssp_graph* g, int rc, dsssp_stats* st) {
     snprintf(why, sizeof why, "%s", dsssp_last_error());
     const std::vector<int> roots = g->roots;
     dsssp_stats rs;
-    // the recomputation runs with the default round cap (2n + 16): after round r of a
-    // computation from the sources every vertex with a shortest path of at most r edges is
-    // final, so it needs fewer than n rounds
+    // the recomputation runs with the default round cap (2n + 16): after list r of a computation
+    // from the sources (a round or a local stretch) every vertex with a shortest path of at most r
+    // edges is final, so it needs fewer than n + 2, near-far lists among them fewer than 2n + 16
     const long long cap = g->o.max_rounds;
     g->o.max_rounds = 0;
     const int rr = dsssp_tree_compute_multi(g, roots.data(), (int32_t)roots.size(), &rs);

@@ -825,7 +825,7 @@ __device__ void run_items(Op& op, const UpdParams& p, const Item* tl, unsigned n
 // ---- local stretches -------------------------------------------------------------------------
 // A relaxation round of few items is one chain of dependent accesses plus a grid barrier, about
 // 8 us however small it is.  A local stretch replaces a run of such rounds: every CTA takes a share
-// of the round's items into a queue in shared memory and relaxes on from there for up to `steps`
+// of the round's items into a queue in shared memory and relaxes on from there for up to `kStretch`
 // steps, pushing what it improves into the next step's queue, with one block barrier a step and
 // no grid barrier.  Four lanes share an item of at most four entries, and the chain of a step is
 // two accesses long: the entry beside the vertex's own state, then the offer beside the
@@ -859,6 +859,13 @@ __device__ __forceinline__ bool local_step(const UpdParams& p, unsigned nt, unsi
 }
 
 __device__ __forceinline__ void keep_stats(const LocalStats& ls);
+
+// Whether relaxations may run in local stretches and far lists go whole into them.  Not under a round
+// cap of the caller's that may bind: the steps of a stretch add up to more than the depth, by how
+// much depends on which CTA was faster, so a cap that is enough for the rounds would stop a batch
+// that converges, and not in every run.  Such a call takes the rounds it counts, each at its own
+// barrier.
+__device__ __forceinline__ bool stretches(const UpdParams& p) { return p.capped == 0; }
 
 // A graph of whose rows nearly all fit a stretch's queue.  On others (RMAT: one row in ten above
 // kLocalDeg) a stretch soon leaves through the lists, and the phases before it are better kept
@@ -1095,9 +1102,9 @@ struct Stretch {
 // list, `before` the threshold till now: what lies below T is near, the rest waits on.  A function
 // of its own, with its own counters, so that the rounds keep their registers.
 enum Begin { kList, kPulls, kWaiting };
-__device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigned nt, unsigned steps_max,
-                                         unsigned rbase, unsigned adv, unsigned long long T, Begin kind, unsigned nd,
-                                         unsigned ns, unsigned long long before) {
+__device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigned nt, unsigned rbase, unsigned adv,
+                                         unsigned long long T, Begin kind, unsigned nd, unsigned ns,
+                                         unsigned long long before) {
     Ctl* const ctl = p.g.ctl;
     const bool odd = (r & 1) != 0;
     const unsigned slot = (r + 1) % 3;
@@ -1142,7 +1149,7 @@ __device__ __noinline__ void relax_local(const UpdParams& p, unsigned r, unsigne
     unsigned k = 0, n, cur = 0, nxt = 1, old = 2;  // the steps' counters rotate
     for (;; k++) {
         n = min(s_qcnt[cur], kQueue);
-        if (n == 0 || k >= steps_max || s_stop[k & 1]) break;
+        if (n == 0 || k >= kStretch || s_stop[k & 1]) break;
         if (n > limit && k > 0) {  // too much for this CTA: everybody's work is dealt out again
             if (threadIdx.x == 0) atomicExch(stopped, 1u);
             break;
@@ -1400,7 +1407,7 @@ __device__ __forceinline__ void clear_slots(Ctl* ctl, unsigned slot) {
 enum Advance { kStop, kSplit, kWhole };
 template <bool kAgg>
 __device__ __noinline__ Advance advance(const UpdParams& p, unsigned r, unsigned nfar, unsigned rbase, unsigned adv,
-                                        unsigned long long T, bool least, unsigned hops) {
+                                        unsigned long long T, bool least) {
     Ctl* const ctl = p.g.ctl;
     const unsigned long long tn = next_threshold(p, nfar, adv, T, least);
     if (tn == 0) return kStop;
@@ -1408,7 +1415,7 @@ __device__ __noinline__ Advance advance(const UpdParams& p, unsigned r, unsigned
         ctl->fc[(adv + 2) % 3] = 0;
         ctl->fmin[(adv + 1) & 1] = 0;
     }
-    const bool whole = !kAgg && hops < p.max_rounds && local_advance(p, nfar);
+    const bool whole = !kAgg && stretches(p) && local_advance(p, nfar);
     if (!whole && !far_advance(p, r, nfar, rbase, adv, T, tn)) return kStop;
     if (threadIdx.x == 0) s_threshold = tn;
     __syncthreads();
@@ -2215,7 +2222,10 @@ __device__ void update_body(const UpdParams& p) {
 
     unsigned nT = 0, nC = 0;  // the sizes of the next relaxation round's lists
     // r counts the lists (a round or a local stretch each), hops the rounds and the steps of
-    // the stretches: the depth of the dependent relaxations
+    // the stretches, the most of any CTA: at least the depth of the dependent relaxations.  The cap
+    // is on r.  A list relaxes every vertex that waits in it, so after r of them all shortest paths
+    // of r edges are found, as after r rounds, and in a plain computation r stays below n + 2.  A
+    // near-far phase settles a vertex at least for each of its lists: below 2n + 16 in all.
     unsigned r = 0, hops = 0;
     if (p.mode == 1) {
         PushBuf pb{pbuf, 0};
@@ -2238,11 +2248,10 @@ __device__ void update_body(const UpdParams& p) {
         if (leader) ctl->ts[1] = globaltimer();
 
         const unsigned ns = __ldcg(&ctl->seed_count), nd = __ldcg(&ctl->walk_done);
-        if (!kAgg && !nf && p.te == 4 && p.max_rounds > 0 && local_step(p, ns + hiT + nd, hiC) && short_rows(p)) {
+        if (!kAgg && !nf && p.te == 4 && stretches(p) && local_step(p, ns + hiT + nd, hiC) && short_rows(p)) {
             // few enough for one stretch: its list is number 2 (rt0; rt1 holds items of the walk)
             if (leader) ctl->ts[2] = ctl->ts[1];
-            relax_local(p, 1, hiT, p.max_rounds < (long long)kStretch ? (unsigned)p.max_rounds : kStretch, rbase, 0, T,
-                        kPulls, nd, ns, 0);
+            relax_local(p, 1, hiT, rbase, 0, T, kPulls, nd, ns, 0);
             if (!grid_sync(ctl, &ctl->rcT[2], &ctl->rcC[2], nT, nC, &ctl->rsteps[2], hops)) return;
             r = 2;
         } else {
@@ -2272,9 +2281,9 @@ __device__ void update_body(const UpdParams& p) {
             // near frontier empty: advance the threshold past the least waiting distance
             nfar = __ldcg(&ctl->fc[adv % 3]);
             if (nfar == 0) break;
-            least = T == 0 || sparse;
+            least = T == 0 || sparse || !stretches(p);
             before = T;
-            const Advance got = advance<kAgg>(p, r, nfar, rbase, adv, T, least, hops);
+            const Advance got = advance<kAgg>(p, r, nfar, rbase, adv, T, least);
             if (got == kStop) break;
             T = s_threshold;
             adv++;
@@ -2290,15 +2299,13 @@ __device__ void update_body(const UpdParams& p) {
                 }
             }
         }
-        if (hops >= p.max_rounds) {
+        if (r >= p.max_rounds) {
             if (leader) set_status(ctl, -5 /* NO_CONVERGENCE */);
             break;
         }
-        if (!kAgg && (kind == kWaiting || local_step(p, nT, nC))) {
+        if (!kAgg && stretches(p) && (kind == kWaiting || local_step(p, nT, nC))) {
             if (leader) clear_slots(ctl, (r + 2) % 3);
-            const long long left = p.max_rounds - hops;
-            relax_local(p, r, nT, left < (long long)kStretch ? (unsigned)left : kStretch, rbase, adv, T, kind, 0, nfar,
-                        before);
+            relax_local(p, r, nT, rbase, adv, T, kind, 0, nfar, before);
             unsigned t2, used;
             if (!grid_sync(ctl, &ctl->rcT[(r + 1) % 3], &ctl->rcC[(r + 1) % 3], t2, nC, &ctl->rsteps[(r + 1) % 3], used))
                 break;
@@ -2316,7 +2323,7 @@ __device__ void update_body(const UpdParams& p) {
                 if (threadIdx.x < 6) s_solo_cnt[threadIdx.x / 2][threadIdx.x % 2] = 0;
                 __syncthreads();
                 for (int steps = 0; steps < kSoloSteps; steps++) {
-                    if ((t == 0 && c == 0) || !small_step(t, c, p.solo_waves) || hops + (rr - r) >= p.max_rounds) break;
+                    if ((t == 0 && c == 0) || !small_step(t, c, p.solo_waves) || rr >= p.max_rounds) break;
                     unsigned* cnt = s_solo_cnt[(rr + 1) % 3];
                     if (threadIdx.x == 0) {
                         s_solo_cnt[(rr + 2) % 3][0] = 0;
@@ -2360,7 +2367,7 @@ __device__ void update_body(const UpdParams& p) {
                 unsigned rr = r;
                 unsigned t = nT, c = nC;
                 for (int steps = 0; steps < kSoloSteps; steps++) {
-                    if ((t == 0 && c == 0) || !group_step(p, t, c) || hops + (rr - r) >= p.max_rounds) break;
+                    if ((t == 0 && c == 0) || !group_step(p, t, c) || rr >= p.max_rounds) break;
                     if (blockIdx.x == 0 && threadIdx.x == 0) {
                         ctl->rcT[(rr + 2) % 3] = 0;
                         ctl->rcC[(rr + 2) % 3] = 0;

@@ -78,7 +78,10 @@ typedef struct {
     int32_t timing;       /* 1 = record CUDA events and phase timestamps into the stats; 2 = also
                              events between the batch front kernels (t_delete_ms, t_append_ms),
                              which costs a batch a few microseconds */
-    int64_t max_rounds;   /* relaxation round cap; 0 = 2n + 16 */
+    int64_t max_rounds;   /* relaxation round cap; 0 = 2n + 16, which no computation passes.  Under a
+                             smaller cap the relaxations take a grid barrier per round, so that the
+                             cap counts rounds and nothing else; without it a run of small rounds
+                             goes without barriers (several times faster on high-diameter graphs) */
     int32_t spare_pct;    /* extra adjacency slots, percent of the laid-out rows, into which a
                              row that runs out of slack moves (no full repack) unless dropping
                              its tombstones leaves it room in place; 0..400 */
@@ -132,7 +135,9 @@ typedef struct {
     int64_t n_invalidated;     /* all vertices of the cut-off subtrees (roots included) */
     int64_t inv_levels;        /* subtree-walk levels */
     int64_t pj_passes;         /* pointer-jumping passes (0 if the walk finished) */
-    int64_t rounds;            /* relaxation rounds */
+    int64_t rounds;            /* relaxation rounds; of a run of small rounds without barriers the
+                                  most that any CTA took, so it may differ from call to call (not
+                                  under a round cap, see max_rounds) */
     int64_t frontier_total;    /* sum of frontier sizes over the rounds */
     int64_t edges_relaxed;     /* adjacency entries scanned by relaxation rounds and seeds */
     int64_t edges_inval;       /* adjacency entries scanned by the subtree walk and pulls */
