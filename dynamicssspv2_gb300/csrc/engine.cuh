@@ -69,7 +69,7 @@ enum StatIdx {
     ST_UPDATES,
     ST_OVF,
     ST_ITEMS,
-    ST_DIST_OVF,
+    ST_DIST_OVF,    // offers that did not fit, to vertices without a distance yet (k_dist_check decides)
     ST_ADVANCES,
     ST_TOMBS,
     ST_LIVE_INS,
@@ -104,7 +104,8 @@ struct __align__(128) Ctl {
     unsigned long long spare_top;     // the spare region's bump pointer after the growth (0: none)
     unsigned tail_count;  // chunks of long row tails that k_delete left to k_append
     unsigned grow_done;   // CTAs past the growth's last phase but one (all: that phase has run or may)
-    unsigned pad1[16];
+    unsigned dist_over;   // k_dist_check: a distance does not fit
+    unsigned pad1[15];
     // line 2
     unsigned bar_count;  // arrivals at the grid barrier since the launch of k_update, which finds 0 here
     unsigned pad2[31];

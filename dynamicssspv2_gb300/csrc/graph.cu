@@ -29,6 +29,7 @@ cudaError_t launch_front(const UpdParams& p, int grid, cudaStream_t s, cudaEvent
 cudaError_t update_occupancy(int block, int* blocks_per_sm);
 cudaError_t launch_update(const UpdParams& p, int grid, int block, cudaStream_t s);
 cudaError_t launch_grow_finish(const UpdParams& p, int grid, cudaStream_t s);
+cudaError_t launch_dist_check(const DevGraph& g, int grid, cudaStream_t s);
 void batch_kernels(const void* fns[4]);
 const void* update_kernel(bool warp_agg);
 const void* delete_kernel(bool tails);
@@ -1221,6 +1222,19 @@ int enqueue_batch(dsssp_graph* g, const int4* d_chg, const int4* src, long long 
     return DSSSP_OK;
 }
 
+// Whether a distance does not fit, once the update kernel has ended (its control block on the host):
+// the distances themselves are looked at only where an offer did not fit.
+int check_distances(dsssp_graph* g, cudaStream_t s, bool* over) {
+    *over = false;
+    if (g->h_ctl->status != 0 || g->h_ctl->stat[ST_DIST_OVF] == 0) return DSSSP_OK;
+    CK(launch_dist_check(make_params(g, nullptr, 0, 0).g, g->num_sms * 8, s), "distance check");
+    CK(cudaMemcpyAsync(&g->h_ctl->dist_over, &g->dg.ctl->dist_over, sizeof(unsigned), cudaMemcpyDeviceToHost, s),
+       "distance check");
+    CK(cudaStreamSynchronize(s), "distance check");
+    *over = g->h_ctl->dist_over != 0;
+    return DSSSP_OK;
+}
+
 // Statuses of the update kernel that leave the batch's adjacency edits in place and the tree
 // unfinished: a timed-out grid barrier, the round cap, an internal list capacity, a parent
 // cycle found by pointer jumping.  (Refused records, found before anything is modified, and a
@@ -1318,7 +1332,9 @@ int finish_batch(dsssp_graph* g, dsssp_stats* st) {
         g->dead += tombs - grow_dropped;
         if (g->h_ctl->stat[ST_LIVE_INS] > 0) g->tails = true;  // insertions appended to row tails
     }
-    g->delta_ok = g->h_ctl->status == 0 && g->h_ctl->stat[ST_DIST_OVF] == 0;
+    bool over = false;
+    const int checked = check_distances(g, s, &over);
+    g->delta_ok = g->h_ctl->status == 0 && !over && checked == DSSSP_OK;
     g->delta_empty = false;
     if (g->h_ctl->status == 0) g->last_rounds = (long long)g->h_ctl->stat[ST_ROUNDS];
     g->delta_lo = g->pend_rb0;
@@ -1326,7 +1342,8 @@ int finish_batch(dsssp_graph* g, dsssp_stats* st) {
     g->delta_epoch = g->epoch;
     const int dev_status = g->h_ctl->status;
     if (dev_status != 0) reset_tags(g, s);
-    if (g->h_ctl->stat[ST_DIST_OVF] > 0 && dev_status == 0) return status_code(DSSSP_E_OVERFLOW);
+    if (checked) return checked;
+    if (over) return status_code(DSSSP_E_OVERFLOW);
     int rc;
     if (dev_status == DSSSP_E_TIMEOUT) {
         const unsigned* d = g->h_ctl->diag;
@@ -1798,8 +1815,10 @@ static int compute_from_sources(dsssp_graph* g, const int32_t* srcs, int32_t k, 
     g->pend_graph = false;
     fill_stats(g, *g->h_ctl, st, ev, 0, 0);
     if (g->h_ctl->status != 0) reset_tags(g, s);
-    if (g->h_ctl->stat[ST_DIST_OVF] > 0 && g->h_ctl->status == 0) return status_code(DSSSP_E_OVERFLOW);
-    return status_code(g->h_ctl->status);
+    bool over = false;
+    rc = check_distances(g, s, &over);
+    if (rc) return rc;
+    return over ? status_code(DSSSP_E_OVERFLOW) : status_code(g->h_ctl->status);
 }
 
 int dsssp_tree_compute(dsssp_graph* g, int32_t src, dsssp_stats* st) {

@@ -24,6 +24,8 @@ namespace dsssp {
 
 cudaError_t update_occupancy(int block, int* blocks_per_sm);
 cudaError_t launch_update(const UpdParams& p, int grid, int block, cudaStream_t s);
+cudaError_t launch_dist_check(const DevGraph& g, int grid, cudaStream_t s);
+cudaError_t load_dist_check();
 void count_launch(int n);
 
 namespace {
@@ -125,6 +127,7 @@ int setup_device(int dev, DeviceSetup** out) {
         if (e != cudaSuccess) return fail(DSSSP_E_CUDA, "sssp_noalloc: cudaGetSymbolAddress: %s", cudaGetErrorString(e));
         int per_sm = 0, sms = 0;
         e = update_occupancy(kBlock, &per_sm);
+        if (e == cudaSuccess) e = load_dist_check();
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess || per_sm < 1)
             return fail(DSSSP_E_COOP, "sssp_noalloc: update kernel has no occupancy (%s)", cudaGetErrorString(e));
@@ -209,6 +212,15 @@ extern "C" int dsssp_sssp_noalloc(int32_t n, int64_t nnz, const int64_t* d_row_o
     memcpy(&dist_ovf, back + offsetof(Ctl, stat) + sizeof(dist_ovf) * ST_DIST_OVF, sizeof(dist_ovf));
     if (status == DSSSP_E_INVAL) return fail(DSSSP_E_INVAL, "sssp_noalloc: malformed CSR (offsets, ids or weights)");
     if (status != 0) return fail(status, "sssp_noalloc: device status %d", status);
+    if (dist_ovf) {  // an offer did not fit: do the distances?
+        unsigned over = 0;
+        e = launch_dist_check(p.g, ds->grid, s);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(&over, base + kOffCtl + offsetof(Ctl, dist_over), sizeof(over), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return fail(DSSSP_E_CUDA, "sssp_noalloc: %s", cudaGetErrorString(e));
+        dist_ovf = over;
+    }
     if (dist_ovf) return fail(DSSSP_E_OVERFLOW, "sssp_noalloc: a distance does not fit below 2^32-1");
     return DSSSP_OK;
 }

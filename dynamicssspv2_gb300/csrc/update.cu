@@ -2141,6 +2141,25 @@ __global__ void k_grow_finish(UpdParams p) {
                 (unsigned)(list >> 32), (unsigned)p.g.ctl->ovf_count);
 }
 
+// Whether a distance does not fit below 2^32-1: a vertex has none at the fixpoint although an entry
+// joins a reachable one to it.  Run only after offers that did not fit have been counted: such an
+// offer alone says nothing, a shorter path may come behind it, and which comes first depends on how
+// far the CTAs' queues are (in rounds it was the path of fewer hops).
+__global__ void k_dist_check(DevGraph g) {
+    const unsigned lane = lane_id();
+    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+    bool over = false;
+    for (long long v = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < g.n; v += warps) {
+        if (g.state[v] == kInfState) continue;
+        const RowDesc rd = g.rows[v];
+        for (int j = (int)lane; j < rd.deg; j += 32) {
+            const int2 e = g.adj[rd.start + j];
+            over |= e.y >= 0 && g.state[e.x] == kInfState;
+        }
+    }
+    if (__any_sync(kFull, over) && lane == 0) g.ctl->dist_over = 1;
+}
+
 template <bool kAgg>
 __device__ void update_body(const UpdParams& p);
 
@@ -2452,6 +2471,18 @@ cudaError_t launch_grow_finish(const UpdParams& p, int grid, cudaStream_t s) {
     k_grow_finish<<<(unsigned)grid, 256, 0, s>>>(p);
     count_launch(1);
     return cudaGetLastError();
+}
+
+cudaError_t launch_dist_check(const DevGraph& g, int grid, cudaStream_t s) {
+    k_dist_check<<<(unsigned)grid, 256, 0, s>>>(g);
+    count_launch(1);
+    return cudaGetLastError();
+}
+
+// Loads the kernel, so that its first launch allocates nothing.
+cudaError_t load_dist_check() {
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, (const void*)k_dist_check);
 }
 
 // The batch kernels as graph-node functions: k_prepare, k_delete, k_append, k_update.

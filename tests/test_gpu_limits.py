@@ -1,4 +1,4 @@
-"""Limits that a call states or meets: the caller's round cap."""
+"""Limits that a call states or meets: the caller's round cap, the range of the distances."""
 import numpy as np
 import pytest
 
@@ -83,3 +83,110 @@ def test_a_round_cap_on_near_far_rounds():
                 with pytest.raises(D.DsssspError) as e:
                     g.tree_compute(0)
                 assert e.value.code == D.E_NO_CONVERGENCE
+
+
+W = 1_500_000_000  # two of these fit a distance, three do not
+
+
+def _late_long_paths(gates, light, leaves):
+    """From vertex 1, behind vertex 0, `gates` pairs of paths to a vertex of their own each: a light one
+    whose vertices carry leaves, and a bare one a hop longer that ends in three edges of W."""
+    u, v, w, n = [[0]], [[1]], [[3]], 2
+    take = lambda k: np.arange(n, n + k)  # noqa: E731
+    ends = take(gates)
+    n += gates
+    prev = np.ones(gates, np.int64)
+    for _ in range(light - 1):
+        at = take(gates)
+        n += gates
+        u.append(prev), v.append(at), w.append(np.ones(gates))
+        hang = take(gates * leaves)
+        n += gates * leaves
+        u.append(np.repeat(at, leaves)), v.append(hang), w.append(np.ones(len(hang)))
+        prev = at
+    u.append(prev), v.append(ends), w.append(np.ones(gates))
+    prev = np.ones(gates, np.int64)
+    for hop in range(light):
+        at = take(gates)
+        n += gates
+        u.append(prev), v.append(at), w.append(np.full(gates, W if hop >= light - 2 else 1))
+        prev = at
+    u.append(prev), v.append(ends), w.append(np.full(gates, W))
+    return n, *_i32(*(np.concatenate(x) for x in (u, v, w)))
+
+
+@pytest.mark.parametrize("gates,opts", [(700, {"ctas_per_sm": 1}), (700, {}), (2000, {"warp_agg": 1}), (700, {"max_rounds": 400})],
+                         ids=str)
+def test_a_path_that_does_not_fit_beside_one_that_does(gates, opts):
+    """Every distance fits, but an offer that does not may come first, by how far the CTAs' queues are: the
+    computation and the batch that joins all of it to the root are not refused for it."""
+    n, u, v, w = _late_long_paths(gates, 60, 12)
+    join = D.make_changes(u[:1], v[:1], w[:1], np.ones(1))
+    with D.Graph(n, u, v, w, **opts) as g:
+        for _ in range(5):
+            g.tree_compute(0)
+        p, d = g.tree_read()
+        check_against_oracle(n, u, v, w, None, 0, p, d, "tree")
+    with D.Graph(n, u[1:], v[1:], w[1:], **opts) as g:
+        g.tree_compute(0)
+        g.snapshot()
+        for _ in range(5):
+            g.restore()
+            g.apply_batch(join)
+        p, d = g.tree_read()
+        check_against_oracle(n, u[1:], v[1:], w[1:], join, 0, p, d, "batch")
+        assert len(g.tree_read_changed()[0]) == n - 1
+
+
+@pytest.mark.parametrize("opts", [{}, {"delta": 1000}, {"max_rounds": 8}], ids=str)
+def test_a_distance_that_does_not_fit_is_refused(opts):
+    """A vertex that only a path of more than 2^32 - 2 reaches: the computation, a batch that makes it so
+    by a deletion or by an insertion and the call without allocation all report the overflow; what
+    fits is exact, and the batch that mends it is accepted."""
+    torch = pytest.importorskip("torch")
+    u, v, w = _i32([0, 1, 2, 3, 0, 0], [1, 2, 3, 4, 4, 5], [W, W, W, 7, 9, 1])
+    n = 6
+
+    def refused(call, *args):
+        with pytest.raises(D.DsssspError) as e:
+            call(*args)
+        assert e.value.code == D.E_OVERFLOW
+
+    cut = D.make_changes(u[4:5], v[4:5], w[4:5], np.zeros(1))
+    back = D.make_changes(u[4:5], v[4:5], w[4:5], np.ones(1))
+    far = D.make_changes([2], [6], [1_400_000_000], [1])
+    with D.Graph(n, u, v, w, **opts) as g:
+        g.tree_compute(0)
+        want = g.tree_read()
+        assert list(want[1]) == [0, W, W + 16, 16, 9, 1]
+        refused(g.apply_batch, cut)  # 3 and 4 only by three edges of W
+        assert list(g.tree_read()[1]) == [0, W, 2 * W, -1, -1, 1]
+        g.apply_batch(back)
+        assert all(np.array_equal(a, b) for a, b in zip(g.tree_read(), want))
+    with D.Graph(n + 1, u[[0, 1, 5]], v[[0, 1, 5]], w[[0, 1, 5]], **opts) as g:
+        g.tree_compute(0)
+        refused(g.apply_batch, far)
+        assert list(g.tree_read()[1]) == [0, W, 2 * W, -1, -1, 1, -1]
+    with D.Graph(n, u[[0, 1, 2, 5]], v[[0, 1, 2, 5]], w[[0, 1, 2, 5]], **opts) as g:
+        refused(g.tree_compute, 0)
+    off = torch.tensor([0, 1, 2, 3, 3], dtype=torch.int64, device="cuda")
+    adj = torch.tensor([[1, W], [2, W], [3, W]], dtype=torch.int32, device="cuda")
+    par = torch.empty(4, dtype=torch.int32, device="cuda")
+    dist = torch.empty(4, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    refused(D.sssp_noalloc, 4, 3, off.data_ptr(), adj.data_ptr(), 0, par.data_ptr(), dist.data_ptr())
+    adj[2, 1] = 2**31 - 1 - W  # 2 * W + that fits
+    torch.cuda.synchronize()
+    D.sssp_noalloc(4, 3, off.data_ptr(), adj.data_ptr(), 0, par.data_ptr(), dist.data_ptr())
+    assert dist.tolist() == [0, W, 2 * W, W + 2**31 - 1]
+
+
+def test_a_cut_off_vertex_beside_a_path_that_does_not_fit():
+    """A pull sees every neighbour's offer: one that does not fit beside one that does is no overflow."""
+    u, v, w = _i32([0, 1, 2, 0, 0], [1, 2, 3, 3, 3], [1_250_000_000, 1_250_000_000, 2 * 10**9, 10**9, 1_900_000_000])
+    with D.Graph(4, u, v, w) as g:
+        g.tree_compute(0)
+        ch = D.make_changes(u[3:4], v[3:4], w[3:4], np.zeros(1))
+        g.apply_batch(ch)
+        p, d = g.tree_read()
+        check_against_oracle(4, u, v, w, ch, 0, p, d, "pull")
