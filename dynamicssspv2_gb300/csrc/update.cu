@@ -1958,8 +1958,11 @@ __global__ void __launch_bounds__(256, 5) k_delete(UpdParams p) {
             const bool mine = c.z >= 0 && (had == kHashEmpty || had == pair);
             const int weight = mine ? atomicCAS(&slot->w, kHashNoWeight, c.z) : kHashNoWeight;
             if (p.g.twin) {
-                // search the shorter row; each match's reverse entry is found through twin[]
-                const bool use_a = ra.deg <= rb.deg;
+                // search the shorter row; each match's reverse entry is found through twin[].  Of rows
+                // of equal degree the lower vertex's, whichever end the record names first: records of
+                // one line then meet at one entry, whose compare-and-swap one of them wins (at an end
+                // each, both won, and the line's two entries were counted twice)
+                const bool use_a = ra.deg < rb.deg || (ra.deg == rb.deg && a <= b);
                 const RowDesc& rs = use_a ? ra : rb;
                 const int sl = p.g.sorted_len[use_a ? a : b];
                 const int col = (int)(use_a ? b : a);

@@ -1,4 +1,5 @@
-"""Limits that a call states or meets: the caller's round cap, the range of the distances."""
+"""Limits that a call states or meets: the caller's round cap, the range of the distances,
+the count of the entries."""
 import numpy as np
 import pytest
 
@@ -190,3 +191,39 @@ def test_a_cut_off_vertex_beside_a_path_that_does_not_fit():
         g.apply_batch(ch)
         p, d = g.tree_read()
         check_against_oracle(4, u, v, w, ch, 0, p, d, "pull")
+
+
+def _regular(kind):
+    if kind == "ring":
+        a = np.arange(4096)
+        return 4096, a, (a + 1) % 4096
+    side = 96  # a torus: every row has four entries
+    a = np.arange(side * side)
+    y, x = a // side, a % side
+    return side * side, np.concatenate([a, a]), np.concatenate([y * side + (x + 1) % side, (y + 1) % side * side + x])
+
+
+@pytest.mark.parametrize("tails", [False, True])
+@pytest.mark.parametrize("kind", ["ring", "torus"])
+def test_lines_deleted_in_both_orientations_are_counted_once(kind, tails):
+    """Rows of equal degree whose lines are deleted by many records of one batch, named from either end
+    side by side: every entry is counted as one tombstone (tails: after the lines have come back by
+    insertion, so that they lie in unsorted tails)."""
+    n, u, v = _regular(kind)
+    w = 1 + np.arange(len(u)) % 7
+    u, v, w = _i32(u, v, w)
+    gone = np.flatnonzero(np.arange(len(u)) % 8 != 0)
+    a, b = u[gone], v[gone]
+    both = D.make_changes(np.stack([a, b] * 4, 1).reshape(-1), np.stack([b, a] * 4, 1).reshape(-1), np.repeat(w[gone], 8),
+                          np.zeros(8 * len(gone)))
+    back = D.make_changes(a, b, w[gone], np.ones(len(gone)))
+    with D.Graph(n, u, v, w, slack_pct=0, slack_min=8) as g:
+        g.tree_compute(0)
+        if tails:
+            g.apply_batch(both)
+            g.apply_batch(back)
+        st = g.apply_batch(both)
+        assert st.tombstoned == 2 * len(gone)
+        assert g.health()["live"] == 2 * (len(u) - len(gone))
+        p, d = g.tree_read()
+        check_against_oracle(n, u, v, w, both, 0, p, d, kind)
