@@ -443,10 +443,8 @@ __global__ void k_set_sources(unsigned long long* state, int n, const int* srcs,
 // ---- host helpers --------------------------------------------------------------------------
 
 int cuda_fail(cudaError_t e, const char* what) {
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        return fail(DSSSP_E_OOM, "%s: out of device memory", what);
-    }
+    cudaGetLastError();  // reported here: the launch checks of a later call must not meet it
+    if (e == cudaErrorMemoryAllocation) return fail(DSSSP_E_OOM, "%s: out of device memory", what);
     return fail(DSSSP_E_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
@@ -1378,11 +1376,12 @@ void* pinned_view(void* p, size_t bytes) {
 }
 
 template <class D>
-void launch_unpack(dsssp_graph* g, int first, int count, int shift, int* parent, D* dist, cudaStream_t s) {
+cudaError_t launch_unpack(dsssp_graph* g, int first, int count, int shift, int* parent, D* dist, cudaStream_t s) {
     const unsigned long long* state = g->dg.state + first;
-    const bool vec = ((uintptr_t)parent & 15) == 0 && ((uintptr_t)dist & 15) == 0;
-    k_tree_unpack<D><<<blocks_for(((long long)count + 3) / 4), kThreads, 0, s>>>(state, count, shift, parent, dist, vec);
+    bool vec = ((uintptr_t)parent & 15) == 0 && ((uintptr_t)dist & 15) == 0;
+    void* args[] = {&state, &count, &shift, &parent, &dist, &vec};
     count_launch(1);
+    return cudaLaunchKernel((const void*)k_tree_unpack<D>, dim3(blocks_for(((long long)count + 3) / 4)), dim3(kThreads), args, 0, s);
 }
 
 // Parents (less shift) and distances of vertices [first, first + count) into host arrays (either may
@@ -1396,8 +1395,7 @@ int read_tree(dsssp_graph* g, int first, int count, int shift, int* parent, D* d
     D* vd = dist ? (D*)pinned_view(dist, sizeof(D) * (size_t)count) : nullptr;
     const bool direct = (!parent || (vp && ((uintptr_t)vp & 3) == 0)) && (!dist || (vd && ((uintptr_t)vd & (sizeof(D) - 1)) == 0));
     if (direct) {
-        if (parent || dist) launch_unpack<D>(g, first, count, shift, vp, vd, s);
-        CK(cudaGetLastError(), "tree read");
+        if (parent || dist) CK(launch_unpack<D>(g, first, count, shift, vp, vd, s), "tree read");
         CK(cudaStreamSynchronize(s), "tree read");
         return DSSSP_OK;
     }
@@ -1407,7 +1405,7 @@ int read_tree(dsssp_graph* g, int first, int count, int shift, int* parent, D* d
         if (rc) return rc;
     }
     D* sd = reinterpret_cast<D*>(g->d_dist);  // n int64 slots hold n of either width
-    launch_unpack<D>(g, first, count, shift, parent ? g->d_par : nullptr, dist ? sd : nullptr, s);
+    CK(launch_unpack<D>(g, first, count, shift, parent ? g->d_par : nullptr, dist ? sd : nullptr, s), "tree read");
     if (parent) CK(cudaMemcpyAsync(parent, g->d_par, sizeof(int) * (size_t)count, cudaMemcpyDeviceToHost, s), "tree read");
     if (dist) CK(cudaMemcpyAsync(dist, sd, sizeof(D) * (size_t)count, cudaMemcpyDeviceToHost, s), "tree read");
     CK(cudaStreamSynchronize(s), "tree read");
@@ -1860,7 +1858,7 @@ int dsssp_tree_read32_async(dsssp_graph* g, int32_t* parent, uint32_t* dist) {
     }
     cudaStream_t s = g->stream;
     if (g->copy_pending) CK(cudaStreamWaitEvent(s, g->ev_copied, 0), "tree read");  // staging in use
-    launch_unpack<unsigned>(g, 0, g->n, 0, parent ? g->a_par : nullptr, dist ? g->a_dist : nullptr, s);
+    CK(launch_unpack<unsigned>(g, 0, g->n, 0, parent ? g->a_par : nullptr, dist ? g->a_dist : nullptr, s), "tree read");
     CK(cudaEventRecord(g->ev_unpacked, s), "tree read");
     CK(cudaStreamWaitEvent(g->copy_stream, g->ev_unpacked, 0), "tree read");
     if (parent)

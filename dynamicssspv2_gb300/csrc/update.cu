@@ -2471,15 +2471,17 @@ cudaError_t launch_front(const UpdParams& p, int grid, cudaStream_t s, cudaEvent
 }
 
 cudaError_t launch_grow_finish(const UpdParams& p, int grid, cudaStream_t s) {
-    k_grow_finish<<<(unsigned)grid, 256, 0, s>>>(p);
+    UpdParams copy = p;
+    void* args[] = {&copy};
     count_launch(1);
-    return cudaGetLastError();
+    return cudaLaunchKernel((const void*)k_grow_finish, dim3((unsigned)grid), dim3(256), args, 0, s);
 }
 
 cudaError_t launch_dist_check(const DevGraph& g, int grid, cudaStream_t s) {
-    k_dist_check<<<(unsigned)grid, 256, 0, s>>>(g);
+    DevGraph copy = g;
+    void* args[] = {&copy};
     count_launch(1);
-    return cudaGetLastError();
+    return cudaLaunchKernel((const void*)k_dist_check, dim3((unsigned)grid), dim3(256), args, 0, s);
 }
 
 // Loads the kernel, so that its first launch allocates nothing.

@@ -1,5 +1,7 @@
 """Limits that a call states or meets: the caller's round cap, the range of the distances,
-the count of the entries."""
+the count of the entries, host memory that is pinned in part."""
+import mmap
+
 import numpy as np
 import pytest
 
@@ -227,3 +229,41 @@ def test_lines_deleted_in_both_orientations_are_counted_once(kind, tails):
         assert g.health()["live"] == 2 * (len(u) - len(gone))
         p, d = g.tree_read()
         check_against_oracle(n, u, v, w, both, 0, p, d, kind)
+
+
+PAGE = 1 << 16
+
+
+@pytest.fixture
+def patchwork():
+    """Six pages of host memory, of which the first, the third and the fourth are pinned, each by itself."""
+    torch = pytest.importorskip("torch")
+    torch.cuda.init()
+    rt = torch.cuda.cudart()
+    mem = np.frombuffer(mmap.mmap(-1, 7 * PAGE), np.uint8)
+    mem = mem[-mem.ctypes.data % PAGE:][: 6 * PAGE]
+    mem[:] = 77
+    at = [mem.ctypes.data + k * PAGE for k in (0, 2, 3)]
+    for p in at:
+        assert int(rt.cudaHostRegister(p, PAGE, 0)) == 0
+    yield mem
+    torch.cuda.synchronize()
+    for p in at:
+        assert int(rt.cudaHostUnregister(p)) == 0
+
+
+def test_a_failed_copy_is_reported_once(patchwork):
+    """A read into an array that the runtime refuses to copy to fails alone: the next call is not told
+    of it again."""
+    torch = pytest.importorskip("torch")
+    n = 3 * PAGE // 4
+    u, v, w = D.gen_er(n, 2 * n, 1, 100, 5)
+    with D.Graph(n, u, v, w) as g:
+        g.tree_compute(0)
+        want = g.tree_read32()
+        with pytest.raises(D.DsssspError) as e:
+            g.tree_read32_async(patchwork[: 4 * n].ctypes.data, None)  # a page of three is not pinned
+        assert e.value.code == D.E_CUDA
+        par, dist = (torch.empty(n, dtype=torch.int32).pin_memory().numpy() for _ in range(2))
+        g.tree_read32(par, dist.view(np.uint32))
+        assert np.array_equal(par, want[0]) and np.array_equal(dist.view(np.uint32), want[1])
