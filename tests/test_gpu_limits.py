@@ -267,3 +267,37 @@ def test_a_failed_copy_is_reported_once(patchwork):
         par, dist = (torch.empty(n, dtype=torch.int32).pin_memory().numpy() for _ in range(2))
         g.tree_read32(par, dist.view(np.uint32))
         assert np.array_equal(par, want[0]) and np.array_equal(dist.view(np.uint32), want[1])
+
+
+def test_pinned_memory_is_pinned_throughout(patchwork):
+    """Kernels read records from pinned memory and write trees to it only where all of the array is
+    pinned, in one piece or in adjoining ones; an array with a pageable page between its pinned ends is
+    left to the runtime's copy, which refuses it, and nothing is applied."""
+    torch = pytest.importorskip("torch")
+    n = PAGE // 4
+    dist = torch.empty(n, dtype=torch.int32).pin_memory().numpy().view(np.uint32)
+    u, v, w = D.gen_er(n, 2 * n, 1, 100, 5)
+    records = D.gen_changes(n, u, v, w, PAGE // 16, PAGE // 16, seed=6)  # two pages of them
+    with D.Graph(n, u, v, w) as g:
+        g.tree_compute(0)
+        g.snapshot()
+        want = g.tree_read32()
+        whole = patchwork[2 * PAGE: 3 * PAGE].view(np.int32)
+        g.tree_read32(whole, dist)
+        assert np.array_equal(whole, want[0]) and np.array_equal(dist, want[1])
+        across = patchwork[3 * PAGE - 2 * n: 3 * PAGE + 2 * n].view(np.int32)  # half in either pinned page
+        g.tree_read32(across, dist)
+        assert np.array_equal(across, want[0])
+        patchwork[2 * PAGE: 4 * PAGE] = records.view(np.uint8)
+        g.apply_batch(patchwork[2 * PAGE: 4 * PAGE].view(D.CHANGE_DTYPE))
+        after = g.tree_read32()
+        check_against_oracle(n, u, v, w, records, 0, *g.tree_read(), "records in two pinned pages")
+        g.restore()
+        gap = patchwork[PAGE // 2: 2 * PAGE + PAGE // 2]
+        gap[:] = records.view(np.uint8)
+        with pytest.raises(D.DsssspError) as e:
+            g.apply_batch(gap.view(D.CHANGE_DTYPE))
+        assert e.value.code == D.E_CUDA
+        assert all(np.array_equal(a, b) for a, b in zip(g.tree_read32(), want))
+        g.apply_batch(records)
+        assert all(np.array_equal(a, b) for a, b in zip(g.tree_read32(), after))
