@@ -1698,12 +1698,19 @@ int dsssp_graph_info(const dsssp_graph* g, int64_t* n, int64_t* entries, int64_t
     if (source) *source = g->src;
     if (device_bytes) {
         const long long N = g->n;
-        long long b = N * (8 + 16 + 4 + 4 + 4 + 4 + 4) + g->cap_total * 8 + 3 * g->dg.tcap * 8 +
-                      3 * g->dg.ccap * 8 + g->chg_cap * (16 + 4 + 32) + (long long)g->hcap * 16 +
-                      (g->dg.twin ? g->cap_total * 4 : 0) +
-                      (long long)sizeof(Ctl);
-        if (g->d_par) b += N * 12;
-        if (g->has_snap) b += N * (8 + 16 + 4) + g->s_cap * 8;
+        // state, rows, sorted lengths, four tag arrays, roots; the adjacency; the work lists
+        long long b = N * (8 + 16 + 4 + 16 + 4) + g->cap_total * (g->dg.twin ? 12 : 8) +
+                      3 * (g->dg.tcap + g->dg.ccap) * (long long)sizeof(Item) + (long long)sizeof(Ctl);
+        if (g->dg.far_tag) b += N * 12;
+        // batches: records, overflow list, slots, tail list, deletion set, seeds; row growth
+        b += g->chg_cap * (16 + 2 * 16 + 2 * 8) + (g->chg_cap ? tail_capacity(g->chg_cap) * 16 : 0) +
+             (long long)g->hcap * (long long)sizeof(DelSlot) + 4 * (2 * g->chg_cap < N ? 2 * g->chg_cap : N);
+        if (g->d_gidx) b += N * 4;
+        b += g->grow_rows * 48 + g->grow_chunks * 12 + g->grow_ends * 8;
+        if (g->d_par) b += N * 12;  // staging of tree reads
+        if (g->a_par) b += N * 8;
+        if (g->d_vtx) b += N * 4;
+        if (g->s_state) b += N * (8 + 16 + 4) + g->s_cap * (g->s_twin ? 12 : 8);
         *device_bytes = b;
     }
     return DSSSP_OK;

@@ -1,5 +1,5 @@
 """Limits that a call states or meets: the caller's round cap, the range of the distances,
-the count of the entries, host memory that is pinned in part."""
+the count of the entries, host memory that is pinned in part, device memory."""
 import mmap
 
 import numpy as np
@@ -301,3 +301,31 @@ def test_pinned_memory_is_pinned_throughout(patchwork):
         assert all(np.array_equal(a, b) for a, b in zip(g.tree_read32(), want))
         g.apply_batch(records)
         assert all(np.array_equal(a, b) for a, b in zip(g.tree_read32(), after))
+
+
+def test_the_footprint_covers_what_a_graph_holds():
+    """What a large sparse graph takes on the device once it has a tree and a batch behind it: the engine's
+    own count of it and, without a spare region, which the estimate does not know of, the estimate by
+    which tenants are admitted.  Allocations come in granules of 2 MiB; the lists of long rows'
+    items (about 1.3 % of the slots at 48 bytes) are beside the estimate too."""
+    torch = pytest.importorskip("torch")
+    from dynamicssspv2_gb300.serve import estimate_footprint
+
+    with D.Graph(100, *D.gen_er(100, 300, 1, 9, 1)) as g:  # modules are loaded, the context is up
+        g.tree_compute(0)
+        g.apply_batch(D.make_changes([1], [2], [3], [1]))
+        g.tree_read()
+    n, m = 1 << 23, 1 << 24
+    u, v, w = D.gen_er(n, m, 1, 100, 7)
+    ch = D.gen_changes(n, u, v, w, 500, 500, seed=8)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    with D.Graph(n, u, v, w, slack_pct=0, slack_min=4, spare_pct=0) as g:
+        g.tree_compute(0)
+        g.apply_batch(ch)
+        used = before - torch.cuda.mem_get_info()[0]
+        held = g.info()["device_bytes"]
+        granules = 40 * (2 << 20)
+        assert held <= used <= held + granules
+        slots = 2 * m + 4 * n
+        assert used <= estimate_footprint(n, m, 0, 4) + 0.013 * slots * 48 + granules
