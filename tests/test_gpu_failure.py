@@ -140,3 +140,69 @@ def test_timed_out_growth_keeps_the_whole_batch(recover):
             check_against_oracle(n, u, v, w, ch, 0, p, d, f"batch {seed}")
             u, v, w = lines_after(n, u, v, w, ch)
             assert g.health()["live"] == 2 * len(u) and g.validate()["violations"] == 0
+
+
+def _deletes_what_grew(g, n, u, v, w, ch, where):
+    """The tree after the batch, and one more batch that deletes every line the first inserted."""
+    p, d = g.tree_read()
+    check_against_oracle(n, u, v, w, ch, 0, p, d, where)
+    u, v, w = lines_after(n, u, v, w, ch)
+    assert g.health()["live"] == 2 * len(u) and g.validate()["violations"] == 0
+    gone = ch[ch["op"] == 1].copy()
+    gone["op"] = 0
+    g.apply_batch(gone)
+    p, d = g.tree_read()
+    check_against_oracle(n, u, v, w, gone, 0, p, d, f"{where}, deleted again")
+    u, v, w = lines_after(n, u, v, w, gone)
+    assert g.health()["live"] == 2 * len(u) and g.validate()["violations"] == 0
+
+
+@pytest.mark.parametrize("twice", [False, True])
+@pytest.mark.parametrize("hub", [0, 700])
+def test_a_growth_that_has_ended_is_ended_again(hub, twice):
+    """The update kernel fails behind the growth of the rows (a round cap of 1), so the growth's last
+    phase is run once more on rows that have grown: rows of one chunk, a hub of several, rows that close
+    up in place (twice: a batch before leaves tombstones) and rows that move."""
+    n, m = 6000, 24000
+    u, v, w = D.gen_er(n, m, 1, 100, 91)
+    if hub:
+        u, v, w = (np.concatenate([a, b]).astype(np.int32) for a, b in
+                   ((u, np.zeros(hub)), (v, 1 + np.arange(hub)), (w, np.full(hub, 150))))
+    with D.Graph(n, u, v, w, slack_pct=0, slack_min=0, spare_pct=200) as g:
+        g.tree_compute(0)
+        if twice:
+            at = np.flatnonzero(np.arange(len(u)) % 5 == 0)
+            ch = D.make_changes(u[at], v[at], w[at], np.zeros(len(at)))
+            g.apply_batch(ch)
+            u, v, w = lines_after(n, u, v, w, ch)
+        ch = D.gen_changes(n, u, v, w, 900, 900, seed=92)
+        if hub:
+            more = D.make_changes(np.zeros(300), 2000 + np.arange(300), np.full(300, 60), np.ones(300))
+            ch = np.concatenate([ch, more])
+        o = g.get_opts()
+        o.max_rounds = 1
+        g.set_opts(o)
+        st = g.apply_batch(ch)
+        assert st.recovered_from == D.E_NO_CONVERGENCE and st.overflow_entries > 0 and st.repacks == 0
+        o.max_rounds = 0
+        g.set_opts(o)
+        _deletes_what_grew(g, n, u, v, w, ch, f"hub {hub}")
+
+
+@pytest.mark.parametrize("lines", [1, 4])
+def test_a_growth_on_one_cta_is_ended_again(lines):
+    """A handful of rows grow on the first CTA alone while the others run out of polls for a late one:
+    the growth's last phase, which has run, is run once more."""
+    n, m = 6000, 24000
+    u, v, w = D.gen_er(n, m, 1, 100, 95)
+    a = 10 + 20 * np.arange(lines)
+    ch = np.concatenate([D.make_changes(a, a + 7, np.full(lines, 3), np.ones(lines)),
+                         D.make_changes(u[:50], v[:50], w[:50], np.zeros(50))])
+    with D.Graph(n, u, v, w, slack_pct=0, slack_min=0, spare_pct=200) as g:
+        g.tree_compute(0)
+        g.debug_set(D.DEBUG_SPIN_LIMIT, 4096)
+        g.debug_set(D.DEBUG_STALL_US, 200_000)
+        st = g.apply_batch(ch)
+        assert st.recovered_from == D.E_TIMEOUT and st.overflow_entries == 2 * lines and st.repacks == 0
+        g.debug_set(D.DEBUG_SPIN_LIMIT, 0)
+        _deletes_what_grew(g, n, u, v, w, ch, f"{lines} lines")
