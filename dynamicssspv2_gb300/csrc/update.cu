@@ -487,11 +487,14 @@ __device__ __forceinline__ void warp_agg_min(bool offer, unsigned c, unsigned lo
 
 // ---- per-edge operations ---------------------------------------------------------------
 // visit4 handles up to four adjacency entries per lane (a, a + stride, ... while below n; none for
-// n <= 0) and is called by all 32 lanes.  A busy round is bound by random accesses (a neighbour's
-// state per entry, 130-150 G/s against about 280 from the L2 with nothing else to do) and
-// instructions in equal parts; prefetching the next items' entries did not help (1.36 -> 1.40 ms for
-// the tree of RMAT scale 22), reading the next item early and leaving a visit in which no lane
-// improved anything did (1.39 -> 1.35 ms).
+// n <= 0) and is called by all 32 lanes.  A busy round makes 130-150 G visits a second, one random
+// access to a neighbour's state each, about half of what loads alone reach in an array of the L2
+// (280 G/s), so these accesses by themselves are not its bound.  Reading the next item early and
+// leaving a visit in which no lane improved anything gained (the tree of RMAT scale 22 1.39 -> 1.35
+// ms); prefetching the next items' entries (1.36 -> 1.40), adjacency words read by four lanes an
+// item (1.361 -> 1.360) and states through the L1 (1.35 -> 1.32 in one build, 1.36 -> 1.37 in
+// another) did not.  The other half of the cost is that an entry is visited about twice: that tree
+// takes 132M visits for 67M entries.
 template <bool kAgg>
 struct RelaxOp {
     const UpdParams* p;

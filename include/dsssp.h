@@ -66,10 +66,14 @@ typedef struct {
     int32_t slack_min;    /* minimum free slots per row */
     int32_t small_deg;    /* edges per thread work item (multiple of 4, 4..64): a frontier
                              vertex of degree d <= small_deg is one thread's item, a longer row
-                             up to large_deg is split into ceil(d/small_deg) thread items */
+                             up to large_deg is split into ceil(d/small_deg) thread items.  Small
+                             rounds run without grid barriers only up to 16, small levels of the
+                             subtree walk (and the pulls of a small batch together with its first
+                             rounds) only with 4 */
     int32_t large_deg;    /* rows above this degree are split into CTA items of `chunk` edges (with
-                             small_deg 4 and large_deg 256, the defaults, a tree from scratch on a
-                             large graph of long rows takes 8 and 512) */
+                             small_deg 4 and large_deg 256, the defaults, also where they were set
+                             by the caller, a tree from scratch on a large graph of long rows
+                             takes 8 and 512) */
     int32_t chunk;        /* edges per CTA work item */
     int32_t bfs_levels;   /* subtree walk levels before switching to pointer jumping */
     int32_t block;        /* threads per CTA of the update kernel (multiple of 32) */
@@ -109,7 +113,9 @@ typedef struct {
     int32_t warp_agg;     /* 1 = warp-aggregated distance offers: lanes of a warp offering to the
                              same vertex are grouped (__match_any_sync) and only the least offer
                              is issued as a 64-bit atomicMin; 0 (the default) = one atomicMin per
-                             improving offer.  Same results either way. */
+                             improving offer.  Same results either way; with 1 every relaxation
+                             round takes its grid barrier (on high-diameter graphs several times
+                             slower). */
     int32_t solo_waves;   /* a walk level or relaxation round with at most this many CTA-waves of
                              work items runs on one CTA with block barriers instead of the whole
                              grid (0..64; 0 = never; default 2) */
@@ -121,8 +127,9 @@ typedef struct {
                              CTAs with a barrier of their own while the other CTAs wait: a shorter
                              barrier and the slowest of group_ctas dependent chains instead of all
                              CTAs' (high-diameter graphs run thousands of such rounds); 0 (the
-                             default) = off: measured slower, the rounds wait on their items'
-                             dependent chains more than on the barrier */
+                             default) = off.  Not 0: neither relaxation rounds nor walk levels run
+                             without barriers as small ones otherwise do, which is about four times
+                             slower on high-diameter graphs */
     int32_t group_waves;  /* see group_ctas (1..64, default 2) */
 } dsssp_opts;
 
@@ -168,7 +175,9 @@ typedef struct {
                                   level 2) */
     int64_t recovered_from;    /* DSSSP_W_RECOMPUTED: the code of the failure recovered from */
     double t_recompute_ms;     /* DSSSP_W_RECOMPUTED: the recomputation of the trees (CUDA events) */
-    double t_seed_ms;          /* the seeding and pull phase alone (part of t_relax_ms) */
+    double t_seed_ms;          /* the seeding and pull phase alone (part of t_relax_ms); 0 where it runs
+                                  together with the first rounds, as in small batches on graphs of
+                                  short rows */
 } dsssp_stats;
 
 /* ---- engine ------------------------------------------------------------------------ */
