@@ -219,9 +219,12 @@ __global__ void k_tree_pack(const int* parent, const long long* dist, int n, uns
 }
 
 // The tree as parents (ids less `shift`) and distances of D's width: 64 bits with DSSSP_UNREACHABLE, or
-// 32 with 0xFFFFFFFF = unreachable, which is the state's own top half.  Four vertices a thread, so
-// the stores are 16 bytes wide where the outputs allow it (vec); the outputs may be pinned host
-// memory.  Bound: the host link (about 190 GB/s) or, for a small tree, the launch.
+// 32 with 0xFFFFFFFF = unreachable, which is the state's own top half.  A thread takes as many vertices
+// as make one store of 16 bytes of distances where the outputs allow it (vec), so that a warp's
+// store is one run of bytes (64-bit distances by two stores a thread, 32 bytes apart from lane to
+// lane, reach 150 GB/s: 4.2M vertices 328 us a read, so 273, by copies from staging 289); the
+// outputs may be pinned host memory.  Bound: the host link (about 190 GB/s) or, for a small tree,
+// the launch.
 template <class D>
 __device__ __forceinline__ D tree_dist(unsigned long long s) {
     if constexpr (sizeof(D) == 4) return (D)(s >> 32);
@@ -229,27 +232,29 @@ __device__ __forceinline__ D tree_dist(unsigned long long s) {
 }
 
 template <class D>
+constexpr int kUnpack = 16 / (int)sizeof(D);  // vertices a thread
+
+template <class D>
 __global__ void k_tree_unpack(const unsigned long long* state, int n, int shift, int* parent, D* dist, bool vec) {
-    const long long v = 4 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
+    constexpr int K = kUnpack<D>;
+    const long long v = K * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
     if (v >= n) return;
-    const int k = n - v < 4 ? (int)(n - v) : 4;
-    int p[4];
-    D d[4];
+    const int k = n - v < K ? (int)(n - v) : K;
+    int p[K];
+    D d[K];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < K; q++) {
         const unsigned long long s = q < k ? __ldcs(&state[v + q]) : kInfState;
         p[q] = s == kInfState ? -1 : (int)(unsigned)s - shift;
         d[q] = tree_dist<D>(s);
     }
-    if (vec && k == 4) {
-        if (parent) *reinterpret_cast<int4*>(parent + v) = make_int4(p[0], p[1], p[2], p[3]);
-        if (dist) {
-            if constexpr (sizeof(D) == 4) {
-                *reinterpret_cast<uint4*>(dist + v) = make_uint4((unsigned)d[0], (unsigned)d[1], (unsigned)d[2], (unsigned)d[3]);
-            } else {
-                reinterpret_cast<longlong2*>(dist + v)[0] = make_longlong2(d[0], d[1]);
-                reinterpret_cast<longlong2*>(dist + v)[1] = make_longlong2(d[2], d[3]);
-            }
+    if (vec && k == K) {
+        if constexpr (K == 4) {
+            if (parent) *reinterpret_cast<int4*>(parent + v) = make_int4(p[0], p[1], p[2], p[3]);
+            if (dist) *reinterpret_cast<uint4*>(dist + v) = make_uint4((unsigned)d[0], (unsigned)d[1], (unsigned)d[2], (unsigned)d[3]);
+        } else {
+            if (parent) *reinterpret_cast<int2*>(parent + v) = make_int2(p[0], p[1]);
+            if (dist) *reinterpret_cast<longlong2*>(dist + v) = make_longlong2(d[0], d[1]);
         }
         return;
     }
@@ -1407,7 +1412,7 @@ cudaError_t launch_unpack(dsssp_graph* g, int first, int count, int shift, int* 
     bool vec = ((uintptr_t)parent & 15) == 0 && ((uintptr_t)dist & 15) == 0;
     void* args[] = {&state, &count, &shift, &parent, &dist, &vec};
     count_launch(1);
-    return cudaLaunchKernel((const void*)k_tree_unpack<D>, dim3(blocks_for(((long long)count + 3) / 4)), dim3(kThreads), args, 0, s);
+    return cudaLaunchKernel((const void*)k_tree_unpack<D>, dim3(blocks_for(((long long)count + kUnpack<D> - 1) / kUnpack<D>)), dim3(kThreads), args, 0, s);
 }
 
 // Parents (less shift) and distances of vertices [first, first + count) into host arrays (either may
@@ -1418,7 +1423,7 @@ template <class D>
 int read_tree(dsssp_graph* g, int first, int count, int shift, int* parent, D* dist) {
     cudaStream_t s = g->stream;
     int* vp = parent ? (int*)pinned_view(parent, sizeof(int) * (size_t)count, true) : nullptr;
-    D* vd = dist ? (D*)pinned_view(dist, sizeof(D) * (size_t)count, true) : nullptr;
+    D* vd = dist && (vp || !parent) ? (D*)pinned_view(dist, sizeof(D) * (size_t)count, true) : nullptr;
     const bool direct = (!parent || (vp && ((uintptr_t)vp & 3) == 0)) && (!dist || (vd && ((uintptr_t)vd & (sizeof(D) - 1)) == 0));
     if (direct) {
         if (parent || dist) CK(launch_unpack<D>(g, first, count, shift, vp, vd, s), "tree read");
