@@ -61,6 +61,7 @@ constexpr int kLocalTe = 16;               // thread items of more edges than th
 constexpr unsigned kFarBuf = 64;           // per-warp staging of far-list pushes
 constexpr int kSpill = 64;                 // per-warp staging of vertices that leave a stretch
 constexpr unsigned kStretch = 256;         // steps of a local stretch at most
+constexpr unsigned kShortStretch = 4, kMinRest = 8, kMaxRest = 256;  // see after_stretch
 static_assert(64 * (kLocalTe / 4) <= kQueue, "a CTA's first items must fit its queue");
 // a stretch keeps all of it in the push buffers: kSpill entries a warp for vertices that leave it,
 // the queues (two, and a third for the walk), the far staging in the third one's place
@@ -870,6 +871,33 @@ __device__ __forceinline__ void keep_stats(const LocalStats& ls);
 // barrier.
 __device__ __forceinline__ bool stretches(const UpdParams& p) { return p.capped == 0; }
 
+// A stretch of at most four steps that leaves work does not pay where the next ones are like it: rows above
+// kLocalDeg leave it at every hop, and a barrier with a new deal of the work costs 7 us where a round
+// of few items on CTA 0 alone costs 3 (small_step).  From the fourth such stretch in a row on, the
+// next lists run as rounds, 8 at first and twice as many after each further one, up to 256.  A spine of
+// 3,000 vertices with 60 leaves each, computation and batches 25.7 and 2.7 ms in stretches throughout,
+// 12.6 and 1.9 ms so, 12.4 and 2.0 ms in rounds; 400 layers of 50 vertices with 20 edges to the next
+// 4.2, 3.4 and 2.9 ms.  Not earlier: RMAT and ER graphs, a few short stretches deep in all, took up to
+// 10 % more (RMAT-18 with 1,000 changes 121 -> 134 us).  Two or 8 steps for four: 4.2 and 3.4 ms on the
+// layers, the rest the same.  The state is in shared memory: the loops' registers are full.
+__shared__ unsigned s_rest[2];  // lists (levels) before number [0] run as rounds; [1] how many the last time
+
+__device__ __forceinline__ void no_rest() {  // read behind the next block barrier
+    if (threadIdx.x < 2) s_rest[threadIdx.x] = 0;
+}
+
+__device__ __forceinline__ void after_stretch(unsigned used, bool left, unsigned next) {
+    if (threadIdx.x == 0) {
+        unsigned span = 0;
+        if (used <= kShortStretch && left) {
+            span = s_rest[1] ? min(2 * s_rest[1], kMaxRest) : 1u;
+            if (span >= kMinRest) s_rest[0] = next + span;
+        }
+        s_rest[1] = span;
+    }
+    __syncthreads();
+}
+
 // A graph of whose rows nearly all fit a stretch's queue.  On others (RMAT: one row in ten above
 // kLocalDeg) a stretch soon leaves through the lists, and the phases before it are better kept
 // apart: seeds, pulls and the first rounds of an RMAT-20 insertion batch 0.071 ms apart, 0.083 in one.
@@ -1408,9 +1436,8 @@ __device__ __forceinline__ void clear_slots(Ctl* ctl, unsigned slot) {
 // list r is the near one, its sizes in s_near; kWhole: a stretch is to take the far list.  A
 // function of its own, so that the rounds keep their registers.
 enum Advance { kStop, kSplit, kWhole };
-template <bool kAgg>
 __device__ __noinline__ Advance advance(const UpdParams& p, unsigned r, unsigned nfar, unsigned rbase, unsigned adv,
-                                        unsigned long long T, bool least) {
+                                        unsigned long long T, bool least, bool local) {
     Ctl* const ctl = p.g.ctl;
     const unsigned long long tn = next_threshold(p, nfar, adv, T, least);
     if (tn == 0) return kStop;
@@ -1418,7 +1445,7 @@ __device__ __noinline__ Advance advance(const UpdParams& p, unsigned r, unsigned
         ctl->fc[(adv + 2) % 3] = 0;
         ctl->fmin[(adv + 1) & 1] = 0;
     }
-    const bool whole = !kAgg && stretches(p) && local_advance(p, nfar);
+    const bool whole = local && local_advance(p, nfar);
     if (!whole && !far_advance(p, r, nfar, rbase, adv, T, tn)) return kStop;
     if (threadIdx.x == 0) s_threshold = tn;
     __syncthreads();
@@ -1470,7 +1497,7 @@ __device__ __forceinline__ unsigned long long walk(const UpdParams& p) {
             need_pj = true;
             break;
         }
-        if (p.te == 4 && local_step(p, hiT - loT, hiC - loC)) {
+        if (p.te == 4 && (unsigned)level >= s_rest[0] && local_step(p, hiT - loT, hiC - loC)) {
             if (leader) {
                 ctl->ltT[(li + 2) % 3] = 0;
                 ctl->ltC[(li + 2) % 3] = 0;
@@ -1486,6 +1513,7 @@ __device__ __forceinline__ unsigned long long walk(const UpdParams& p) {
             hiT += addT;
             hiC += addC;
             level += (int)used;
+            after_stretch(used, addT != 0 || addC != 0, (unsigned)level);
             li++;
             continue;
         }
@@ -2179,6 +2207,7 @@ __device__ void update_body(const UpdParams& p);
 template <bool kAgg>
 __global__ void __launch_bounds__(256, 3) k_update(const __grid_constant__ UpdParams p) {
     if (threadIdx.x < 8) s_lstat[threadIdx.x] = 0;
+    no_rest();
     if (threadIdx.x == 0) {
         s_nbar = 0;
         s_gen = ld_acquire(&p.g.ctl->bar_gen);
@@ -2288,6 +2317,8 @@ __device__ void update_body(const UpdParams& p) {
     if (leader && p.mode == 1) ctl->ts[2] = globaltimer();
 
     // ---- C. relaxation rounds ---------------------------------------------------------------
+    no_rest();  // ... of the walk: behind a barrier as well
+    __syncthreads();
     for (;; r++) {
         // nT, nC: the sizes of round r's lists (read at the barrier before)
         if (!nf && p.late_delta != 0 && hops >= p.late_after) {
@@ -2298,6 +2329,7 @@ __device__ void update_body(const UpdParams& p) {
             T = 0;
         }
         Begin kind = kList;
+        const bool local = !kAgg && stretches(p) && r >= s_rest[0];
         bool least = true;
         unsigned nfar = 0;
         unsigned long long before = 0;
@@ -2308,7 +2340,7 @@ __device__ void update_body(const UpdParams& p) {
             if (nfar == 0) break;
             least = T == 0 || sparse || !stretches(p);
             before = T;
-            const Advance got = advance<kAgg>(p, r, nfar, rbase, adv, T, least);
+            const Advance got = advance(p, r, nfar, rbase, adv, T, least, local);
             if (got == kStop) break;
             T = s_threshold;
             adv++;
@@ -2328,7 +2360,7 @@ __device__ void update_body(const UpdParams& p) {
             if (leader) set_status(ctl, -5 /* NO_CONVERGENCE */);
             break;
         }
-        if (!kAgg && stretches(p) && (kind == kWaiting || local_step(p, nT, nC))) {
+        if (local && (kind == kWaiting || local_step(p, nT, nC))) {
             if (leader) clear_slots(ctl, (r + 2) % 3);
             relax_local(p, r, nT, rbase, adv, T, kind, 0, nfar, before);
             unsigned t2, used;
@@ -2336,6 +2368,7 @@ __device__ void update_body(const UpdParams& p) {
                 break;
             nT = t2;
             hops += used;
+            after_stretch(used, nT != 0 || nC != 0, r + 1);
             if (!least && used == 0 && nT == 0 && nC == 0) sparse = true;
             continue;
         }

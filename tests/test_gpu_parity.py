@@ -1105,3 +1105,37 @@ def test_tree_reads_into_pinned_and_pageable_memory(n):
             par, dist = pinned(np.int32, off), pinned(np.int64, off)
             D._check(D._lib.dsssp_tree_read_range(g.handle, a, c, par.ctypes.data, dist.ctypes.data), "tree_read_range")
             assert np.array_equal(par[:c], want[0][a:]) and np.array_equal(dist[:c], want[1][a:]) and par[c] == dist[c] == 77
+
+
+@pytest.mark.parametrize("leaves", [30, 31, 60, 254, 255])
+@pytest.mark.parametrize("opts", [{}, {"delta": 64}, {"bfs_levels": 400}, {"small_deg": 16}], ids=str)
+def test_deep_graphs_of_long_rows(leaves, opts):
+    """A spine long enough that its stretches, one hop each where the rows are above 32 entries, give way
+    to rounds more than once, ends in a bare chain (stretches again) and in a second spine: the tree and a
+    batch that cuts it near its root, against the oracle and a graph of rounds alone."""
+    parts, n, tail = [], 1, 0
+    for kind, length in (("spine", 90), ("chain", 300), ("spine", 60)):
+        at = n + np.arange(length)
+        parts.append((np.concatenate([[tail], at[:-1]]), at))
+        n += length
+        if kind == "spine":
+            parts.append((np.repeat(at, leaves), n + np.arange(length * leaves)))
+            n += length * leaves
+        tail = at[-1]
+    u, v = (np.ascontiguousarray(np.concatenate(x), np.int32) for x in zip(*parts))
+    w = (1 + np.arange(len(u)) * 2654435761 % 41).astype(np.int32)
+    cut = D.make_changes(u[2:3], v[2:3], w[2:3], np.zeros(1))
+    ch = np.concatenate([D.gen_changes(n, u, v, w, 30, 30, seed=leaves), cut,
+                         D.make_changes(u[2:3], v[2:3], w[2:3] + 60, np.ones(1))])
+    got = []
+    for extra in ({}, {"group_ctas": 2, "solo_waves": 0}):
+        with D.Graph(n, u, v, w, **{**opts, **extra}) as g:
+            for _ in range(2):
+                g.tree_compute(0)
+                p0, d0 = g.tree_read()
+                check_against_oracle(n, u, v, w, None, 0, p0, d0, f"{leaves} leaves")
+            g.apply_batch(ch)
+            p1, d1 = g.tree_read()
+            check_against_oracle(n, u, v, w, ch, 0, p1, d1, f"{leaves} leaves, batch")
+            got.append((p0, p1))
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
