@@ -58,6 +58,7 @@ static_assert(kBuf > kAddsPerCheck, "a push buffer must take one visit's adds af
 constexpr int kSoloSteps = 256;            // consecutive solo steps before the grid re-syncs
 constexpr unsigned kQueue = 256;           // items of a CTA's queue in a local stretch (two queues)
 constexpr int kLocalTe = 16;               // thread items of more edges than this keep to the rounds
+constexpr unsigned kFewHops = 16;          // an advance that buys fewer is widened (see advance)
 constexpr unsigned kFarBuf = 64;           // per-warp staging of far-list pushes
 constexpr int kSpill = 64;                 // per-warp staging of vertices that leave a stretch
 constexpr unsigned kStretch = 256;         // steps of a local stretch at most
@@ -83,6 +84,8 @@ __shared__ unsigned s_stop[2];             // ... another CTA has ended the stre
 __shared__ unsigned s_qcnt[3];             // local stretches: items of the steps' queues, rotating
 __shared__ unsigned s_near[2];  // advance: the sizes of the near list
 __shared__ unsigned long long s_threshold;
+__shared__ unsigned long long s_width;  // near-far: the bucket width
+__shared__ unsigned s_advanced;         // ... the hops as of the last advance
 __shared__ unsigned long long s_lstat[8];  // ... their counters, added to the kernel's at the end
 __shared__ unsigned s_wlist[kMaxWarps][kListRegion];  // k_delete / k_append list staging
 
@@ -1360,7 +1363,7 @@ __device__ __forceinline__ void keep_stats(const LocalStats& ls) {
 // and a barrier.  0 when nothing waits or the kernel must stop.
 __device__ __forceinline__ unsigned long long next_threshold(const UpdParams& p, unsigned nfar, unsigned adv,
                                                           unsigned long long T, bool least) {
-    const unsigned long long width = p.delta ? p.delta : p.late_delta;
+    const unsigned long long width = s_width;
     if (!least) return T + width;
     Ctl* const ctl = p.g.ctl;
     const DevGraph& g = p.g;
@@ -1437,8 +1440,19 @@ __device__ __forceinline__ void clear_slots(Ctl* ctl, unsigned slot) {
 // function of its own, so that the rounds keep their registers.
 enum Advance { kStop, kSplit, kWhole };
 __device__ __noinline__ Advance advance(const UpdParams& p, unsigned r, unsigned nfar, unsigned rbase, unsigned adv,
-                                        unsigned long long T, bool least, bool local) {
+                                        unsigned long long T, bool least, bool local, unsigned hops) {
     Ctl* const ctl = p.g.ctl;
+    if (p.delta == 0) {
+        // A plain computation that goes on near-far has a width by the mean weight alone, which says little
+        // where weights differ widely: a path of 8,000 edges of 250,000 beside 3M of 1 and 2 took an
+        // advance of 12 us for each edge, 98 ms against 25 ms of plain rounds.  An advance that has bought
+        // few hops doubles the width: 12.5 ms.  (Grids buy about 80 hops with each and keep theirs.)
+        if (threadIdx.x == 0) {
+            if (adv > 0 && hops - s_advanced < kFewHops && s_width < kDistInf) s_width *= 2;
+            s_advanced = hops;
+        }
+        __syncthreads();
+    }
     const unsigned long long tn = next_threshold(p, nfar, adv, T, least);
     if (tn == 0) return kStop;
     if (blockIdx.x == 0 && threadIdx.x == 0) {  // read by every CTA before the last barrier, written after the next
@@ -2210,6 +2224,8 @@ __global__ void __launch_bounds__(256, 3) k_update(const __grid_constant__ UpdPa
     no_rest();
     if (threadIdx.x == 0) {
         s_nbar = 0;
+        s_width = p.delta ? p.delta : p.late_delta;
+        s_advanced = 0;
         s_gen = ld_acquire(&p.g.ctl->bar_gen);
         s_ggen = ld_acquire(&p.g.ctl->grp_gen);
         const unsigned lim = __ldcg(&p.g.ctl->spin_limit);
@@ -2340,7 +2356,7 @@ __device__ void update_body(const UpdParams& p) {
             if (nfar == 0) break;
             least = T == 0 || sparse || !stretches(p);
             before = T;
-            const Advance got = advance(p, r, nfar, rbase, adv, T, least, local);
+            const Advance got = advance(p, r, nfar, rbase, adv, T, least, local, hops);
             if (got == kStop) break;
             T = s_threshold;
             adv++;

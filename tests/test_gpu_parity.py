@@ -1139,3 +1139,22 @@ def test_deep_graphs_of_long_rows(leaves, opts):
             check_against_oracle(n, u, v, w, ch, 0, p1, d1, f"{leaves} leaves, batch")
             got.append((p0, p1))
     assert all(np.array_equal(a, b) for a, b in zip(*got))
+
+
+def test_a_deep_computation_under_weights_that_differ_widely():
+    """A path of heavy edges beside a large light component: the width that a deep computation takes from
+    the mean weight is less than one of them, and widens, so that an advance buys several hops."""
+    n, k = 1 << 19, 3000
+    u, v, w = D.gen_er(n, 3 * n // 2, 1, 2, 41)
+    path = n + np.arange(k)
+    u = np.concatenate([u, [0], path[:-1]]).astype(np.int32)
+    v = np.concatenate([v, path]).astype(np.int32)
+    w = np.concatenate([w, 250_000 + np.arange(k) % 7]).astype(np.int32)
+    got = []
+    for opts in ({}, {"delta": 0}):
+        with D.Graph(n + k, u, v, w, **opts) as g:
+            st = g.tree_compute(0)
+            assert st.rounds > k and (st.advances == 0 if opts else 0 < st.advances < k // 4)
+            assert g.validate()["violations"] == 0
+            got.append(g.tree_read())
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
