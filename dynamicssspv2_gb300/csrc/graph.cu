@@ -919,9 +919,11 @@ int repack(dsssp_graph* g, const int4* d_ovf, int n_ovf, cudaStream_t s) {
 // 0.83, 1.39 -> 1.34 and 2.67 -> 2.30 ms, of scale 20 with 8 million 0.465 -> 0.443, ER of 2^20 vertices
 // with 16 and 32 edges each 1.68 -> 1.61 and 2.60 -> 2.41 ms; RMAT-18 the same, RMAT-16 0.157 -> 0.165, and
 // on shorter rows (ER with 4 edges each) 0.57 -> 0.64 ms.  The default sizes are known by their values:
-// a caller that sets 4 and 256 itself gets the wide items too, any other setting stays.
+// a caller that sets 4 and 256 itself gets the wide items too, any other setting stays.  Not with
+// aggregated offers or group rounds, where every round takes a barrier (RMAT-18 with group rounds on 16
+// CTAs 242 -> 268 us by wide items).
 bool wide_items(const dsssp_graph* g) {
-    return g->o.small_deg == 4 && g->o.large_deg == 256 && g->n >= (1 << 18) &&
+    return g->o.small_deg == 4 && g->o.large_deg == 256 && g->o.warp_agg == 0 && g->o.group_ctas == 0 && g->n >= (1 << 18) &&
            64ull * g->h_ctl->long_rows > (unsigned long long)g->n;
 }
 
