@@ -1,5 +1,6 @@
 """Limits that a call states or meets: the caller's round cap, the range of the distances,
 the count of the entries, host memory that is pinned in part, device memory."""
+import gc
 import mmap
 
 import numpy as np
@@ -318,6 +319,7 @@ def test_the_footprint_covers_what_a_graph_holds():
     n, m = 1 << 23, 1 << 24
     u, v, w = D.gen_er(n, m, 1, 100, 7)
     ch = D.gen_changes(n, u, v, w, 500, 500, seed=8)
+    gc.collect()  # graphs of other tests are gone
     torch.cuda.synchronize()
     before = torch.cuda.mem_get_info()[0]
     with D.Graph(n, u, v, w, slack_pct=0, slack_min=4, spare_pct=0) as g:
